@@ -1201,7 +1201,7 @@ int mpm_step(MpmHandle* h, int nsteps, void* stream) {
     }
     cudaStream_t s = S(stream);
     if (h->ndim == 1) {   // Linear1D: re-sorted every step, status checked at the end
-        for (int t = 0; t < nsteps; ++t) TRY(line_step(h, s));
+        TRY(line_steps(h, nsteps, s));
         TRY(read_ctl(h, s));
         int st = h->h_ctl->status;
         TRY(check_status(h, st));

@@ -226,7 +226,12 @@ struct LineTapeSlot {
     int* cs;
     float* n[4];
 };
-int line_step(MpmHandle* h, cudaStream_t s, const LineTapeSlot* tape = nullptr);   // mpm_line.cu
+// n 1-D steps (mpm_line.cu); `tape` is the slot of the first, consecutive
+// steps follow at 9 particle, 4 node and one index array each.
+int line_steps(MpmHandle* h, int n, cudaStream_t s, const LineTapeSlot* tape = nullptr);
+// Bars up to this size run their steps (and reverse steps) in one CTA.
+constexpr int LINE_FUSED_MAX = 2048;
+inline bool line_fused(const MpmHandle* h) { return h->np <= LINE_FUSED_MAX && h->nx < LINE_FUSED_MAX; }
 int line_setup_volume(MpmHandle* h, cudaStream_t s);
 int to_device(MpmHandle* h, const void* src, size_t bytes, int on_device, cudaStream_t s,
               const void** dsrc);

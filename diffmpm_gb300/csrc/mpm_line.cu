@@ -183,6 +183,300 @@ k_line_g2p(const __grid_constant__ SimDev S, const int* __restrict__ eid, Contro
     if (ne < 0 || ne >= S.nx) atomicOr(&ctl->status, ST_OUT_OF_MESH);
 }
 
+// ---------------------------------------------------------------------------
+// Whole runs of steps in one CTA, for bars of at most LINE_FUSED_MAX particles
+// and elements (every known use of the 1-D elements).  A step as separate
+// kernels is ~26 dependent launches of one or two CTAs, so launches are all of
+// its time (216 particles: 102 us a step).  Here a thread keeps its particles
+// in registers for all steps, nodes and element lists live in shared memory,
+// and a step is six barriers.  The lists are rebuilt only after a step in
+// which a particle changed element.  Bound by the latency of the barriers and
+// of the serial node sums: 216 particles 102 -> 4.5 us a step, one particle
+// with its adjoint 163 -> 6 us a step.  Contributions are formed once per
+// particle and stored in list order; a node adds them in the order of
+// for_node_particles, so every sum has the same terms in the same order as
+// the separate kernels: the same bits.
+// ---------------------------------------------------------------------------
+struct LineTape {   // of the whole run (LineTapeSlot by step), or P == nullptr
+    float* P;       // [step][9][np]
+    int* pid;       // [step][np]
+    int* cs;        // [step][nx + 2]
+    float* N;       // [step][4][nn]
+};
+
+struct LineShared {
+    float *m, *va, *vb, *a, *V0, *c;   // nodes, reset volume per element, contributions [4][np] in list order
+    int *start, *cnt, *pid;            // element lists: starts [nx + 2], scratch [nx + 1], original index per slot
+    __device__ LineShared(char* raw, int np, int nx) {
+        float* f = reinterpret_cast<float*>(raw);
+        const int nn = nx + 1;
+        m = f; va = m + nn; vb = va + nn; a = vb + nn; V0 = a + nn; c = V0 + nx;
+        start = reinterpret_cast<int*>(c + 4 * (size_t)np);
+        cnt = start + nx + 2;
+        pid = cnt + nn;
+    }
+};
+inline size_t line_shared_bytes(int np, int nx) {
+    return 4 * ((size_t)4 * (nx + 1) + nx + 4 * (size_t)np + (nx + 2) + (nx + 1) + (size_t)np);
+}
+
+// Sum the two contribution rows of node i in for_node_particles' order.
+__device__ __forceinline__ void line_node_sums(const LineShared& W, int np, int nx, int i, float& s0, float& s1) {
+    int a = 0, ae = 0, b = 0, be = 0;
+    if (i >= 1) { a = W.start[i - 1]; ae = W.start[i]; }
+    if (i < nx) { b = W.start[i]; be = W.start[i + 1]; }
+    const float *l0 = W.c, *r0 = W.c + np, *l1 = W.c + 2 * np, *r1 = W.c + 3 * np;
+    s0 = s1 = 0.0f;
+    #pragma unroll 1
+    while (a < ae || b < be) {
+        const bool left = a < ae && (b >= be || W.pid[a] < W.pid[b]);
+        if (left) { s0 = fa(s0, r0[a]); s1 = fa(s1, r1[a]); ++a; }
+        else { s0 = fa(s0, l0[b]); s1 = fa(s1, l1[b]); ++b; }
+    }
+}
+
+// A particle's element lists entry: bucket (nx: outside the mesh), geometry, slot.
+struct LineP {
+    float x, v;
+    PState s;
+    float vol, mass, Ep, mp, N0, N1, gc, gr, x0, x1;
+    int e, slot, pid, mat, code;
+};
+
+template <bool REINIT, bool USL, int PPT>
+__global__ void __launch_bounds__(1024)
+k_line_steps(const __grid_constant__ SimDev S, int par, int step0, int nsteps, Control* __restrict__ ctl,
+             const LineTape tape) {
+    extern __shared__ char s_raw[];
+    __shared__ int s_warp[32];
+    __shared__ int s_carry;
+    const int np = S.np, nx = S.nx, nn = nx + 1, T = blockDim.x, tid = threadIdx.x;
+    const LineShared W(s_raw, np, nx);
+    LineP P[PPT];
+    int status = 0;
+    #pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+        const int q = tid + u * T;
+        if (q >= np) continue;
+        LineP& p = P[u];
+        p.x = S.x[q]; p.v = S.vx[q];
+        p.s = PState{S.sxx[par][q], S.syy[par][q], S.szz[par][q], S.sxy[par][q],
+                     S.exx[q], S.eyy[q], S.exy[q], S.rho[par][q], S.vsc[par][q]};
+        p.vol = S.vol[par][q];
+        p.mass = REINIT ? 0.0f : S.mass[q];
+        p.Ep = S.E ? S.E[q] : -1.0f;
+        p.pid = S.pid[q];
+        p.mat = S.mat[q];
+        p.code = S.pvc ? S.pvc[2 * q] : 0;
+        p.e = locate_axis(p.x, S.hx, nx);
+        if (p.e < 0 || p.e >= nx) { status |= ST_OUT_OF_MESH; p.e = nx; }
+    }
+    for (int i = tid; i < nn; i += T) { W.vb[i] = S.nvbx[i]; W.a[i] = 0.0f; }
+    bool rebuild = true;
+    #pragma unroll 1
+    for (int t = 0; t < nsteps; ++t) {
+        if (rebuild) {
+            // counting sort by element, each element's entries by original index
+            for (int i = tid; i <= nx; i += T) W.cnt[i] = 0;
+            if (tid == 0) s_carry = 0;
+            __syncthreads();
+            #pragma unroll
+            for (int u = 0; u < PPT; ++u)
+                if (tid + u * T < np) P[u].slot = atomicAdd(&W.cnt[P[u].e], 1);
+            __syncthreads();
+            #pragma unroll 1
+            for (int base = 0; base <= nx; base += T) {   // exclusive scan of the counts
+                const int i = base + tid, lane = tid & 31;
+                const int v = i <= nx ? W.cnt[i] : 0;
+                int x = v;
+                #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (lane == 31) s_warp[tid >> 5] = x;
+                __syncthreads();
+                int before = s_carry;
+                for (int w = 0; w < (tid >> 5); ++w) before += s_warp[w];
+                if (i <= nx) W.start[i] = before + x - v;
+                __syncthreads();
+                if (tid == T - 1) s_carry = before + x;
+            }
+            if (tid == 0) W.start[nx + 1] = np;
+            __syncthreads();
+            #pragma unroll
+            for (int u = 0; u < PPT; ++u)
+                if (tid + u * T < np) W.pid[W.start[P[u].e] + P[u].slot] = P[u].pid;
+            __syncthreads();
+            #pragma unroll
+            for (int u = 0; u < PPT; ++u)
+                if (tid + u * T < np) {
+                    LineP& p = P[u];
+                    int rank = 0;
+                    for (int j = W.start[p.e]; j < W.start[p.e + 1]; ++j) rank += W.pid[j] < p.pid;
+                    p.slot = W.start[p.e] + rank;
+                    const LineElem g = line_elem(p.e, S.hx);
+                    p.gc = g.c; p.gr = g.r; p.x0 = g.x0; p.x1 = g.x1;
+                }
+            for (int e = tid; e < nx; e += T) {
+                const LineElem g = line_elem(e, S.hx);
+                W.V0[e] = fdv(fs(g.x1, g.x0), (float)(W.start[e + 1] - W.start[e]));
+            }
+            __syncthreads();
+            #pragma unroll
+            for (int u = 0; u < PPT; ++u)
+                if (tid + u * T < np) W.pid[P[u].slot] = P[u].pid;
+            __syncthreads();
+        }
+        if (tape.P) {
+            float* o = tape.P + (size_t)t * 9 * np;
+            #pragma unroll
+            for (int u = 0; u < PPT; ++u)
+                if (tid + u * T < np) {
+                    const LineP& p = P[u];
+                    const float v[9] = {p.x, p.v, p.s.sxx, p.s.syy, p.s.szz, p.s.sxy, p.s.rho, p.vol, p.s.vsc};
+                    #pragma unroll
+                    for (int k = 0; k < 9; ++k) o[(size_t)k * np + p.slot] = v[k];
+                    tape.pid[(size_t)t * np + p.slot] = p.pid;
+                }
+            for (int i = tid; i < nx + 2; i += T) tape.cs[(size_t)t * (nx + 2) + i] = W.start[i];
+        }
+        // mass and momentum of the nodes
+        #pragma unroll
+        for (int u = 0; u < PPT; ++u)
+            if (tid + u * T < np) {
+                LineP& p = P[u];
+                const float xi = natural(p.x, p.gc, p.gr);
+                p.N0 = shape2(0, xi);
+                p.N1 = shape2(1, xi);
+                p.mp = REINIT ? fm(p.e < nx ? W.V0[p.e] : 0.0f, p.s.rho) : p.mass;
+                const float mv = fm(p.mp, p.v);
+                W.c[p.slot] = fm(p.mp, p.N0);
+                W.c[np + p.slot] = fm(p.mp, p.N1);
+                W.c[2 * np + p.slot] = fm(p.N0, mv);
+                W.c[3 * np + p.slot] = fm(p.N1, mv);
+            }
+        __syncthreads();
+        for (int i = tid; i < nn; i += T) {
+            float m, mom;
+            line_node_sums(W, np, nx, i, m, mom);
+            mom = flush(mom);
+            float v = m == 0.0f ? W.vb[i] : fdv(mom, m);
+            v = flush(v);
+            const int c = cons0(S, i);
+            if (c) v = S.cons_vel[c - 1];
+            W.m[i] = m;
+            W.va[i] = v;
+        }
+        __syncthreads();
+        // (USF) stress update; internal and external force contributions
+        auto stress = [&](LineP& p, const float* nv) {
+            const int e = min(p.e, nx - 1);
+            const float r = flush(fa(fm(dshape2(0, p.gr), nv[e]), fm(dshape2(1, p.gr), nv[e + 1])));
+            const float dvol = fm(S.dt, r);
+            const float f = strain_stress_update(S.mats[p.mat], p.Ep, S.dt, r, 0.0f, 0.0f, dvol, p.s);
+            p.vol = fm(REINIT ? W.V0[e] : p.vol, f);
+        };
+        #pragma unroll
+        for (int u = 0; u < PPT; ++u)
+            if (tid + u * T < np) {
+                LineP& p = P[u];
+                const float Vs = REINIT ? W.V0[min(p.e, nx - 1)] : p.vol;
+                if (!USL) stress(p, W.va);
+                const float mg = fm(p.mp, S.gx), vs = fm(-(USL ? Vs : p.vol), p.s.sxx);
+                W.c[p.slot] = fm(p.N0, mg);
+                W.c[np + p.slot] = fm(p.N1, mg);
+                W.c[2 * np + p.slot] = fm(vs, dshape2(0, p.gr));
+                W.c[3 * np + p.slot] = fm(vs, dshape2(1, p.gr));
+            }
+        __syncthreads();
+        for (int i = tid; i < nn; i += T) {
+            float fext, fint;
+            line_node_sums(W, np, nx, i, fext, fint);
+            if (S.cnf_ptr) {
+                const float time = step_time(step0 + t, S.dt);
+                #pragma unroll 1
+                for (int j = S.cnf_ptr[i]; j < S.cnf_ptr[i + 1]; ++j)
+                    fext = fa(fext, fm(fn_value(S, S.cnf_fn[j], time), S.cnf_val[j]));
+            }
+            float a = nan_to_num(fdv(fa(fa(fint, fext), 0.0f), W.m[i]));
+            float v = fa(W.va[i], fm(a, S.dt));
+            const int c = cons0(S, i);
+            if (c) {
+                v = S.cons_vel[c - 1];
+                a = 0.0f;
+            }
+            W.vb[i] = flush(v);
+            W.a[i] = flush(a);
+        }
+        __syncthreads();
+        if (tape.P) {
+            float* o = tape.N + (size_t)t * 4 * nn;
+            for (int i = tid; i < nn; i += T) {
+                o[i] = W.m[i];
+                o[nn + i] = W.va[i];
+                o[2 * nn + i] = W.vb[i];
+                o[3 * nn + i] = W.a[i];
+            }
+        }
+        bool moved = false;
+        #pragma unroll
+        for (int u = 0; u < PPT; ++u)
+            if (tid + u * T < np) {
+                LineP& p = P[u];
+                const int e = min(p.e, nx - 1);
+                const float vh = fa(fm(p.N0, W.vb[e]), fm(p.N1, W.vb[e + 1]));
+                const float ah = fa(fm(p.N0, W.a[e]), fm(p.N1, W.a[e + 1]));
+                float v = S.velocity_update ? vh : fa(p.v, fm(ah, S.dt));
+                if (p.code) v = S.pvc_vel[p.code - 1];
+                p.v = v;
+                p.x = fa(p.x, fm(vh, S.dt));
+                if (USL) stress(p, W.vb);
+                if (!(p.e < nx && p.x >= p.x0 && p.x < p.x1)) {
+                    int ne = locate_axis(p.x, S.hx, nx);
+                    if (ne < 0 || ne >= nx) { status |= ST_OUT_OF_MESH; ne = nx; }
+                    moved = moved || ne != p.e;
+                    p.e = ne;
+                }
+            }
+        rebuild = __syncthreads_or(moved) != 0;
+    }
+    const int o = (par + nsteps) & 1;
+    #pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+        const int q = tid + u * T;
+        if (q >= np) continue;
+        const LineP& p = P[u];
+        S.x[q] = p.x; S.vx[q] = p.v;
+        S.sxx[o][q] = p.s.sxx; S.syy[o][q] = p.s.syy; S.szz[o][q] = p.s.szz; S.sxy[o][q] = p.s.sxy;
+        S.exx[q] = p.s.exx; S.eyy[q] = p.s.eyy; S.exy[q] = p.s.exy;
+        S.rho[o][q] = p.s.rho; S.vsc[o][q] = p.s.vsc; S.vol[o][q] = p.vol;
+    }
+    for (int i = tid; i < nn; i += T) {
+        S.nm[i] = W.m[i];
+        S.nvax[i] = W.va[i];
+        S.nvbx[i] = W.vb[i];
+        S.nax[i] = W.a[i];
+    }
+    if (status) atomicOr(&ctl->status, status);
+}
+
+template <bool REINIT, bool USL>
+cudaError_t launch_line_steps(const SimDev& S, int par, int step0, int n, Control* ctl, const LineTape& tape,
+                              cudaStream_t s) {
+    const size_t bytes = line_shared_bytes(S.np, S.nx);
+    // a thread per particle and node up to 1024 threads, two particles a thread above
+    const int want = S.np > S.nx ? S.np : S.nx + 1;
+    const int T = want >= 1024 ? 1024 : (want + 31) / 32 * 32;
+    auto go = [&](auto kernel) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+        kernel<<<1, T, bytes, s>>>(S, par, step0, n, ctl, tape);
+        return cudaGetLastError();
+    };
+    return S.np <= T ? go(k_line_steps<REINIT, USL, 1>) : go(k_line_steps<REINIT, USL, 2>);
+}
+
 // Element of each storage slot: the bucket it was sorted into.
 __global__ void k_line_eid(const int* __restrict__ cstart, int nx, int* __restrict__ eid) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -248,7 +542,7 @@ int line_setup_volume(MpmHandle* h, cudaStream_t s) {
 
 // One step: re-sort by element, nodal kinematics, (USF) stress update, forces
 // and nodal update, G2P, (USL) stress update.
-int line_step(MpmHandle* h, cudaStream_t s, const LineTapeSlot* tape) {
+static int line_step(MpmHandle* h, cudaStream_t s, const LineTapeSlot* tape) {
     TRY(resort(h, s));
     const SimDev& S = h->hs;
     const int par = parity(h), nb = blocks(h->nx + 1), pb = blocks((int)h->np);
@@ -282,6 +576,40 @@ int line_step(MpmHandle* h, cudaStream_t s, const LineTapeSlot* tape) {
     }
     h->step++;
     h->needs_resort = true;
+    return MPM_OK;
+}
+
+// n steps in one launch (bars of at most LINE_FUSED_MAX particles and elements).
+static int line_steps_fused(MpmHandle* h, int n, cudaStream_t s, const LineTapeSlot* tape) {
+    const int par = parity(h);
+    const LineTape tp = tape ? LineTape{tape->p[0], tape->pid, tape->cs, tape->n[0]} : LineTape{};
+    const int step = (int)h->step;
+    cudaError_t e;
+    if (h->reinit)
+        e = h->usl ? launch_line_steps<true, true>(h->hs, par, step, n, h->ctl, tp, s)
+                   : launch_line_steps<true, false>(h->hs, par, step, n, h->ctl, tp, s);
+    else
+        e = h->usl ? launch_line_steps<false, true>(h->hs, par, step, n, h->ctl, tp, s)
+                   : launch_line_steps<false, false>(h->hs, par, step, n, h->ctl, tp, s);
+    CK(h, e);
+    h->step += n;
+    h->resorts += n;
+    h->needs_resort = true;
+    return MPM_OK;
+}
+
+int line_steps(MpmHandle* h, int n, cudaStream_t s, const LineTapeSlot* tape) {
+    if (n > 0 && line_fused(h)) return line_steps_fused(h, n, s, tape);
+    LineTapeSlot slot;
+    if (tape) slot = *tape;
+    for (int t = 0; t < n; ++t) {
+        TRY(line_step(h, s, tape ? &slot : nullptr));
+        if (!tape) continue;
+        for (float*& p : slot.p) p += 9 * (size_t)h->np;
+        slot.pid += h->np;
+        slot.cs += h->nx + 2;
+        for (float*& p : slot.n) p += 4 * (size_t)h->nn;
+    }
     return MPM_OK;
 }
 

@@ -22,6 +22,7 @@
 // keeps from the previous step is not differentiated.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "mpm_device.cuh"
@@ -40,7 +41,7 @@ enum { LS_G, LS_H, LS_R, LS_M, LS_X, LS_V, LS_N };
 enum { LNS_F, LNS_M, LNS_VA, LNS_P, LNS_N };
 
 struct LineAdjoint {
-    int T = 0;                 // recorded steps
+    int T = 0, cap = 0;        // recorded steps; steps the tape arrays hold
     int64_t np = 0, nn = 0;
     int nx = 0;
     uint64_t gen = 0;
@@ -183,18 +184,14 @@ __device__ __forceinline__ float start_volume(const LineStep& A, int q, int e) {
 }
 
 // pass 0 (USL): the stress update after G2P used the updated velocities
-__global__ void k_lrev0(const __grid_constant__ LineStep A) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.np) return;
+__device__ __forceinline__ void lrev0(const LineStep& A, int q) {
     const int o = A.pid[q], e = A.eid[q];
     const float sb[4] = {A.L[LA_SXX][o], A.L[LA_SYY][o], A.L[LA_SZZ][o], A.L[LA_SXY][o]};
     A.sc[LS_R][q] = rev_stress(A, q, o, e, start_volume(A, q, e), A.vB, sb, 0.0f);
 }
 
 // pass 1: G2P (particle.py:208-247)
-__global__ void k_lrev1(const __grid_constant__ LineStep A) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.np) return;
+__device__ __forceinline__ void lrev1(const LineStep& A, int q) {
     const int o = A.pid[q], e = A.eid[q];
     const Elem g = elem_of(A, e);
     float N0, N1, d0, d1;
@@ -213,9 +210,7 @@ __global__ void k_lrev1(const __grid_constant__ LineStep A) {
 
 // pass 2: transposed G2P (and USL strain-rate gather), reverse nodal update
 // (element.py:305-329)
-__global__ void k_lrev2(const __grid_constant__ LineStep A) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > A.nx) return;
+__device__ __forceinline__ void lrev2(const LineStep& A, int i) {
     float vbb = 0.0f, ab = 0.0f;
     for_node(A, i, [&](int q, int e, int k) {
         const Elem g = elem_of(A, e);
@@ -243,9 +238,7 @@ __global__ void k_lrev2(const __grid_constant__ LineStep A) {
 
 // pass 3: forces (element.py:236-268, 548-600) and the USF stress update
 template <bool USL>
-__global__ void k_lrev3(const __grid_constant__ LineStep A) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.np) return;
+__device__ __forceinline__ void lrev3(const LineStep& A, int q) {
     const int o = A.pid[q], e = A.eid[q];
     const Elem g = elem_of(A, e);
     float N0, N1, d0, d1;
@@ -282,9 +275,7 @@ __global__ void k_lrev3(const __grid_constant__ LineStep A) {
 
 // pass 4: (USF) transposed strain-rate gather, reverse nodal velocity
 // (element.py:191-202, 331-334)
-__global__ void k_lrev4(const __grid_constant__ LineStep A) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > A.nx) return;
+__device__ __forceinline__ void lrev4(const LineStep& A, int i) {
     float vab = A.ns[LNS_VA][i];
     if (!A.usl) {
         for_node(A, i, [&](int q, int e, int k) {
@@ -304,9 +295,7 @@ __global__ void k_lrev4(const __grid_constant__ LineStep A) {
 }
 
 // pass 5: mass and momentum (element.py:122-189) and m = V0 rho
-__global__ void k_lrev5(const __grid_constant__ LineStep A) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= A.np) return;
+__device__ __forceinline__ void lrev5(const LineStep& A, int q) {
     const int o = A.pid[q], e = A.eid[q];
     const Elem g = elem_of(A, e);
     float N0, N1, d0, d1;
@@ -320,6 +309,86 @@ __global__ void k_lrev5(const __grid_constant__ LineStep A) {
     A.L[LA_X][o] = fa(A.sc[LS_X][q], fa(fm(m, DM), fm(fm(m, v), DP)));
     A.L[LA_V][o] = fa(A.sc[LS_V][q], fm(m, SP));
     if (A.reinit) A.L[LA_RHO][o] = fa(A.L[LA_RHO][o], fm(g.V0, mb));   // m = V0 rho
+}
+
+// The passes as kernels of their own (a thread per particle or node).
+template <class F>
+__device__ __forceinline__ void lrev_index(int n, F&& f) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) f(i);
+}
+__global__ void k_lrev0(const __grid_constant__ LineStep A) { lrev_index(A.np, [&](int q) { lrev0(A, q); }); }
+__global__ void k_lrev1(const __grid_constant__ LineStep A) { lrev_index(A.np, [&](int q) { lrev1(A, q); }); }
+__global__ void k_lrev2(const __grid_constant__ LineStep A) { lrev_index(A.nx + 1, [&](int i) { lrev2(A, i); }); }
+template <bool USL>
+__global__ void k_lrev3(const __grid_constant__ LineStep A) { lrev_index(A.np, [&](int q) { lrev3<USL>(A, q); }); }
+__global__ void k_lrev4(const __grid_constant__ LineStep A) { lrev_index(A.nx + 1, [&](int i) { lrev4(A, i); }); }
+__global__ void k_lrev5(const __grid_constant__ LineStep A) { lrev_index(A.np, [&](int q) { lrev5(A, q); }); }
+
+// The arrays of recorded step t.
+__host__ __device__ inline void set_line_step(LineStep& A, const float* P, const int* pid, const int* cs,
+                                              const float* N, size_t t) {
+    const size_t np = A.np, nn = (size_t)A.nx + 1;
+    P += t * LP_N * np;
+    A.x = P + LP_X * np; A.v = P + LP_V * np;
+    A.sxx = P + LP_SXX * np; A.syy = P + LP_SYY * np; A.szz = P + LP_SZZ * np;
+    A.sxy = P + LP_SXY * np; A.rho = P + LP_RHO * np;
+    A.vol = P + LP_VOL * np; A.vsc = P + LP_VSC * np;
+    A.pid = pid + t * np;
+    A.cs = cs + t * (nn + 1);
+    N += t * LN_N * nn;
+    A.M = N + LN_M * nn; A.vA = N + LN_VA * nn;
+    A.vB = N + LN_VB * nn; A.a = N + LN_A * nn;
+}
+
+// All reverse steps in one CTA (bars the forward runs in one CTA): the
+// adjoints and scratch live in shared memory and the passes of a step are
+// separated by barriers, where as kernels they were seven dependent launches
+// a step.  The per-element pass runs first as in the separate kernels.
+template <bool USL>
+__global__ void __launch_bounds__(1024)
+k_lrev_steps(const __grid_constant__ LineStep A0, const float* P, const int* pid, const int* cs, const float* N,
+             int T) {
+    extern __shared__ float s_f[];
+    __shared__ LineStep A;
+    const int np = A0.np, nn = A0.nx + 1, tid = threadIdx.x, B = blockDim.x;
+    int* eid = reinterpret_cast<int*>(s_f + (size_t)(LA_N + LS_N) * np + (size_t)LNS_N * nn);
+    if (tid == 0) {
+        A = A0;
+        for (int k = 0; k < LA_N; ++k) A.L[k] = s_f + (size_t)k * np;
+        for (int k = 0; k < LS_N; ++k) A.sc[k] = s_f + (size_t)(LA_N + k) * np;
+        for (int k = 0; k < LNS_N; ++k) A.ns[k] = s_f + (size_t)(LA_N + LS_N) * np + (size_t)k * nn;
+        A.eid = eid;
+    }
+    for (int i = tid; i < LA_N * np; i += B) s_f[i] = A0.L[0][i];   // (the LA_N arrays are one block)
+    __syncthreads();
+    #pragma unroll 1
+    for (int t = T - 1; t >= 0; --t) {
+        if (tid == 0) set_line_step(A, P, pid, cs, N, t);
+        __syncthreads();
+        for (int e = tid; e < A.nx; e += B)
+            for (int q = A.cs[e]; q < A.cs[e + 1]; ++q) eid[q] = e;
+        __syncthreads();
+        // (passes 0 and 1 work on the same particle: one thread takes both)
+        for (int q = tid; q < np; q += B) {
+            if (USL) lrev0(A, q);
+            lrev1(A, q);
+        }
+        __syncthreads();
+        for (int i = tid; i < nn; i += B) lrev2(A, i);
+        __syncthreads();
+        for (int q = tid; q < np; q += B) lrev3<USL>(A, q);
+        __syncthreads();
+        for (int i = tid; i < nn; i += B) lrev4(A, i);
+        __syncthreads();
+        for (int q = tid; q < np; q += B) lrev5(A, q);
+        __syncthreads();
+    }
+    for (int i = tid; i < LA_N * np; i += B) A0.L[0][i] = s_f[i];
+}
+
+inline size_t lrev_shared_bytes(int np, int nx) {
+    return 4 * ((size_t)(LA_N + LS_N + 1) * np + (size_t)LNS_N * (nx + 1));
 }
 
 // A float per particle from storage to original order.
@@ -375,49 +444,58 @@ int line_record(MpmHandle* h, int nsteps, cudaStream_t s) {
     if (!h->initialized) return fail(h, MPM_ERR_STATE, "initialize first");
     if (nsteps < 1) return fail(h, MPM_ERR_INVALID, "nsteps must be >= 1");
     if (h->np <= 0) return fail(h, MPM_ERR_STATE, "no particles");
-    line_adjoint_free(h);
-    LineAdjoint* a = new LineAdjoint();
-    h->line_adj = a;
-    a->T = nsteps;
-    a->np = h->np;
-    a->nn = h->nn;
-    a->nx = h->nx;
     const size_t np = (size_t)h->np, nn = (size_t)h->nn, T = (size_t)nsteps;
     const size_t bytes = T * (np * (LP_N + 1) + (size_t)(h->nx + 2) + nn * LN_N) * 4;
-    if (bytes > ((size_t)64 << 30))
-        return fail(h, MPM_ERR_NOMEM, "a 1-D recording of %d steps needs %zu bytes", nsteps, bytes);
-    TRY(line_alloc(h, a, &a->P, T * LP_N * np));
-    TRY(line_alloc(h, a, &a->pid, T * np));
-    TRY(line_alloc(h, a, &a->cs, T * (size_t)(h->nx + 2)));
-    TRY(line_alloc(h, a, &a->N, T * LN_N * nn));
-    TRY(line_alloc(h, a, &a->mat0, np));
-    TRY(line_alloc(h, a, &a->eid, np));
-    TRY(line_alloc(h, a, &a->L, (size_t)LA_N * np));
-    TRY(line_alloc(h, a, &a->sc, (size_t)LS_N * np));
-    TRY(line_alloc(h, a, &a->ns, (size_t)LNS_N * nn));
+    // the arrays of the last recording serve the next one of the same bar that
+    // is no longer (a training loop records the same run again and again)
+    LineAdjoint* a = h->line_adj;
+    if (a && (a->np != h->np || a->nn != h->nn || a->cap < nsteps)) {
+        line_adjoint_free(h);
+        a = nullptr;
+    }
+    if (a) {
+        a->valid = false;
+        a->T = nsteps;
+    } else {
+        a = h->line_adj = new LineAdjoint();
+        a->T = nsteps;
+        a->np = h->np;
+        a->nn = h->nn;
+        a->nx = h->nx;
+        if (bytes > ((size_t)64 << 30))
+            return fail(h, MPM_ERR_NOMEM, "a 1-D recording of %d steps needs %zu bytes", nsteps, bytes);
+        TRY(line_alloc(h, a, &a->P, T * LP_N * np));
+        TRY(line_alloc(h, a, &a->pid, T * np));
+        TRY(line_alloc(h, a, &a->cs, T * (size_t)(h->nx + 2)));
+        TRY(line_alloc(h, a, &a->N, T * LN_N * nn));
+        TRY(line_alloc(h, a, &a->mat0, np));
+        TRY(line_alloc(h, a, &a->eid, np));
+        TRY(line_alloc(h, a, &a->L, (size_t)LA_N * np));
+        TRY(line_alloc(h, a, &a->sc, (size_t)LS_N * np));
+        TRY(line_alloc(h, a, &a->ns, (size_t)LNS_N * nn));
+        a->cap = nsteps;
+    }
     const PSet& p = h->ps[h->pcur];
     if (np > 0) k_lmat0<<<lblocks((int64_t)np), LA_THREADS, 0, s>>>(p.mat, p.pid, (int)np, 1, a->mat0);
     if (!h->reinit) {   // solve semantics: the constant mass
-        TRY(line_alloc(h, a, &a->mass0, np));
+        if (!a->mass0) TRY(line_alloc(h, a, &a->mass0, np));
         if (np > 0) k_lscatter<<<lblocks((int64_t)np), LA_THREADS, 0, s>>>(p.mass, p.pid, (int)np, a->mass0);
     }
     if (h->has_pvc) {
-        TRY(line_alloc(h, a, &a->pvc0, np));
+        if (!a->pvc0) TRY(line_alloc(h, a, &a->pvc0, np));
         if (np > 0) k_lmat0<<<lblocks((int64_t)np), LA_THREADS, 0, s>>>(p.pvc, p.pid, (int)np, 2, a->pvc0);
     }
     CK(h, cudaGetLastError());
     if (h->has_E) {
-        TRY(line_alloc(h, a, &a->E0, np));
+        if (!a->E0) TRY(line_alloc(h, a, &a->E0, np));
         TRY(gather_field(h, MPM_FIELD_YOUNGS_MODULUS, a->E0, s));
     }
-    for (int t = 0; t < nsteps; ++t) {
-        LineTapeSlot slot;
-        for (int k = 0; k < LP_N; ++k) slot.p[k] = a->P + ((size_t)t * LP_N + k) * np;
-        slot.pid = a->pid + (size_t)t * np;
-        slot.cs = a->cs + (size_t)t * (h->nx + 2);
-        for (int k = 0; k < LN_N; ++k) slot.n[k] = a->N + ((size_t)t * LN_N + k) * nn;
-        TRY(line_step(h, s, &slot));
-    }
+    LineTapeSlot slot;
+    for (int k = 0; k < LP_N; ++k) slot.p[k] = a->P + (size_t)k * np;
+    slot.pid = a->pid;
+    slot.cs = a->cs;
+    for (int k = 0; k < LN_N; ++k) slot.n[k] = a->N + (size_t)k * nn;
+    TRY(line_steps(h, nsteps, s, &slot));
     TRY(read_ctl(h, s));
     int st = h->h_ctl->status;
     TRY(check_status(h, st));
@@ -458,23 +536,26 @@ int line_adjoint(MpmHandle* h, const float* dl_dloc, const float* dl_dvel, float
     A.ncons = h->d_ncons;
     A.mats = h->d_mats;
     A.mat0 = a->mat0;
-    A.E0 = a->E0;
-    A.pvc0 = a->pvc0;
+    A.E0 = h->has_E ? a->E0 : nullptr;
+    A.pvc0 = h->has_pvc ? a->pvc0 : nullptr;
     for (int k = 0; k < LA_N; ++k) A.L[k] = L + (size_t)k * np;
     for (int k = 0; k < LS_N; ++k) A.sc[k] = a->sc + (size_t)k * np;
     for (int k = 0; k < LNS_N; ++k) A.ns[k] = a->ns + (size_t)k * a->nn;
+    if (line_fused(h)) {
+        const size_t bytes = lrev_shared_bytes((int)np, a->nx);
+        const int want = (int)std::max<int64_t>(np, a->nx + 1), T = want >= 1024 ? 1024 : (want + 31) / 32 * 32;
+        auto go = [&](auto kernel) {
+            const cudaError_t e =
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e != cudaSuccess) return e;
+            kernel<<<1, T, bytes, s>>>(A, a->P, a->pid, a->cs, a->N, a->T);
+            return cudaGetLastError();
+        };
+        CK(h, A.usl ? go(k_lrev_steps<true>) : go(k_lrev_steps<false>));
+    }
     const int pb = lblocks(np), nb = lblocks(a->nx + 1);
-    for (int t = a->T - 1; t >= 0; --t) {
-        const float* P = a->P + (size_t)t * LP_N * np;
-        A.x = P + LP_X * np; A.v = P + LP_V * np;
-        A.sxx = P + LP_SXX * np; A.syy = P + LP_SYY * np; A.szz = P + LP_SZZ * np;
-        A.sxy = P + LP_SXY * np; A.rho = P + LP_RHO * np;
-        A.vol = P + LP_VOL * np; A.vsc = P + LP_VSC * np;
-        A.pid = a->pid + (size_t)t * np;
-        A.cs = a->cs + (size_t)t * (a->nx + 2);
-        const float* N = a->N + (size_t)t * LN_N * a->nn;
-        A.M = N + LN_M * a->nn; A.vA = N + LN_VA * a->nn;
-        A.vB = N + LN_VB * a->nn; A.a = N + LN_A * a->nn;
+    for (int t = a->T - 1; t >= 0 && !line_fused(h); --t) {
+        set_line_step(A, a->P, a->pid, a->cs, a->N, t);
         CK(h, launch_line_eid(A.cs, a->nx, a->eid, s));
         if (A.usl) k_lrev0<<<pb, LA_THREADS, 0, s>>>(A);
         k_lrev1<<<pb, LA_THREADS, 0, s>>>(A);
