@@ -133,46 +133,73 @@ int clear_status(MpmHandle* h, cudaStream_t s) {
     return MPM_OK;
 }
 
+// The arguments of a re-sort of h: its current arrays into the other buffer set.
+SortJob sort_job(MpmHandle* h) {
+    SortScratch& w = h->sw;
+    PSet& src = h->ps[h->pcur];
+    PSet& dst = h->ps[h->pcur ^ 1];
+    SortJob J{};
+    J.np = (int)h->np;
+    J.nx = h->nx;
+    J.ny = h->ny;
+    J.hx = h->hx;
+    J.hy = h->hy;
+    J.x = src.x;
+    J.y = src.y;
+    J.count = w.count;
+    J.key = w.key;
+    J.rank = w.rank;
+    J.perm = w.perm;
+    J.start = h->cstart[h->cs_cur ^ 1];
+    J.cflag = h->cflag;
+    J.ctl = h->ctl;
+    std::vector<float**> a = movable_f32(h, src, false), b = movable_f32(h, dst, false);
+    J.nf = (int)a.size();
+    for (int i = 0; i < J.nf; ++i) {
+        J.src[i] = reinterpret_cast<const uint32_t*>(*a[i]);
+        J.dst[i] = reinterpret_cast<uint32_t*>(*b[i]);
+    }
+    J.mat_src = src.mat;
+    J.mat_dst = dst.mat;
+    if (h->has_pvc) {
+        J.pvc_src = reinterpret_cast<const uint16_t*>(src.pvc);
+        J.pvc_dst = reinterpret_cast<uint16_t*>(dst.pvc);
+    }
+    if (h->has_trac) {
+        J.trfn_src = reinterpret_cast<const uint16_t*>(src.tr_fn);
+        J.trfn_dst = reinterpret_cast<uint16_t*>(dst.tr_fn);
+        J.trtau_src = reinterpret_cast<const float2*>(src.tr_tau);
+        J.trtau_dst = reinterpret_cast<float2*>(dst.tr_tau);
+    }
+    return J;
+}
+
+// The sorted buffers become the current ones (the device descriptor is the
+// caller's to update).
+void sort_done(MpmHandle* h) {
+    h->pcur ^= 1;
+    h->cs_cur ^= 1;
+    bind_particles(h);
+    drop_graphs(h);   // the step graphs hold the descriptor by value
+    h->needs_resort = false;
+    h->resorts++;
+}
+
 // Stable re-sort of the particles by current cell.
 int resort(MpmHandle* h, cudaStream_t s) {
     if (h->np <= 0) {
         h->needs_resort = false;
         return MPM_OK;
     }
-    const int np = (int)h->np, nb = h->ncell + 1;
     adjoint_note_resort(h);
-    SortScratch& w = h->sw;
-    CK(h, cudaMemsetAsync(w.count, 0, sizeof(int) * nb, s));
-    CK(h, cudaMemsetAsync(w.cursor, 0, sizeof(int) * nb, s));
-    CK(h, launch_resort_keys(h->ds, np, h->nx, h->ny, h->hx, h->hy, w, h->ctl, s));
-    int* start = h->cstart[h->cs_cur ^ 1];
-    CK(h, launch_exclusive_scan(w.count, start, nb, w.block_sums, s));
-    CK(h, launch_resort_place(np, start, w, s));
-    PSet& src = h->ps[h->pcur];
-    PSet& dst = h->ps[h->pcur ^ 1];
-    if (h->ndim == 1) CK(h, launch_line_segsort(nb, start, w.perm, src.pid, s));
-    else CK(h, launch_resort_segsort(nb, start, w, s));
-    std::vector<float**> a = movable_f32(h, src, false), b = movable_f32(h, dst, false);
-    for (size_t i = 0; i < a.size(); ++i)
-        CK(h, launch_gather_u32(reinterpret_cast<const uint32_t*>(*a[i]),
-                                reinterpret_cast<uint32_t*>(*b[i]), w.perm, np, s));
-    CK(h, launch_gather_u8(src.mat, dst.mat, w.perm, np, s));
-    if (h->has_pvc) CK(h, launch_gather_pair_u8(src.pvc, dst.pvc, w.perm, np, s));
-    if (h->has_trac) {
-        CK(h, launch_gather_pair_u8(reinterpret_cast<const uint8_t*>(src.tr_fn),
-                                    reinterpret_cast<uint8_t*>(dst.tr_fn), w.perm, np, s));
-        CK(h, launch_gather_pair_u32(reinterpret_cast<const uint32_t*>(src.tr_tau),
-                                     reinterpret_cast<uint32_t*>(dst.tr_tau), w.perm, np, s));
-    }
-    h->pcur ^= 1;
-    h->cs_cur ^= 1;
-    CK(h, cudaMemsetAsync(h->cflag, 0, h->ncell, s));
-    if (h->ndim == 1) CK(h, launch_line_eid(start, h->nx, h->line_eid, s));
-    bind_particles(h);
-    drop_graphs(h);   // the step graphs hold the descriptor by value
+    const SortJob J = sort_job(h);
+    const bool line = h->ndim == 1;
+    CK(h, launch_sort_order(J, h->sw.block_sums, !line, s));
+    if (line) CK(h, launch_line_segsort(h->ncell + 1, J.start, J.perm, h->ps[h->pcur].pid, s));
+    CK(h, launch_sort_move(J, s));
+    if (line) CK(h, launch_line_eid(J.start, h->nx, h->line_eid, s));
+    sort_done(h);
     CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
-    h->needs_resort = false;
-    h->resorts++;
     return MPM_OK;
 }
 
@@ -318,6 +345,7 @@ int alloc_particles(MpmHandle* h, int64_t n) {
     }
     TRY(dalloc(h, &h->passive, 5 * n));
     TRY(dalloc(h, &h->sw.key, n));
+    TRY(dalloc(h, &h->sw.rank, n));
     TRY(dalloc(h, &h->sw.perm, n));
     if (h->ndim == 1) TRY(dalloc(h, &h->line_eid, n));
     const size_t nsnap = movable_f32(h, h->ps[0], true).size();
@@ -339,8 +367,9 @@ void free_particles(MpmHandle* h) {
     dfree(h, h->passive);
     h->passive = nullptr;
     dfree(h, h->sw.key);
+    dfree(h, h->sw.rank);
     dfree(h, h->sw.perm);
-    h->sw.key = h->sw.perm = nullptr;
+    h->sw.key = h->sw.rank = h->sw.perm = nullptr;
     dfree(h, h->line_eid);
     h->line_eid = nullptr;
     for (float* f : h->snap_f) dfree(h, f);
@@ -359,11 +388,6 @@ int to_device(MpmHandle* h, const void* src, size_t bytes, int on_device, cudaSt
     TRY(ensure_stage(h, bytes));
     CK(h, cudaMemcpyAsync(h->stage, src, bytes, cudaMemcpyHostToDevice, s));
     *dsrc = h->stage;
-    return MPM_OK;
-}
-
-int set_ptr_table(MpmHandle* h, const std::vector<float*>& ptrs, cudaStream_t s) {
-    CK(h, cudaMemcpyAsync(h->d_ptrs, ptrs.data(), sizeof(float*) * ptrs.size(), cudaMemcpyHostToDevice, s));
     return MPM_OK;
 }
 
@@ -415,19 +439,19 @@ int passive_slot(int field, int c) {
     return -1;
 }
 
-int copy_passive(MpmHandle* h, int field, float* aos, bool to_aos, cudaStream_t s) {
-    for (int c = 0; c < 6; ++c) {
-        const int slot = passive_slot(field, c);
-        if (slot < 0) continue;
-        float* pas = h->passive + slot;
-        if (to_aos)
-            CK(h, cudaMemcpy2DAsync(aos + c, 6 * sizeof(float), pas, 5 * sizeof(float), sizeof(float),
-                                    h->np, cudaMemcpyDeviceToDevice, s));
-        else
-            CK(h, cudaMemcpy2DAsync(pas, 5 * sizeof(float), aos + c, 6 * sizeof(float), sizeof(float),
-                                    h->np, cudaMemcpyDeviceToDevice, s));
+FieldMap field_map(MpmHandle* h, int field, const float* aos) {
+    FieldMap F{};
+    const std::vector<float*> c = comps(h, field);
+    F.ncomp = (int)c.size();
+    for (int k = 0; k < F.ncomp; ++k) {
+        F.comp[k] = c[k];
+        F.slot[k] = (signed char)(c[k] ? -1 : passive_slot(field, k));
     }
-    return MPM_OK;
+    F.np = (int)h->np;
+    F.pid = h->ps[h->pcur].pid;
+    F.passive = h->passive;
+    F.aos = const_cast<float*>(aos);
+    return F;
 }
 
 // Roll the block that started at step0 back to its snapshot and replay its B
@@ -639,7 +663,6 @@ int mpm_create(const MpmDesc* d, MpmHandle** out) {
     A(&h->cstart[1], (size_t)h->ncell + 2);
     A(&h->cflag, (size_t)h->ncell);
     A(&h->sw.count, (size_t)h->ncell + 1);
-    A(&h->sw.cursor, (size_t)h->ncell + 1);
     A(&h->sw.block_sums, (size_t)(h->ncell + 2) / 1024 + 3);
     A(&h->snap_cflag, (size_t)h->ncell);
     A(&h->snap_nvbx, (size_t)h->nn);
@@ -647,7 +670,6 @@ int mpm_create(const MpmDesc* d, MpmHandle** out) {
     A(&h->snap_ctl, 1);
     A(&h->ds, 1);
     A(&h->ctl, 1);
-    A(&h->d_ptrs, 16);
 #undef A
     cudaError_t e = cudaMallocHost(&h->h_ctl, sizeof(Control));
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_tile_counts, 2 * sizeof(int));
@@ -871,14 +893,9 @@ int keep_parity_data(MpmHandle* h, int64_t step) {
 // A float particle field (original order) from device memory `d` into the
 // current particle set, on stream s without waiting.
 int write_float_field(MpmHandle* h, int field, const float* d, cudaStream_t s) {
-    std::vector<float*> c = comps(h, field);
-    if (c.empty()) return fail(h, MPM_ERR_INVALID, "field %d is not writable", field);
-    const int nc = (int)c.size();
-    PSet& p = h->ps[h->pcur];
-    TRY(set_ptr_table(h, c, s));
-    CK(h, launch_gather_in(h->d_ptrs, nc, p.pid, (int)h->np, d, s));
-    if (field == MPM_FIELD_STRESS || field == MPM_FIELD_STRAIN)
-        TRY(copy_passive(h, field, const_cast<float*>(d), false, s));
+    const FieldMap F = field_map(h, field, d);
+    if (F.ncomp == 0) return fail(h, MPM_ERR_INVALID, "field %d is not writable", field);
+    CK(h, launch_field(F, true, s));
     if (field == MPM_FIELD_LOC && h->initialized) h->needs_resort = true;
     return MPM_OK;
 }
@@ -902,13 +919,10 @@ int gather_field(MpmHandle* h, int field, void* d, cudaStream_t s) {
     } else if (field == MPM_FIELD_MATERIAL_ID) {
         CK(h, launch_scatter_out_u8(p.mat, p.pid, (int)n, static_cast<int32_t*>(d), s));
     } else {
-        std::vector<float*> c = comps(h, field);
-        if (c.empty() || (field == MPM_FIELD_YOUNGS_MODULUS && !h->has_E))
+        const FieldMap F = field_map(h, field, static_cast<const float*>(d));
+        if (F.ncomp == 0 || (field == MPM_FIELD_YOUNGS_MODULUS && !h->has_E))
             return fail(h, MPM_ERR_INVALID, "field %d is not readable", field);
-        TRY(set_ptr_table(h, c, s));
-        CK(h, launch_scatter_out(h->d_ptrs, nc, p.pid, (int)n, static_cast<float*>(d), s));
-        if (field == MPM_FIELD_STRESS || field == MPM_FIELD_STRAIN)
-            TRY(copy_passive(h, field, static_cast<float*>(d), true, s));
+        CK(h, launch_field(F, false, s));
     }
     return MPM_OK;
 }
@@ -1044,8 +1058,8 @@ int mpm_set_tractions(MpmHandle* h, int n, const int64_t* pid, const int32_t* di
     CK(h, cudaMemcpyAsync(st, tau32.data(), sizeof(float) * 2 * np, cudaMemcpyHostToDevice, s));
     char* st8 = st + ((sizeof(float) * 2 * np + 63) / 64) * 64;
     CK(h, cudaMemcpyAsync(st8, fn.data(), 2 * np, cudaMemcpyHostToDevice, s));
-    CK(h, launch_gather_pair_u32(reinterpret_cast<const uint32_t*>(st), reinterpret_cast<uint32_t*>(p.tr_tau), p.pid, (int)np, s));
-    CK(h, launch_gather_pair_u8(reinterpret_cast<const uint8_t*>(st8), reinterpret_cast<uint8_t*>(p.tr_fn), p.pid, (int)np, s));
+    CK(h, launch_gather_pairs(reinterpret_cast<const float2*>(st), reinterpret_cast<float2*>(p.tr_tau), p.pid, (int)np, s));
+    CK(h, launch_gather_pairs(reinterpret_cast<const uint16_t*>(st8), reinterpret_cast<uint16_t*>(p.tr_fn), p.pid, (int)np, s));
     h->has_trac = true;
     bind_particles(h);
     drop_graphs(h);
@@ -1093,7 +1107,7 @@ int mpm_set_particle_velocity_constraints(MpmHandle* h, int n, const int64_t* pi
     PSet& p = h->ps[h->pcur];
     TRY(ensure_stage(h, 2 * np));
     CK(h, cudaMemcpyAsync(h->stage, code.data(), 2 * np, cudaMemcpyHostToDevice, s));
-    CK(h, launch_gather_pair_u8(static_cast<const uint8_t*>(h->stage), p.pvc, p.pid, (int)np, s));
+    CK(h, launch_gather_pairs(static_cast<const uint16_t*>(h->stage), reinterpret_cast<uint16_t*>(p.pvc), p.pid, (int)np, s));
     h->has_pvc = true;
     bind_particles(h);
     drop_graphs(h);

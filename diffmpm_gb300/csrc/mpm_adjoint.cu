@@ -85,7 +85,6 @@ struct AdjointState {
     int64_t seg_first = 0;     // first step of the segment being reversed
     float* lam[NLAM] = {};
     float* lam_tmp = nullptr;
-    float** d_lam = nullptr;
     float* pscr[NPS] = {};
     float* nscr[NNS] = {};
     int* cnt = nullptr;
@@ -159,14 +158,12 @@ void free_buffers(MpmHandle* h, AdjointState* a) {
     for (float*& p : a->pscr) { dfree(h, p); p = nullptr; }
     for (float*& p : a->nscr) { dfree(h, p); p = nullptr; }
     dfree(h, a->lam_tmp);
-    dfree(h, a->d_lam);
     dfree(h, a->cnt);
     dfree(h, a->mismatch);
     if (a->h_mismatch) cudaFreeHost(a->h_mismatch);
     a->mismatch = nullptr;
     a->h_mismatch = nullptr;
     a->lam_tmp = nullptr;
-    a->d_lam = nullptr;
     a->cnt = nullptr;
     a->np_alloc = -1;
     a->valid = false;
@@ -229,12 +226,9 @@ int ensure_adjoint_buffers(MpmHandle* h, AdjointState* a, int slots, cudaStream_
         for (float*& p : a->pscr) TRY(dalloc(h, &p, np));
         for (float*& p : a->nscr) TRY(dalloc(h, &p, nn));
         TRY(dalloc(h, &a->lam_tmp, np * NLAM));
-        TRY(dalloc(h, &a->d_lam, NLAM));
         TRY(dalloc(h, &a->cnt, (size_t)h->ncell));
         TRY(dalloc(h, &a->mismatch, 1));
         CK(h, cudaMallocHost(&a->h_mismatch, sizeof(int)));
-        CK(h, cudaMemcpyAsync(a->d_lam, a->lam, sizeof(float*) * NLAM, cudaMemcpyHostToDevice, s));
-        TRY(sync(h, s));
     }
     return MPM_OK;
 }
@@ -471,12 +465,26 @@ int recompute_segment(MpmHandle* h, AdjointState* a, int seg, int len, cudaStrea
     return clear_status(h, s);
 }
 
+// Adjoint arrays first .. first + ncomp - 1, stored in the order `pid`,
+// against the original-order array `aos`.
+FieldMap lam_map(MpmHandle* h, AdjointState* a, int first, int ncomp, const int* pid, const float* aos) {
+    FieldMap F{};
+    for (int k = 0; k < ncomp; ++k) {
+        F.comp[k] = a->lam[first + k];
+        F.slot[k] = -1;
+    }
+    F.ncomp = ncomp;
+    F.np = (int)h->np;
+    F.pid = pid;
+    F.aos = const_cast<float*>(aos);
+    return F;
+}
+
 // Move the adjoint arrays from the storage order `from` to the storage order `to`.
 int permute(MpmHandle* h, AdjointState* a, const int* from, const int* to, cudaStream_t s) {
     if (from == to) return MPM_OK;
-    const int np = (int)h->np;
-    CK(h, launch_scatter_out(a->d_lam, NLAM, from, np, a->lam_tmp, s));
-    CK(h, launch_gather_in(a->d_lam, NLAM, to, np, a->lam_tmp, s));
+    CK(h, launch_field(lam_map(h, a, 0, NLAM, from, a->lam_tmp), false, s));
+    CK(h, launch_field(lam_map(h, a, 0, NLAM, to, a->lam_tmp), true, s));
     return MPM_OK;
 }
 
@@ -576,35 +584,25 @@ int reverse_graph(MpmHandle* h, AdjointState* a, int len, cudaStream_t s) {
 }
 
 // Zero the adjoint arrays; particle (n, 2) seeds in original order -> lam[0..3]
-// in the storage order `pid`.  The zeros are one memset of the permutation
-// scratch gathered into all NLAM arrays (two launches instead of NLAM).
-// With wait == false the caller synchronises the stream before it returns
-// (a host seed may be staged in h->stage: the copies and gathers are
-// stream-ordered, so the second seed's copy follows the first one's gather).
+// in the storage order `pid`.
 int seed(MpmHandle* h, AdjointState* a, const float* dl_dloc, const float* dl_dvel,
-         const int* pid, int on_device, cudaStream_t s, bool wait = true) {
-    const int np = (int)h->np;
-    CK(h, cudaMemsetAsync(a->lam_tmp, 0, sizeof(float) * NLAM * (size_t)np, s));
-    CK(h, launch_gather_in(a->d_lam, NLAM, pid, np, a->lam_tmp, s));
+         const int* pid, int on_device, cudaStream_t s) {
+    CK(h, launch_field(lam_map(h, a, 0, NLAM, pid, nullptr), true, s));
     const float* src[2] = {dl_dloc, dl_dvel};
     for (int k = 0; k < 2; ++k) {
         if (!src[k]) continue;
         const void* d = nullptr;
         TRY(to_device(h, src[k], sizeof(float) * 2 * h->np, on_device, s, &d));
-        CK(h, launch_gather_in(a->d_lam + 2 * k, 2, pid, np, static_cast<const float*>(d), s));
-        if (wait) TRY(sync(h, s));
+        CK(h, launch_field(lam_map(h, a, 2 * k, 2, pid, static_cast<const float*>(d)), true, s));
+        TRY(sync(h, s));
     }
     return MPM_OK;
 }
 
 // Adjoint arrays lam[first..] in storage order `pid` -> particle (n, ncomp)
-// array in original order.  With wait == false the caller synchronises the
-// stream before it returns (a host destination is written by an
-// asynchronous copy out of h->stage, which the next emit reuses in stream
-// order; a larger stage is allocated only after cudaFree has waited for the
-// device).
+// array in original order.
 int emit(MpmHandle* h, AdjointState* a, float* dst, int first, int ncomp, const int* pid,
-         int on_device, cudaStream_t s, bool wait = true) {
+         int on_device, cudaStream_t s) {
     if (!dst) return MPM_OK;
     const size_t bytes = sizeof(float) * ncomp * h->np;
     float* d = dst;
@@ -612,17 +610,17 @@ int emit(MpmHandle* h, AdjointState* a, float* dst, int first, int ncomp, const 
         TRY(ensure_stage(h, bytes));
         d = static_cast<float*>(h->stage);
     }
-    CK(h, launch_scatter_out(a->d_lam + first, ncomp, pid, (int)h->np, d, s));
+    CK(h, launch_field(lam_map(h, a, first, ncomp, pid, d), false, s));
     if (!on_device) CK(h, cudaMemcpyAsync(dst, d, bytes, cudaMemcpyDeviceToHost, s));
-    return wait ? sync(h, s) : MPM_OK;
+    return sync(h, s);
 }
 
 int emit_all(MpmHandle* h, AdjointState* a, float* dl_dE, float* dl_dloc0, float* dl_dvel0,
-             int on_device, cudaStream_t s, bool wait = true) {
+             int on_device, cudaStream_t s) {
     const int* pid = a->epochs[0].pid;   // the order of the first checkpoint
-    TRY(emit(h, a, dl_dE, 9, 1, pid, on_device, s, wait));
-    TRY(emit(h, a, dl_dloc0, 0, 2, pid, on_device, s, wait));
-    return emit(h, a, dl_dvel0, 2, 2, pid, on_device, s, wait);
+    TRY(emit(h, a, dl_dE, 9, 1, pid, on_device, s));
+    TRY(emit(h, a, dl_dloc0, 0, 2, pid, on_device, s));
+    return emit(h, a, dl_dvel0, 2, 2, pid, on_device, s);
 }
 
 int check_supported(MpmHandle* h) {
@@ -843,6 +841,56 @@ int batch_recompute(MpmBatch* b, BatchAdjoint* x, int seg, int len, cudaStream_t
     return MPM_OK;
 }
 
+// seed() for every member, one launch per seed array.  A host seed is staged in
+// its member's own staging buffer; the second seed's copy follows the first
+// one's transfer on the stream.
+int batch_seed(MpmBatch* b, const float* const* dl_dloc, const float* const* dl_dvel, int on_device,
+               cudaStream_t s) {
+    const int n = (int)b->sims.size();
+    std::vector<FieldMap> maps;
+    for (MpmHandle* h : b->sims) maps.push_back(lam_map(h, h->adj, 0, NLAM, h->ps[h->pcur].pid, nullptr));
+    int r = fields_many(b, maps, true, s);
+    const float* const* src[2] = {dl_dloc, dl_dvel};
+    for (int k = 0; k < 2 && r == MPM_OK; ++k) {
+        if (!src[k]) continue;
+        maps.clear();
+        for (int i = 0; i < n; ++i) {
+            MpmHandle* h = b->sims[i];
+            if (!src[k][i]) continue;
+            const void* d = nullptr;
+            BTRY(b, i, to_device(h, src[k][i], sizeof(float) * 2 * h->np, on_device, s, &d));
+            maps.push_back(lam_map(h, h->adj, 2 * k, 2, h->ps[h->pcur].pid, static_cast<const float*>(d)));
+        }
+        r = fields_many(b, maps, true, s);
+    }
+    return r;
+}
+
+// emit() for every member with a destination, one launch; the caller
+// synchronises the stream before it returns.
+int batch_emit(MpmBatch* b, float* const* dst, int first, int ncomp, int on_device, cudaStream_t s) {
+    const int n = (int)b->sims.size();
+    std::vector<FieldMap> maps;
+    for (int i = 0; i < n; ++i) {
+        MpmHandle* h = b->sims[i];
+        if (!dst[i]) continue;
+        float* d = dst[i];
+        if (!on_device) {
+            BTRY(b, i, ensure_stage(h, sizeof(float) * ncomp * h->np));
+            d = static_cast<float*>(h->stage);
+        }
+        maps.push_back(lam_map(h, h->adj, first, ncomp, h->adj->epochs[0].pid, d));
+    }
+    const int r = fields_many(b, maps, false, s);
+    if (r != MPM_OK || on_device) return r;
+    for (int i = 0; i < n; ++i) {
+        MpmHandle* h = b->sims[i];
+        if (dst[i])
+            BCK(b, cudaMemcpyAsync(dst[i], h->stage, sizeof(float) * ncomp * h->np, cudaMemcpyDeviceToHost, s));
+    }
+    return MPM_OK;
+}
+
 int ensure_batch_adjoint(MpmBatch* b, cudaStream_t s) {
     if (!b->badj) b->badj = new BatchAdjoint();
     BatchAdjoint* x = b->badj;
@@ -977,16 +1025,10 @@ int mpm_batch_adjoint(MpmBatch* b, const float* const* dl_dloc, const float* con
     if (r != MPM_OK) return r;
     BatchAdjoint* x = b->badj;
     for (int i = 0; i < n; ++i) BTRY(b, i, ensure_adjoint_buffers(b->sims[i], b->sims[i]->adj, K, s));
-    for (int i = 0; i < n; ++i) {
-        MpmHandle* h = b->sims[i];
-        // (no wait per simulation: the segment loop synchronises the stream,
-        // and a failure here waits for the seeds already in flight)
-        const int e = seed(h, h->adj, dl_dloc[i], dl_dvel ? dl_dvel[i] : nullptr, h->ps[h->pcur].pid,
-                           on_device, s, false);
-        if (e != MPM_OK) {
-            cudaStreamSynchronize(s);
-            return from_sim(b, i, e);
-        }
+    r = batch_seed(b, dl_dloc, dl_dvel, on_device, s);
+    if (r != MPM_OK) {
+        cudaStreamSynchronize(s);   // seeds already in flight
+        return r;
     }
     x->bases.assign(n, AdjStep{});
     std::vector<int> cur(n, -1);   // epoch whose pointers bases[i] holds
@@ -1059,12 +1101,9 @@ int mpm_batch_adjoint(MpmBatch* b, const float* const* dl_dloc, const float* con
         // (the host copy of the arguments must outlive the uploads)
         if (r == MPM_OK && cudaStreamSynchronize(s) != cudaSuccess) r = bfail(b, MPM_ERR_CUDA, "synchronise");
     }
-    for (int i = 0; i < n && r == MPM_OK; ++i) {
-        MpmHandle* h = b->sims[i];
-        const int e = emit_all(h, h->adj, dl_dE ? dl_dE[i] : nullptr, dl_dloc0 ? dl_dloc0[i] : nullptr,
-                               dl_dvel0 ? dl_dvel0[i] : nullptr, on_device, s, false);
-        if (e != MPM_OK) r = from_sim(b, i, e);
-    }
+    if (r == MPM_OK && dl_dE) r = batch_emit(b, dl_dE, 9, 1, on_device, s);
+    if (r == MPM_OK && dl_dloc0) r = batch_emit(b, dl_dloc0, 0, 2, on_device, s);
+    if (r == MPM_OK && dl_dvel0) r = batch_emit(b, dl_dvel0, 2, 2, on_device, s);
     // leave every simulation at the recorded end state (read_statuses
     // synchronises the stream: the gradients' copies are complete on return)
     std::vector<CopySeg> v;

@@ -128,10 +128,67 @@ int read_statuses(MpmBatch* b, cudaStream_t s) {
     return MPM_OK;
 }
 
+int upload_table(MpmBatch* b, const void* src, size_t bytes, cudaStream_t s) {
+    if (b->table_bytes < bytes) {
+        cudaFree(b->d_table);
+        b->d_table = nullptr;
+        b->table_bytes = 0;
+        BCK(b, cudaMalloc(&b->d_table, bytes + bytes / 2));
+        b->table_bytes = bytes + bytes / 2;
+    }
+    BCK(b, cudaMemcpyAsync(b->d_table, src, bytes, cudaMemcpyHostToDevice, s));
+    return MPM_OK;
+}
+
+int fields_many(MpmBatch* b, const std::vector<FieldMap>& maps, bool in, cudaStream_t s) {
+    if (maps.empty()) return MPM_OK;
+    const int r = upload_table(b, maps.data(), sizeof(FieldMap) * maps.size(), s);
+    if (r != MPM_OK) return r;
+    int most = 0;
+    for (const FieldMap& F : maps) most = std::max(most, F.np);
+    BCK(b, launch_field_many(static_cast<const FieldMap*>(b->d_table), (int)maps.size(), most, in, s));
+    return MPM_OK;
+}
+
+int resort_many(MpmBatch* b, const std::vector<int>& members, cudaStream_t s) {
+    std::vector<int> rest;   // one or very large: the kernels of a single simulation
+    std::vector<MpmHandle*> many;
+    for (int i : members) {
+        MpmHandle* h = b->sims[i];
+        if (h->np <= 0) h->needs_resort = false;
+        else if (members.size() == 1 || h->ncell > SORT_MANY_CELLS) rest.push_back(i);
+        else many.push_back(h);
+    }
+    for (int i : rest) BTRY(b, i, resort(b->sims[i], s));
+    if (many.empty()) return MPM_OK;
+    // the sort jobs, then (once the buffers are swapped) the descriptors
+    const size_t n = many.size(), at = (sizeof(SortJob) * n + 255) / 256 * 256;
+    std::vector<char> table(at + sizeof(DescPut) * n);
+    SortJob* jobs = reinterpret_cast<SortJob*>(table.data());
+    DescPut* puts = reinterpret_cast<DescPut*>(table.data() + at);
+    int most_np = 0, most_cells = 0;
+    for (size_t k = 0; k < n; ++k) {
+        MpmHandle* h = many[k];
+        adjoint_note_resort(h);
+        jobs[k] = sort_job(h);
+        most_np = std::max(most_np, (int)h->np);
+        most_cells = std::max(most_cells, h->ncell);
+        sort_done(h);
+        puts[k].dst = h->ds;
+        puts[k].S = h->hs;
+    }
+    const int r = upload_table(b, table.data(), table.size(), s);
+    if (r != MPM_OK) return r;
+    BCK(b, launch_sort_many(static_cast<const SortJob*>(b->d_table), (int)n, most_np, most_cells, s));
+    BCK(b, launch_put_descs(reinterpret_cast<const DescPut*>(static_cast<const char*>(b->d_table) + at), (int)n, s));
+    return MPM_OK;
+}
+
 // One block of B steps for every simulation (see the file comment).
 int batch_block(MpmBatch* b, int B, cudaStream_t s) {
     const int n = (int)b->sims.size();
     if ((int)b->since_resort.size() != n) b->since_resort.assign(n, 0);
+    std::vector<int> drifted;
     for (int i = 0; i < n; ++i) {
         // a drifted simulation keeps its sort for resort_every - 1 more blocks
         // (its drifted cells take the gathering path); a two-cell drift
@@ -139,16 +196,18 @@ int batch_block(MpmBatch* b, int B, cudaStream_t s) {
         if (!b->sims[i]->needs_resort) {
             b->since_resort[i] = 0;
         } else if (++b->since_resort[i] >= b->resort_every) {
-            BTRY(b, i, resort(b->sims[i], s));
+            drifted.push_back(i);
             b->since_resort[i] = 0;
         }
     }
+    int r = resort_many(b, drifted, s);
+    if (r != MPM_OK) return r;
     std::vector<CopySeg> v;
     for (MpmHandle* h : b->sims) snapshot_segments(h, true, v);
     BTRY(b, 0, run_segments(b->sims[0], b->segbuf, v, s));
     std::vector<int64_t> step0(n);
     for (int i = 0; i < n; ++i) step0[i] = b->sims[i]->step;
-    int r = run_batch_graph(b, B, s);
+    r = run_batch_graph(b, B, s);
     if (r != MPM_OK) return r;
     for (MpmHandle* h : b->sims) {
         h->step += B;
@@ -282,6 +341,7 @@ int mpm_batch_destroy(MpmBatch* b) {
     cudaFree(b->d_tcounts);
     if (b->h_tcounts) cudaFreeHost(b->h_tcounts);
     cudaFree(b->d_stage);
+    cudaFree(b->d_table);
     cudaFree(b->d_ctls);
     cudaFree(b->d_tiles);
     cudaFree(b->d_status);
@@ -335,12 +395,15 @@ int mpm_batch_write_field(MpmBatch* b, int field, const void* src, int on_device
         d = static_cast<const char*>(b->d_stage);
     }
     size_t off = 0;
-    for (int i = 0; i < (int)b->sims.size(); ++i) {
-        MpmHandle* h = b->sims[i];
+    std::vector<FieldMap> maps;
+    for (MpmHandle* h : b->sims) {
         h->gen++;
-        BTRY(b, i, write_float_field(h, field, reinterpret_cast<const float*>(d + off), s));
+        maps.push_back(field_map(h, field, reinterpret_cast<const float*>(d + off)));
+        if (field == MPM_FIELD_LOC && h->initialized) h->needs_resort = true;
         off += sizeof(float) * ncomp_of(h, field) * h->np;
     }
+    const int r = fields_many(b, maps, true, s);
+    if (r != MPM_OK) return r;
     BCK(b, cudaStreamSynchronize(s));
     return MPM_OK;
 }
@@ -358,11 +421,15 @@ int mpm_batch_read_field(MpmBatch* b, int field, void* dst, int on_device, void*
         d = static_cast<char*>(b->d_stage);
     }
     size_t off = 0;
+    std::vector<FieldMap> maps;
     for (int i = 0; i < (int)b->sims.size(); ++i) {
         MpmHandle* h = b->sims[i];
-        BTRY(b, i, gather_field(h, field, d + off, s));
+        if (batch_writable(field)) maps.push_back(field_map(h, field, reinterpret_cast<const float*>(d + off)));
+        else BTRY(b, i, gather_field(h, field, d + off, s));
         off += sizeof(float) * ncomp_of(h, field) * h->np;
     }
+    const int r = fields_many(b, maps, false, s);
+    if (r != MPM_OK) return r;
     if (!on_device) BCK(b, cudaMemcpyAsync(dst, b->d_stage, total, cudaMemcpyDeviceToHost, s));
     BCK(b, cudaStreamSynchronize(s));
     return MPM_OK;
@@ -384,15 +451,20 @@ int mpm_batch_write_nodal_field(MpmBatch* b, int field, const float* src, int on
         d = static_cast<const char*>(b->d_stage);
     }
     size_t off = 0;
+    std::vector<FieldMap> maps;
     for (MpmHandle* h : b->sims) {
         h->gen++;
-        const float* df = reinterpret_cast<const float*>(d + off);
-        if (field == MPM_NODE_MASS)
-            BCK(b, cudaMemcpyAsync(h->nm, df, sizeof(float) * h->nn, cudaMemcpyDeviceToDevice, s));
-        else if (field == MPM_NODE_VELOCITY) BCK(b, launch_deinterleave2(df, h->nn, h->nvbx, h->nvby, s));
-        else BCK(b, launch_deinterleave2(df, h->nn, h->nax, h->nay, s));
+        FieldMap F{};
+        F.ncomp = nc;
+        F.np = h->nn;
+        F.comp[0] = field == MPM_NODE_MASS ? h->nm : field == MPM_NODE_VELOCITY ? h->nvbx : h->nax;
+        F.comp[1] = field == MPM_NODE_MASS ? nullptr : field == MPM_NODE_VELOCITY ? h->nvby : h->nay;
+        F.aos = reinterpret_cast<float*>(const_cast<char*>(d + off));
+        maps.push_back(F);
         off += sizeof(float) * nc * h->nn;
     }
+    const int r = fields_many(b, maps, true, s);
+    if (r != MPM_OK) return r;
     BCK(b, cudaStreamSynchronize(s));
     return MPM_OK;
 }
@@ -401,17 +473,22 @@ int mpm_batch_restart(MpmBatch* b, void* stream) {
     if (!b) return MPM_ERR_INVALID;
     cudaStream_t s = S(stream);
     const int n = (int)b->sims.size();
+    std::vector<int> every(n);
     for (int i = 0; i < n; ++i) {
         MpmHandle* h = b->sims[i];
         h->gen++;
         BTRY(b, i, keep_parity_data(h, 0));
         h->step = 0;
-        BCK(b, cudaMemsetAsync(h->ctl, 0, sizeof(Control), s));
-        BTRY(b, i, resort(h, s));
+        every[i] = i;
+    }
+    BCK(b, launch_zero_controls(b->d_ctls, n, s));
+    int r = resort_many(b, every, s);
+    if (r != MPM_OK) return r;
+    for (MpmHandle* h : b->sims) {
         if (!h->reinit) BCK(b, launch_setup_volume(h->ds, (int)h->np, parity(h), s));
         h->initialized = true;
     }
-    int r = read_statuses(b, s);
+    r = read_statuses(b, s);
     if (r != MPM_OK) return r;
     for (int i = 0; i < n; ++i) {
         MpmHandle* h = b->sims[i];

@@ -26,6 +26,8 @@ struct MpmBatch {
     int nact = 0, nemp = 0;
     void* d_stage = nullptr;            // staging of whole-batch field transfers
     size_t stage_bytes = 0;
+    void* d_table = nullptr;            // argument tables of launches over many members
+    size_t table_bytes = 0;
     mpm::Control** d_ctls = nullptr;
     int4* d_tiles = nullptr;
     int ntiles = 0;
@@ -57,6 +59,13 @@ int prepare_tiles(MpmBatch* b, cudaStream_t s);
 // n steps of every simulation as 3n batched launches over the active tiles
 // plus one over the empty tiles per step (no status handling).
 int launch_batch_steps(MpmBatch* b, int n, cudaStream_t s);
+// Copy a host argument table into b->d_table (valid until the next upload on
+// the stream).
+int upload_table(MpmBatch* b, const void* src, size_t bytes, cudaStream_t s);
+// Re-sort the listed members together.
+int resort_many(MpmBatch* b, const std::vector<int>& members, cudaStream_t s);
+// The mapped transfers of several members in one launch.
+int fields_many(MpmBatch* b, const std::vector<FieldMap>& maps, bool in, cudaStream_t s);
 // Gather every control block into b->h_status and clear the status words.
 int read_statuses(MpmBatch* b, cudaStream_t s);
 // Advance every simulation by nsteps steps in blocks (re-sorts, snapshots,

@@ -125,7 +125,6 @@ struct MpmHandle {
     // staging and pointer tables
     void* stage = nullptr;
     size_t stage_bytes = 0;
-    float** d_ptrs = nullptr;
     int* line_eid = nullptr;         // 1-D: element of each storage slot this step
     // asynchronous output (mpm_output_enqueue): its own staging buffer and a
     // ring of events, one per outstanding copy
@@ -203,6 +202,11 @@ int sync(MpmHandle* h, cudaStream_t s);
 int read_ctl(MpmHandle* h, cudaStream_t s);
 int clear_status(MpmHandle* h, cudaStream_t s);
 int resort(MpmHandle* h, cudaStream_t s);
+// The parts of a re-sort, for launches over many simulations.
+SortJob sort_job(MpmHandle* h);
+void sort_done(MpmHandle* h);
+// A field of h against the original-order array `aos` (ncomp 0: not a stored field).
+FieldMap field_map(MpmHandle* h, int field, const float* aos);
 // n steps from ctl->step (the tiles classified for the current sort).
 int launch_steps(MpmHandle* h, int n, cudaStream_t s);
 // Phase `phase` (0 nodal kinematics, 1 forces, 2 G2P) of step ctl->step + k.

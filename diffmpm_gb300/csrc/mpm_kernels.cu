@@ -1585,64 +1585,6 @@ cudaError_t launch_particle_kinematics_batch(const StepConfig& c, const TileDesc
 }
 
 // ---------------------------------------------------------------------------
-// Re-sort: key = current cell (ncell for a particle outside the mesh), counting
-// sort with atomic placement, then each bucket sorted by storage index, so the
-// result is the stable order whatever the placement order was.
-// ---------------------------------------------------------------------------
-__global__ void k_resort_keys(const SimDev* __restrict__ sim, int np, int nx, int ny, float hx,
-                              float hy, int* __restrict__ count, int* __restrict__ key,
-                              Control* __restrict__ ctl) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= np) return;
-    const int i = locate_axis(sim->x[q], hx, nx);
-    const int j = locate_axis(sim->y[q], hy, ny);
-    int k;
-    if (i < 0 || i >= nx || j < 0 || j >= ny) {
-        k = nx * ny;
-        atomicOr(&ctl->status, ST_OUT_OF_MESH);
-    } else {
-        k = j * nx + i;
-    }
-    key[q] = k;
-    atomicAdd(&count[k], 1);
-}
-
-cudaError_t launch_resort_keys(const SimDev* sim, int np, int nx, int ny, float hx, float hy,
-                               const SortScratch& w, Control* ctl, cudaStream_t s) {
-    if (np > 0)
-        k_resort_keys<<<(np + 255) / 256, 256, 0, s>>>(sim, np, nx, ny, hx, hy, w.count, w.key, ctl);
-    return cudaGetLastError();
-}
-
-// exclusive scan, 1024 elements per block
-__device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
-    __shared__ int warp_sums[32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int x = v;
-    #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        int w = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0;
-        #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        warp_sums[lane] = w;
-    }
-    __syncthreads();
-    const int base = wid ? warp_sums[wid - 1] : 0;
-    if (total) *total = warp_sums[(blockDim.x >> 5) - 1];
-    __syncthreads();
-    return base + x - v;
-}
-
-// ---------------------------------------------------------------------------
 // Tile classification.  A tile whose cells and the ring of sort-cells around
 // them store no particle receives none during a step block (a particle is at
 // most one cell from its sort-cell, and the sort changes only between
@@ -1846,124 +1788,6 @@ cudaError_t launch_empty_nodes_batch(const TileDesc* td, int ntiles, int k, cuda
     return cudaGetLastError();
 }
 
-__global__ void k_scan_blocks(const int* __restrict__ in, int* __restrict__ out, int n,
-                              int* __restrict__ block_sums) {
-    const int i = blockIdx.x * 1024 + threadIdx.x;
-    const int v = i < n ? in[i] : 0;
-    int total;
-    const int ex = block_exclusive_scan(v, &total);
-    if (i < n) out[i] = ex;
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-__global__ void k_scan_sums(int* __restrict__ block_sums, int nb) {
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nb; base += 1024) {
-        const int i = base + threadIdx.x;
-        const int v = i < nb ? block_sums[i] : 0;
-        int total;
-        const int ex = block_exclusive_scan(v, &total);
-        if (i < nb) block_sums[i] = ex + carry;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) block_sums[nb] = carry;
-}
-
-__global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ block_sums) {
-    const int i = blockIdx.x * 1024 + threadIdx.x;
-    if (i < n) out[i] += block_sums[blockIdx.x];
-    if (i == n) out[n] = block_sums[gridDim.x];   // grand total
-}
-
-cudaError_t launch_exclusive_scan(const int* in, int* out, int n, int* block_sums,
-                                  cudaStream_t s) {
-    const int nb = (n + 1024) / 1024;   // room for out[n]
-    k_scan_blocks<<<nb, 1024, 0, s>>>(in, out, n, block_sums);
-    k_scan_sums<<<1, 1024, 0, s>>>(block_sums, nb);
-    k_scan_add<<<nb, 1024, 0, s>>>(out, n, block_sums);
-    return cudaGetLastError();
-}
-
-__global__ void k_resort_place(int np, const int* __restrict__ start, const int* __restrict__ key,
-                               int* __restrict__ cursor, int* __restrict__ perm) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= np) return;
-    const int k = key[q];
-    perm[start[k] + atomicAdd(&cursor[k], 1)] = q;
-}
-
-cudaError_t launch_resort_place(int np, const int* start, const SortScratch& w, cudaStream_t s) {
-    if (np > 0) k_resort_place<<<(np + 255) / 256, 256, 0, s>>>(np, start, w.key, w.cursor, w.perm);
-    return cudaGetLastError();
-}
-
-__global__ void k_resort_segsort(int nbucket, const int* __restrict__ start,
-                                 int* __restrict__ perm) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nbucket) return;
-    const int b = start[c], e = start[c + 1];
-    #pragma unroll 1
-    for (int i = b + 1; i < e; ++i) {
-        const int v = perm[i];
-        int j = i - 1;
-        #pragma unroll 1
-        while (j >= b && perm[j] > v) {
-            perm[j + 1] = perm[j];
-            --j;
-        }
-        perm[j + 1] = v;
-    }
-}
-
-cudaError_t launch_resort_segsort(int nbucket, const int* start, const SortScratch& w,
-                                  cudaStream_t s) {
-    if (nbucket > 0) k_resort_segsort<<<(nbucket + 255) / 256, 256, 0, s>>>(nbucket, start, w.perm);
-    return cudaGetLastError();
-}
-
-template <class T>
-__global__ void k_gather(const T* __restrict__ src, T* __restrict__ dst,
-                         const int* __restrict__ perm, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = src[perm[i]];
-}
-
-template <class T>
-__global__ void k_gather_pair(const T* __restrict__ src, T* __restrict__ dst,
-                              const int* __restrict__ perm, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const int p = perm[i];
-        dst[2 * i] = src[2 * p];
-        dst[2 * i + 1] = src[2 * p + 1];
-    }
-}
-
-cudaError_t launch_gather_u32(const uint32_t* src, uint32_t* dst, const int* perm, int n,
-                              cudaStream_t s) {
-    if (n > 0) k_gather<uint32_t><<<(n + 255) / 256, 256, 0, s>>>(src, dst, perm, n);
-    return cudaGetLastError();
-}
-cudaError_t launch_gather_u8(const uint8_t* src, uint8_t* dst, const int* perm, int n,
-                             cudaStream_t s) {
-    if (n > 0) k_gather<uint8_t><<<(n + 255) / 256, 256, 0, s>>>(src, dst, perm, n);
-    return cudaGetLastError();
-}
-cudaError_t launch_gather_pair_u32(const uint32_t* src, uint32_t* dst, const int* perm, int n,
-                                   cudaStream_t s) {
-    if (n > 0) k_gather_pair<uint32_t><<<(n + 255) / 256, 256, 0, s>>>(src, dst, perm, n);
-    return cudaGetLastError();
-}
-cudaError_t launch_gather_pair_u8(const uint8_t* src, uint8_t* dst, const int* perm, int n,
-                                  cudaStream_t s) {
-    if (n > 0) k_gather_pair<uint8_t><<<(n + 255) / 256, 256, 0, s>>>(src, dst, perm, n);
-    return cudaGetLastError();
-}
-
 // Volume set-up of a freshly sorted population (particle.py:158-178):
 // V = V_el / count, size = sqrt(V), m = V rho.
 __global__ void k_setup_volume(const SimDev* __restrict__ sim, int np, int parity) {
@@ -1982,38 +1806,6 @@ __global__ void k_setup_volume(const SimDev* __restrict__ sim, int np, int parit
 
 cudaError_t launch_setup_volume(const SimDev* sim, int np, int parity, cudaStream_t s) {
     if (np > 0) k_setup_volume<<<(np + 255) / 256, 256, 0, s>>>(sim, np, parity);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// Field transfers
-// ---------------------------------------------------------------------------
-__global__ void k_scatter_out(const float* const* __restrict__ comp, int ncomp,
-                              const int* __restrict__ pid, int np, float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    const int o = pid[i];
-    for (int c = 0; c < ncomp; ++c) out[(size_t)o * ncomp + c] = comp[c] ? comp[c][i] : 0.0f;
-}
-
-cudaError_t launch_scatter_out(const float* const* comp_ptrs, int ncomp, const int* pid, int np,
-                               float* out, cudaStream_t s) {
-    if (np > 0) k_scatter_out<<<(np + 255) / 256, 256, 0, s>>>(comp_ptrs, ncomp, pid, np, out);
-    return cudaGetLastError();
-}
-
-__global__ void k_gather_in(float* const* __restrict__ comp, int ncomp,
-                            const int* __restrict__ pid, int np, const float* __restrict__ in) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    const int o = pid[i];
-    for (int c = 0; c < ncomp; ++c)
-        if (comp[c]) comp[c][i] = in[(size_t)o * ncomp + c];
-}
-
-cudaError_t launch_gather_in(float* const* comp_ptrs, int ncomp, const int* pid, int np,
-                             const float* in, cudaStream_t s) {
-    if (np > 0) k_gather_in<<<(np + 255) / 256, 256, 0, s>>>(comp_ptrs, ncomp, pid, np, in);
     return cudaGetLastError();
 }
 
@@ -2244,6 +2036,16 @@ __global__ void k_gather_status(Control* const* __restrict__ ctls, int n, Contro
     Control* c = ctls[i];
     out[i] = *c;
     c->status = 0;
+}
+
+__global__ void k_zero_controls(Control* const* __restrict__ ctls, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) *ctls[i] = Control{};
+}
+
+cudaError_t launch_zero_controls(Control* const* ctls, int n, cudaStream_t s) {
+    if (n > 0) k_zero_controls<<<(n + 127) / 128, 128, 0, s>>>(ctls, n);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_gather_status(Control* const* ctls, int n, Control* out, cudaStream_t s) {

@@ -89,40 +89,72 @@ cudaError_t launch_forces_batch(const StepConfig& c, const TileDesc* td, int nti
 cudaError_t launch_particle_kinematics_batch(const StepConfig& c, const TileDesc* td, int ntiles,
                                              int k, cudaStream_t s);
 
-// Re-sort of one simulation's particles by current cell, stable in storage order.
+// Re-sort of a simulation's particles by current cell, stable in storage
+// order (mpm_sort.cu): the arguments of one simulation, current arrays to the
+// other buffer set.
 struct SortScratch {
     int* count;        // ncell + 1 (last bucket: particles outside the mesh)
-    int* cursor;       // ncell + 1
     int* key;          // np
+    int* rank;         // np
     int* perm;         // np
     int* block_sums;   // ceil((ncell + 2) / 1024) + 1
 };
-cudaError_t launch_resort_keys(const SimDev* sim, int np, int nx, int ny, float hx, float hy,
-                               const SortScratch& w, Control* ctl, cudaStream_t s);
-cudaError_t launch_exclusive_scan(const int* in, int* out, int n, int* block_sums, cudaStream_t s);
-cudaError_t launch_resort_place(int np, const int* start, const SortScratch& w, cudaStream_t s);
-cudaError_t launch_resort_segsort(int nbucket, const int* start, const SortScratch& w,
-                                  cudaStream_t s);
-
-// dst[i] = src[perm[i]] for 4-byte and 1-byte elements.
-cudaError_t launch_gather_u32(const uint32_t* src, uint32_t* dst, const int* perm, int n,
-                              cudaStream_t s);
-cudaError_t launch_gather_u8(const uint8_t* src, uint8_t* dst, const int* perm, int n,
-                             cudaStream_t s);
-cudaError_t launch_gather_pair_u32(const uint32_t* src, uint32_t* dst, const int* perm, int n,
-                                   cudaStream_t s);
-cudaError_t launch_gather_pair_u8(const uint8_t* src, uint8_t* dst, const int* perm, int n,
-                                  cudaStream_t s);
+constexpr int SORT_FIELDS = 18;   // 4-byte arrays that move with a particle
+struct SortJob {
+    int np, nx, ny, nf;
+    float hx, hy;
+    const float *x, *y;
+    int *count, *key, *rank, *perm, *start;
+    uint8_t* cflag;
+    Control* ctl;
+    const uint32_t* src[SORT_FIELDS];
+    uint32_t* dst[SORT_FIELDS];
+    const uint8_t* mat_src;
+    uint8_t* mat_dst;
+    const uint16_t* pvc_src;    // byte pairs; null when absent
+    uint16_t* pvc_dst;
+    const uint16_t* trfn_src;   // byte pairs; null when absent
+    uint16_t* trfn_dst;
+    const float2* trtau_src;
+    float2* trtau_dst;
+};
+// Clears the counts and drift flags, then count, start and perm (each bucket
+// in storage order with `buckets`); the arrays' move is apart.
+cudaError_t launch_sort_order(const SortJob& J, int* block_sums, bool buckets, cudaStream_t s);
+cudaError_t launch_sort_move(const SortJob& J, cudaStream_t s);
+// All of it for n simulations (device table), each of at most SORT_MANY_CELLS
+// cells: one CTA scans a simulation's counts.
+constexpr int SORT_MANY_CELLS = 1 << 18;
+cudaError_t launch_sort_many(const SortJob* jobs, int n, int most_np, int most_cells, cudaStream_t s);
+// *puts[i].dst = puts[i].S
+struct DescPut {
+    SimDev* dst;
+    SimDev S;
+};
+cudaError_t launch_put_descs(const DescPut* puts, int n, cudaStream_t s);
 
 // Solve-semantics volume set-up after a sort (V = V_el / count, m = V rho, size = sqrt V).
 cudaError_t launch_setup_volume(const SimDev* sim, int np, int parity, cudaStream_t s);
 
-// Field transfer between original order (AoS, ncomp per particle) and storage order (SoA).
-// comp_ptrs: device array of ncomp float* (storage order); pid: storage -> original.
-cudaError_t launch_scatter_out(const float* const* comp_ptrs, int ncomp, const int* pid, int np,
-                               float* out, cudaStream_t s);
-cudaError_t launch_gather_in(float* const* comp_ptrs, int ncomp, const int* pid, int np,
-                             const float* in, cudaStream_t s);
+// dst[i] = src[perm[i]] for pairs of bytes and of floats.
+cudaError_t launch_gather_pairs(const uint16_t* src, uint16_t* dst, const int* perm, int n, cudaStream_t s);
+cudaError_t launch_gather_pairs(const float2* src, float2* dst, const int* perm, int n, cudaStream_t s);
+
+// Transfer of a field between original order (aos: ncomp values per particle,
+// null reads as zeros) and storage order (an array per component; a component
+// without one lives in slot[c] of the original-order `passive` array, or is
+// zero); pid: storage -> original (null: the same order).
+constexpr int PASSIVE_N = 5;
+struct FieldMap {
+    float* comp[12];
+    signed char slot[12];
+    int ncomp, np;
+    const int* pid;
+    float* passive;
+    float* aos;
+};
+cudaError_t launch_field(const FieldMap& F, bool in, cudaStream_t s);
+cudaError_t launch_field_many(const FieldMap* maps, int n, int most_np, bool in, cudaStream_t s);
 cudaError_t launch_gather_in_u8(uint8_t* dst, const int* pid, int np, const int32_t* in,
                                 cudaStream_t s);
 cudaError_t launch_scatter_out_u8(const uint8_t* src, const int* pid, int np, int32_t* out,
@@ -169,6 +201,8 @@ cudaError_t launch_copy_segments(const CopyChunk* chunks, unsigned nchunks, int 
 cudaError_t launch_compare_segments(const CopyChunk* chunks, unsigned nchunks, int* mismatch,
                                     cudaStream_t s);
 
+// *ctls[i] = 0 for i < n.
+cudaError_t launch_zero_controls(Control* const* ctls, int n, cudaStream_t s);
 // out[i] = *ctls[i], then ctls[i]->status = 0, for i < n.
 cudaError_t launch_gather_status(Control* const* ctls, int n, Control* out, cudaStream_t s);
 
