@@ -10,6 +10,7 @@
 // and replayed one step at a time with a re-sort before every step.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -53,14 +54,7 @@ void dfree(MpmHandle* h, void* p) {
     cudaFree(p);
 }
 
-void drop_graphs(MpmHandle* h) {
-    for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);
-    h->graphs.clear();
-    h->graph_gen++;
-}
-
 int upload_desc(MpmHandle* h) {
-    drop_graphs(h);
     CK(h, cudaMemcpy(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice));
     return MPM_OK;
 }
@@ -180,7 +174,6 @@ void sort_done(MpmHandle* h) {
     h->pcur ^= 1;
     h->cs_cur ^= 1;
     bind_particles(h);
-    drop_graphs(h);   // the step graphs hold the descriptor by value
     h->needs_resort = false;
     h->resorts++;
 }
@@ -234,6 +227,12 @@ StepConfig step_config(const MpmHandle* h) {
 // Split the tiles into active and empty ones for the current sort (see
 // launch_classify_tiles); every launched sequence of steps starts with it.
 int classify_tiles(MpmHandle* h, cudaStream_t s) {
+    if (h->ntiles < h->empty_split_min) {   // never enough empty tiles to launch apart
+        h->step_tiles = h->dtiles;
+        h->nact = h->ntiles;
+        h->nemp = 0;
+        return MPM_OK;
+    }
     CK(h, launch_classify_tiles(h->hs, h->dtiles, h->ntiles, h->d_tile_flags, h->d_active, h->d_empty,
                                 h->d_tile_counts, s));
     CK(h, cudaMemcpyAsync(h->h_tile_counts, h->d_tile_counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -253,9 +252,8 @@ int classify_tiles(MpmHandle* h, cudaStream_t s) {
     return MPM_OK;
 }
 
-// Graph-cache key of a step sequence: its length and the grids it launches.
-int64_t seq_key(const MpmHandle* h, int n) {
-    return (int64_t)n | ((int64_t)h->nact << 24) | ((int64_t)h->nemp << 44);
+StepKey step_key(const MpmHandle* h) {
+    return StepKey{h->hs, step_config(h), h->step_tiles, h->nact, h->nemp};
 }
 
 // One phase of step (ctl->step + k) over the active tiles (the empty tiles'
@@ -285,32 +283,40 @@ int launch_steps(MpmHandle* h, int n, cudaStream_t s) {
 
 
 
-int run_graph(MpmHandle* h, int n, cudaStream_t s) {
-    if (h->graphs_trac != h->has_trac) {
-        drop_graphs(h);
-        h->graphs_trac = h->has_trac;
-    }
+// n steps: whole graphs of GRAPH_STEPS steps (of the most recently used
+// GRAPH_CACHE configurations), then the rest as launches.
+int run_steps(MpmHandle* h, int n, cudaStream_t s) {
+    constexpr size_t GRAPH_CACHE = 8;
     TRY(classify_tiles(h, s));
-    const int64_t key = seq_key(h, n);
-    auto it = h->graphs.find(key);
-    if (it == h->graphs.end()) {
-        cudaGraph_t g = nullptr;
-        CK(h, cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
-        int r = launch_steps(h, n, h->cap);
-        cudaError_t e = cudaStreamEndCapture(h->cap, &g);
-        if (r != MPM_OK) {
-            if (g) cudaGraphDestroy(g);
-            return r;
+    if (n >= GRAPH_STEPS) {
+        const StepKey key = step_key(h);
+        size_t at = 0;
+        while (at < h->graphs.size() && !(h->graphs[at].key == key)) ++at;
+        if (at == h->graphs.size()) {
+            cudaGraph_t g = nullptr;
+            CK(h, cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
+            const int r = launch_steps(h, GRAPH_STEPS, h->cap);
+            cudaError_t e = cudaStreamEndCapture(h->cap, &g);
+            if (r != MPM_OK) {
+                if (g) cudaGraphDestroy(g);
+                return r;
+            }
+            CK(h, e);
+            cudaGraphExec_t ex = nullptr;
+            e = cudaGraphInstantiate(&ex, g, 0);
+            cudaGraphDestroy(g);
+            CK(h, e);
+            if (h->graphs.size() == GRAPH_CACHE) {
+                cudaGraphExecDestroy(h->graphs.back().exec);
+                h->graphs.pop_back();
+            }
+            h->graphs.insert(h->graphs.begin(), StepGraph{key, ex});
+        } else if (at > 0) {
+            std::rotate(h->graphs.begin(), h->graphs.begin() + at, h->graphs.begin() + at + 1);
         }
-        CK(h, e);
-        cudaGraphExec_t ex = nullptr;
-        e = cudaGraphInstantiate(&ex, g, 0);
-        cudaGraphDestroy(g);
-        CK(h, e);
-        it = h->graphs.emplace(key, ex).first;
+        for (; n >= GRAPH_STEPS; n -= GRAPH_STEPS) CK(h, cudaGraphLaunch(h->graphs[0].exec, s));
     }
-    CK(h, cudaGraphLaunch(it->second, s));
-    return MPM_OK;
+    return n > 0 ? launch_steps(h, n, s) : MPM_OK;
 }
 
 int check_status(MpmHandle* h, int& st) {
@@ -753,7 +759,7 @@ int mpm_destroy(MpmHandle* h) {
     mpm::adjoint_free(h);
     mpm::line_adjoint_free(h);
     segbuf_free(h->segbuf);
-    drop_graphs(h);
+    for (StepGraph& g : h->graphs) cudaGraphExecDestroy(g.exec);
     if (h->cap) cudaStreamDestroy(h->cap);
     for (cudaEvent_t& e : h->out_ev)
         if (e) cudaEventDestroy(e);
@@ -775,7 +781,6 @@ int mpm_set_particles(MpmHandle* h, int64_t n, const float* loc, const int32_t* 
     TRY(sync(h, s));
     if (h->np != n) {
         free_particles(h);
-        drop_graphs(h);
         if (n > 0) TRY(alloc_particles(h, n));
         h->np = n;
     }
@@ -871,8 +876,7 @@ namespace mpm {
 namespace host {
 
 // Before the step counter changes to `step`: when its parity changes, swap the
-// ping-pong pairs so that the current data stays addressed by the new parity
-// (graphs, which hold the descriptor by value, are dropped).
+// ping-pong pairs so that the current data stays addressed by the new parity.
 int keep_parity_data(MpmHandle* h, int64_t step) {
     if ((step & 1) == (h->step & 1) || h->np <= 0) return MPM_OK;
     for (int k = 0; k < 2; ++k) {
@@ -886,7 +890,6 @@ int keep_parity_data(MpmHandle* h, int64_t step) {
         std::swap(p.vol[0], p.vol[1]);
     }
     bind_particles(h);
-    drop_graphs(h);
     return upload_desc(h);
 }
 
@@ -1062,7 +1065,6 @@ int mpm_set_tractions(MpmHandle* h, int n, const int64_t* pid, const int32_t* di
     CK(h, launch_gather_pairs(reinterpret_cast<const uint16_t*>(st8), reinterpret_cast<uint16_t*>(p.tr_fn), p.pid, (int)np, s));
     h->has_trac = true;
     bind_particles(h);
-    drop_graphs(h);
     CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
     return sync(h, s);
 }
@@ -1078,7 +1080,6 @@ int mpm_set_particle_velocity_constraints(MpmHandle* h, int n, const int64_t* pi
     if (n <= 0 || np == 0) {
         h->has_pvc = false;
         bind_particles(h);
-        drop_graphs(h);
         return upload_desc(h);
     }
     if (!pid || !dir || !velocity) return fail(h, MPM_ERR_INVALID, "null constraint list");
@@ -1110,7 +1111,6 @@ int mpm_set_particle_velocity_constraints(MpmHandle* h, int n, const int64_t* pi
     CK(h, launch_gather_pairs(static_cast<const uint16_t*>(h->stage), reinterpret_cast<uint16_t*>(p.pvc), p.pid, (int)np, s));
     h->has_pvc = true;
     bind_particles(h);
-    drop_graphs(h);
     CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
     return sync(h, s);
 }
@@ -1227,7 +1227,7 @@ int mpm_step(MpmHandle* h, int nsteps, void* stream) {
         if (h->needs_resort) TRY(resort(h, s));
         const int64_t step0 = h->step;
         TRY(take_snapshot(h, s));
-        TRY(run_graph(h, B, s));
+        TRY(run_steps(h, B, s));
         h->step += B;
         TRY(read_ctl(h, s));
         // a two-cell drift corrupts the rest of the block (a particle may even be
@@ -1342,7 +1342,6 @@ int mpm_set_kernel_variant(MpmHandle* h, int nk_ctas, int g2p_ctas, int forces_l
         h->nk_ctas = nk_ctas;
         h->g2p_ctas = g2p_ctas;
         h->forces_lpc = forces_lpc;
-        drop_graphs(h);   // the captured graphs hold the other builds
     }
     return MPM_OK;
 }

@@ -64,6 +64,15 @@ struct Epoch {               // arrays of one sort epoch inside a segment
 
 }  // namespace
 
+// The segment graphs of one configuration of the step launches: the re-run
+// with its tape copies (keyed by 2 * length + start parity) and the reverse
+// steps (keyed by length).
+struct AdjGraphs {
+    StepKey key;
+    std::map<int64_t, cudaGraphExec_t> rerun, rev;
+    SegBuf tp[2], tn;          // tape copy tables of the re-run graphs
+};
+
 struct AdjointState {
     int K = 0, nseg = 0;
     int64_t step0 = 0, nsteps = 0;
@@ -90,14 +99,10 @@ struct AdjointState {
     int* cnt = nullptr;
     int* mismatch = nullptr;   // device counter of the re-run check
     int* h_mismatch = nullptr; // pinned
-    // CUDA graphs of whole segments without a re-sort: the re-run with its
-    // tape copies (keyed by 2 * length + start parity) and the reverse steps
-    // (keyed by length).  They hold the step descriptor and every buffer
-    // pointer by value, so they are dropped when the handle's step graphs are
-    // (g_gen != graph_gen) and whenever a buffer here is (re)allocated.
-    std::map<int64_t, cudaGraphExec_t> g_rerun, g_rev;
-    SegBuf g_tp[2], g_tn;      // tape copy tables of the re-run graphs
-    uint64_t g_gen = ~0ull;
+    // CUDA graphs of whole segments without a re-sort, for the most recently
+    // used configurations first; dropped whenever a buffer here is
+    // (re)allocated.
+    std::vector<AdjGraphs> graphs;
 };
 
 // Scratch of a batched adjoint (owned by the batch).
@@ -119,14 +124,16 @@ struct BatchAdjoint {
 
 namespace {
 
+void free_adj_graphs(AdjGraphs& g) {
+    for (auto& kv : g.rerun) cudaGraphExecDestroy(kv.second);
+    for (auto& kv : g.rev) cudaGraphExecDestroy(kv.second);
+    for (SegBuf& b : g.tp) segbuf_free(b);
+    segbuf_free(g.tn);
+}
+
 void drop_adj_graphs(AdjointState* a) {
-    for (auto& kv : a->g_rerun) cudaGraphExecDestroy(kv.second);
-    for (auto& kv : a->g_rev) cudaGraphExecDestroy(kv.second);
-    a->g_rerun.clear();
-    a->g_rev.clear();
-    for (SegBuf& b : a->g_tp) segbuf_free(b);
-    segbuf_free(a->g_tn);
-    a->g_gen = ~0ull;
+    for (AdjGraphs& g : a->graphs) free_adj_graphs(g);
+    a->graphs.clear();
 }
 
 void free_buffers(MpmHandle* h, AdjointState* a) {
@@ -327,21 +334,31 @@ bool resorts_at(const AdjointState* a, int64_t step) {
     return std::binary_search(a->resort_steps.begin(), a->resort_steps.end(), step);
 }
 
-// Tape copy tables of the segment graphs, for the handle's current
-// descriptors (the previous graphs are dropped when those changed).
+// The graphs of the handle's current step configuration (the first of
+// a->graphs), with the tape copy tables of its buffers.
 int prepare_adj_graphs(MpmHandle* h, AdjointState* a, cudaStream_t s) {
-    if (a->g_gen == h->graph_gen) return MPM_OK;
-    drop_adj_graphs(a);
+    constexpr size_t KEEP = 4;
+    const StepKey key = step_key(h);
+    size_t at = 0;
+    while (at < a->graphs.size() && !(a->graphs[at].key == key)) ++at;
+    if (at < a->graphs.size()) {
+        std::rotate(a->graphs.begin(), a->graphs.begin() + at, a->graphs.begin() + at + 1);
+        return MPM_OK;
+    }
+    if (a->graphs.size() == KEEP) {
+        free_adj_graphs(a->graphs.back());
+        a->graphs.pop_back();
+    }
+    a->graphs.insert(a->graphs.begin(), AdjGraphs{key, {}, {}, {}, {}});
+    AdjGraphs& g = a->graphs[0];
     for (int par = 0; par < 2; ++par) {
         std::vector<CopySeg> v;
         tape_particle_segments(h, a, par, v);
-        TRY(upload_segments(h, a->g_tp[par], v, s));
+        TRY(upload_segments(h, g.tp[par], v, s));
     }
     std::vector<CopySeg> vn;
     tape_node_segments(h, a, vn);
-    TRY(upload_segments(h, a->g_tn, vn, s));
-    a->g_gen = h->graph_gen;
-    return MPM_OK;
+    return upload_segments(h, g.tn, vn, s);
 }
 
 // Capture the launches that `body` issues on the handle's capture stream
@@ -374,15 +391,16 @@ int run_cached_graph(MpmHandle* h, std::map<int64_t, cudaGraphExec_t>& map, int6
 // step the tape copy of the start state, the step's kernels (at step offset
 // t) and the tape copy of the nodal results; the step counter advances once.
 int rerun_graph(MpmHandle* h, AdjointState* a, int len, cudaStream_t s) {
-    TRY(prepare_adj_graphs(h, a, s));
     TRY(classify_tiles(h, s));   // the restored checkpoint's sort
+    TRY(prepare_adj_graphs(h, a, s));
+    AdjGraphs& g = a->graphs[0];
     const int par0 = parity(h);
-    TRY(run_cached_graph(h, a->g_rerun, seq_key(h, 2 * len + par0), s, [&](cudaStream_t c) -> int {
+    TRY(run_cached_graph(h, g.rerun, 2 * len + par0, s, [&](cudaStream_t c) -> int {
         for (int t = 0; t < len; ++t) {
-            const SegBuf& tp = a->g_tp[(par0 + t) & 1];
+            const SegBuf& tp = g.tp[(par0 + t) & 1];
             CK(h, launch_copy_segments(tp.blk, tp.nblocks, t, c));
             for (int p = 0; p < 3; ++p) TRY(launch_phase(h, p, t, c));
-            CK(h, launch_copy_segments(a->g_tn.blk, a->g_tn.nblocks, t, c));
+            CK(h, launch_copy_segments(g.tn.blk, g.tn.nblocks, t, c));
         }
         CK(h, launch_advance_step(h->ctl, len, c));
         return MPM_OK;
@@ -570,14 +588,10 @@ int reverse_step(MpmHandle* h, AdjointState* a, int t, cudaStream_t s) {
 }
 
 // The reverse steps of a segment of `len` steps in one sort epoch as one
-// graph (keyed by the length and the number of tiles it launches).
+// graph (for the step configuration of its re-run).
 int reverse_graph(MpmHandle* h, AdjointState* a, int len, cudaStream_t s) {
     TRY(prepare_adj_graphs(h, a, s));
-    const int4* tiles;
-    int ntiles;
-    reverse_tiles(h, a, tiles, ntiles);
-    const int64_t key = (int64_t)len | ((int64_t)ntiles << 24);
-    return run_cached_graph(h, a->g_rev, key, s, [&](cudaStream_t c) -> int {
+    return run_cached_graph(h, a->graphs[0].rev, len, s, [&](cudaStream_t c) -> int {
         for (int t = len - 1; t >= 0; --t) TRY(reverse_step(h, a, t, c));
         return MPM_OK;
     });

@@ -83,29 +83,32 @@ int launch_batch_steps(MpmBatch* b, int n, cudaStream_t s) {
     return MPM_OK;
 }
 
-int run_batch_graph(MpmBatch* b, int n, cudaStream_t s) {
-    int r0 = prepare_tiles(b, s);
+// n steps: whole graphs of GRAPH_STEPS steps, then the rest as launches.
+int run_batch_steps(MpmBatch* b, int n, cudaStream_t s) {
+    const int r0 = prepare_tiles(b, s);
     if (r0 != MPM_OK) return r0;
-    const int64_t key = (int64_t)n | ((int64_t)b->nact << 24) | ((int64_t)b->nemp << 44);
-    auto it = b->graphs.find(key);
-    if (it == b->graphs.end()) {
-        cudaGraph_t g = nullptr;
-        BCK(b, cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
-        int r = launch_batch_steps(b, n, b->cap);
-        cudaError_t e = cudaStreamEndCapture(b->cap, &g);
-        if (r != MPM_OK) {
-            if (g) cudaGraphDestroy(g);
-            return r;
+    if (n >= GRAPH_STEPS) {
+        const int64_t key = (int64_t)b->nact | ((int64_t)b->nemp << 32);
+        auto it = b->graphs.find(key);
+        if (it == b->graphs.end()) {
+            cudaGraph_t g = nullptr;
+            BCK(b, cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
+            const int r = launch_batch_steps(b, GRAPH_STEPS, b->cap);
+            cudaError_t e = cudaStreamEndCapture(b->cap, &g);
+            if (r != MPM_OK) {
+                if (g) cudaGraphDestroy(g);
+                return r;
+            }
+            BCK(b, e);
+            cudaGraphExec_t ex = nullptr;
+            e = cudaGraphInstantiate(&ex, g, 0);
+            cudaGraphDestroy(g);
+            BCK(b, e);
+            it = b->graphs.emplace(key, ex).first;
         }
-        BCK(b, e);
-        cudaGraphExec_t ex = nullptr;
-        e = cudaGraphInstantiate(&ex, g, 0);
-        cudaGraphDestroy(g);
-        BCK(b, e);
-        it = b->graphs.emplace(key, ex).first;
+        for (; n >= GRAPH_STEPS; n -= GRAPH_STEPS) BCK(b, cudaGraphLaunch(it->second, s));
     }
-    BCK(b, cudaGraphLaunch(it->second, s));
-    return MPM_OK;
+    return n > 0 ? launch_batch_steps(b, n, s) : MPM_OK;
 }
 
 int check_ready(MpmBatch* b) {
@@ -207,7 +210,7 @@ int batch_block(MpmBatch* b, int B, cudaStream_t s) {
     BTRY(b, 0, run_segments(b->sims[0], b->segbuf, v, s));
     std::vector<int64_t> step0(n);
     for (int i = 0; i < n; ++i) step0[i] = b->sims[i]->step;
-    r = run_batch_graph(b, B, s);
+    r = run_batch_steps(b, B, s);
     if (r != MPM_OK) return r;
     for (MpmHandle* h : b->sims) {
         h->step += B;

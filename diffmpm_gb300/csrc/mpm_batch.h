@@ -37,7 +37,7 @@ struct MpmBatch {
     int resort_every = 1;               // re-sort a drifted simulation every this many blocks
     std::vector<int> since_resort;      // blocks each simulation has run since it drifted
     cudaStream_t cap = nullptr;
-    std::map<int64_t, cudaGraphExec_t> graphs;   // keyed by steps and tile counts
+    std::map<int64_t, cudaGraphExec_t> graphs;   // of GRAPH_STEPS steps, keyed by the tile counts
     mpm::SegBuf segbuf;
     std::vector<mpm::Checkpoint> tune;  // per-simulation state saved by the autotuner
     mpm::BatchAdjoint* badj = nullptr;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstring>
 #include <map>
 #include <string>
 #include <vector>
@@ -25,6 +26,25 @@ struct PSet {
     int8_t* tr_fn = nullptr;
     uint8_t* pvc = nullptr;     // particle velocity constraint codes (2 per particle)
     int* pid = nullptr;
+};
+
+// What the launches of a step hold by value: the simulation's descriptor, the
+// kernel builds, the tile list and the grids over it.  A captured graph serves
+// every later step for which these are the same; a re-sort swaps the two
+// buffer sets and so alternates between two of them.
+struct StepKey {
+    SimDev desc;
+    StepConfig cfg;
+    const int4* tiles;
+    int nact, nemp;
+    bool operator==(const StepKey& o) const {
+        return memcmp(&desc, &o.desc, sizeof(SimDev)) == 0 && cfg == o.cfg && tiles == o.tiles &&
+               nact == o.nact && nemp == o.nemp;
+    }
+};
+struct StepGraph {
+    StepKey key;
+    cudaGraphExec_t exec;
 };
 
 struct AdjointState;   // checkpoints, tape and adjoint arrays (mpm_adjoint.cu)
@@ -133,11 +153,9 @@ struct MpmHandle {
     size_t out_stage_bytes = 0;
     cudaEvent_t out_ev[OUT_SLOTS] = {};
     int64_t out_tickets = 0;
-    // graphs
+    // graphs of GRAPH_STEPS steps, the most recently used first
     cudaStream_t cap = nullptr;
-    std::map<int64_t, cudaGraphExec_t> graphs;   // keyed by steps and the tile counts
-    bool graphs_trac = false;
-    uint64_t graph_gen = 0;            // bumped whenever the step graphs are dropped
+    std::vector<mpm::StepGraph> graphs;
     bool has_pvc = false;              // particle velocity constraints set
     float* d_pvc_vel = nullptr;
     bool initialized = false, needs_resort = false;
@@ -192,7 +210,6 @@ int dalloc(MpmHandle* h, T** p, size_t count) {
 void dfree(MpmHandle* h, void* p);
 inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 
-void drop_graphs(MpmHandle* h);
 int upload_desc(MpmHandle* h);
 void bind_particles(MpmHandle* h);
 int parity(const MpmHandle* h);
@@ -215,8 +232,7 @@ int launch_phase(MpmHandle* h, int phase, int k, cudaStream_t s);
 // current sort; call before a sequence of launch_phase (it waits for the
 // counts, so not inside a stream capture).
 int classify_tiles(MpmHandle* h, cudaStream_t s);
-// Graph-cache key of a step sequence: its length and the grids it launches.
-int64_t seq_key(const MpmHandle* h, int n);
+StepKey step_key(const MpmHandle* h);
 int check_status(MpmHandle* h, int& st);
 int take_snapshot(MpmHandle* h, cudaStream_t s);
 int replay_block(MpmHandle* h, int64_t step0, int B, int& st, cudaStream_t s);

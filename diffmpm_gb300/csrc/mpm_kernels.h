@@ -30,6 +30,10 @@ struct StepConfig {
     // per cell (1), particle per lane on a staged row (2); the same bits
     // every way
     int forces_lpc = 0;
+    bool operator==(const StepConfig& o) const {
+        return usl == o.usl && reinit == o.reinit && traction == o.traction && nk_ctas == o.nk_ctas &&
+               g2p_ctas == o.g2p_ctas && forces_lpc == o.forces_lpc;
+    }
 };
 
 // One explicit step = three launches over the (active) tile list.  The descriptor is
@@ -70,6 +74,11 @@ cudaError_t launch_empty_nodes(const SimDev& S, const int4* empty, int ntiles, C
 cudaError_t launch_classify_tiles_batch(const SimDev* const* sims, const int4* tiles, int ntiles, int* flags,
                                         int4* active, int4* empty, int* counts, cudaStream_t s);
 cudaError_t launch_empty_nodes_batch(const TileDesc* td, int ntiles, int k, cudaStream_t s);
+// Steps of a captured step graph (a block of steps launches it repeatedly and
+// the remainder without a graph): a graph of a whole block of 100 steps cost
+// 1.2 ms to capture and instantiate, one of 20 a fifth, and 20 steps on the GPU
+// last longer than the host needs for the next launch.
+constexpr int GRAPH_STEPS = 20;
 // The kernels above work on step (ctl->step + k); these advance the counter
 // once a sequence of steps has been launched.
 cudaError_t launch_advance_step(Control* ctl, int by, cudaStream_t s);
