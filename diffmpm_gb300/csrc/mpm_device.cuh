@@ -244,24 +244,33 @@ __device__ __forceinline__ float node_sum(const float (*s)[SC_STRIDE], int tid) 
 // j = q - (rb4 + kP).  Every source array must start on a 16-byte boundary
 // and hold a multiple of 4 slots (the last piece may read up to 3 slots past
 // re).
-template <int NF, int P, class F>
+// Pass p0 of a row: every field's pieces, as one group.
+template <int NF, int P>
+__device__ __forceinline__ void row_issue16(float (*buf)[P], const float* const (&src)[NF], int p0, int re,
+                                            int lane) {
+    const int p1 = min(p0 + P, re);
+    #pragma unroll
+    for (int k = 0; k < NF; ++k) {
+        if (!src[k]) continue;
+        #pragma unroll
+        for (int o = 4 * lane; o < P; o += 128)
+            if (p0 + o < p1) cp_async16(&buf[k][o], src[k] + p0 + o);
+    }
+    cp_async_commit();
+}
+
+// ISSUED: the caller issued the first pass (row_issue16 at rb rounded down).
+template <int NF, int P, bool ISSUED = false, class F>
 __device__ __forceinline__ void row_pass16(float (*buf)[P], const float* const (&src)[NF], int rb,
                                            int re, int cb, int ce, int lane, F&& f) {
     static_assert(P % 4 == 0, "passes start on 16-byte boundaries");
+    const int first = rb & ~3;
     #pragma unroll 1
-    for (int p0 = rb & ~3; p0 < re; p0 += P) {
-        const int p1 = min(p0 + P, re);
-        #pragma unroll
-        for (int k = 0; k < NF; ++k) {
-            if (!src[k]) continue;
-            #pragma unroll
-            for (int o = 4 * lane; o < P; o += 128)
-                if (p0 + o < p1) cp_async16(&buf[k][o], src[k] + p0 + o);
-        }
-        cp_async_commit();
+    for (int p0 = first; p0 < re; p0 += P) {
+        if (!ISSUED || p0 > first) row_issue16<NF, P>(buf, src, p0, re, lane);
         cp_async_wait<0>();
         __syncwarp();
-        const int lo = max(cb, p0), hi = min(ce, p1);
+        const int lo = max(cb, p0), hi = min(ce, min(p0 + P, re));
         #pragma unroll 1
         for (int q = lo; q < hi; ++q) f(q, q - p0);
         __syncwarp();

@@ -24,9 +24,11 @@
 
 namespace mpm {
 
-__device__ __forceinline__ int load_step(const Control* ctl) {
-    return *reinterpret_cast<const volatile int*>(&ctl->step);
-}
+// The step counter at the start of the launched sequence.  No kernel that reads
+// it writes it, so it goes through L1: as a volatile load every warp of the
+// grid fetched the same word from L2, which queued there (1024^2: 1850 cycles
+// at the start of every forces CTA, 430 for the load before it).
+__device__ __forceinline__ int load_step(const Control* ctl) { return __ldg(&ctl->step); }
 
 // Batched launches: per step block, every tile gets a record with its
 // simulation's descriptor and control pointer, the storage starts of its
@@ -249,86 +251,62 @@ __device__ __forceinline__ int cell_of(const int* cs, int last, int q) {
     return lo;
 }
 
-// The tile set-up loads, all issued before any is consumed so that they cost
-// one round trip: the storage starts of the tile's cell row cj (lane l: column
-// c0x + l, lane 0 also column c0x + 32), whether a particle is stored in the
-// sort-cells [c0x-1, c0x+33) x [c0y-1, c0y+17) (a particle is at most one
-// cell from its sort-cell, so when the cells of a tile and the ring of cells
-// around them store no particle, no particle is in the tile's cells), and
-// whether any of them has its drift flag set (the tile then takes the
-// gathering path).
+// The tile set-up loads, returned unconsumed so that they stay in flight
+// behind the work that needs none of them: the storage starts of the tile's
+// cell row cj (lane l: column c0x + l, lane 0 also column c0x + 32) and this
+// thread's drift flags of the sort-cells [c0x-1, c0x+33) x [c0y-1, c0y+17)
+// (a particle is at most one cell from its sort-cell; when one of them is set
+// the tile takes the gathering path).
 struct TileLoads {
-    int cs, cs32;     // row starts
-    int occ, drift;   // this thread's share of the two block-wide ORs
+    int cs, cs32;          // row starts
+    uint8_t f0, f1;        // drift flags
+    __device__ __forceinline__ int drift() const { return f0 | f1; }
 };
 
-// The drift-flag share of tile_loads.
-__device__ __forceinline__ int tile_drift(const SimDev& S, int c0x, int c0y) {
-    int drift = 0;
-    for (int idx = threadIdx.x; idx < HALO_W * HALO_H; idx += TILE_THREADS) {
+__device__ __forceinline__ void drift_loads(const SimDev& S, int c0x, int c0y, TileLoads& L) {
+    static_assert(HALO_W * HALO_H <= 2 * TILE_THREADS, "two flags per thread");
+    L.f0 = L.f1 = 0;
+    #pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int idx = threadIdx.x + e * TILE_THREADS;
         const int si = c0x - 1 + idx % HALO_W, sj = c0y - 1 + idx / HALO_W;
-        if (si >= 0 && si < S.nx && sj >= 0 && sj < S.ny) drift |= S.cflag[sj * S.nx + si];
+        if (idx < HALO_W * HALO_H && si >= 0 && si < S.nx && sj >= 0 && sj < S.ny)
+            (e ? L.f1 : L.f0) = S.cflag[sj * S.nx + si];
     }
-    return drift;
 }
 
-// tile_loads for a batched tile: the row starts and the occupancy come from
-// its record (rec, in shared memory); only the drift flags are loaded.
+// tile_loads for a batched tile: the row starts come from its record (rec, in
+// shared memory); only the drift flags are loaded.
 __device__ __forceinline__ TileLoads record_loads(const SimDev& S, const TileDesc& rec, int c0x, int c0y,
                                                   int r, int lane) {
     TileLoads L;
     L.cs = rec.cs[r][lane];
     L.cs32 = lane == 0 ? rec.cs[r][32] : 0;
-    L.occ = rec.occ;
-    L.drift = rec.occ ? tile_drift(S, c0x, c0y) : 0;   // an empty tile needs no drift flags
+    drift_loads(S, c0x, c0y, L);
     return L;
 }
 
 __device__ __forceinline__ TileLoads tile_loads(const SimDev& S, int c0x, int c0y, int cj, int lane) {
-    TileLoads L{0, 0, 0, 0};
+    TileLoads L;
+    L.cs = L.cs32 = 0;
     if (cj >= 0 && cj < S.ny) {
         const int base = cj * S.nx;
         L.cs = S.cstart[base + min(max(c0x + lane, 0), S.nx)];
         if (lane == 0) L.cs32 = S.cstart[base + min(max(c0x + 32, 0), S.nx)];
     }
-    const int x0 = max(c0x - 1, 0), x1 = min(c0x + TILE_CX + 1, S.nx);
-    const int y0 = max(c0y - 1, 0), y1 = min(c0y + TILE_CY + 1, S.ny);
-    if (x0 < x1)
-        for (int r = y0 + (int)threadIdx.x; r < y1; r += TILE_THREADS)
-            L.occ |= S.cstart[r * S.nx + x1] != S.cstart[r * S.nx + x0];
-    for (int idx = threadIdx.x; idx < HALO_W * HALO_H; idx += TILE_THREADS) {
-        const int si = c0x - 1 + idx % HALO_W, sj = c0y - 1 + idx / HALO_W;
-        if (si >= 0 && si < S.nx && sj >= 0 && sj < S.ny) L.drift |= S.cflag[sj * S.nx + si];
-    }
+    drift_loads(S, c0x, c0y, L);
     return L;
 }
 
-// Per-warp staging of the chunks of a row: chunk c of [rb, re) holds storage
-// indices rb + 32c + lane; field f of it lands in buf[c % DEPTH][f][lane].
-template <int NF, int DEPTH>
-struct RowStage {
-    float (*buf)[NF][32];
-    const float* src[NF];
-    int rb, re, nch, lane;
-
-    __device__ __forceinline__ void issue(int c) {
-        const int q = rb + 32 * c + lane;
-        if (c < nch && q < re) {
-            #pragma unroll
-            for (int f = 0; f < NF; ++f)
-                if (src[f]) cp_async4(&buf[c % DEPTH][f][lane], src[f] + q);
-        }
-        cp_async_commit();
-    }
-    __device__ __forceinline__ void prime() {
-        #pragma unroll
-        for (int c = 0; c < DEPTH - 1; ++c) issue(c);
-    }
-    // Issue chunk c + DEPTH - 1 and wait until chunk c has landed.
-    __device__ __forceinline__ const float (*advance(int c))[32] {
-        issue(c + DEPTH - 1);
-        cp_async_wait<DEPTH - 1>();
-        return buf[c % DEPTH];
+// Storage range [rb, re) of the warp's cell row and [cb, ce) of the lane's cell.
+struct RowRange {
+    int rb, re, cb, ce;
+    __device__ __forceinline__ RowRange(const TileLoads& L, int lane) {
+        rb = __shfl_sync(0xffffffffu, L.cs, 0);
+        re = __shfl_sync(0xffffffffu, L.cs32, 0);
+        cb = L.cs;
+        const int next = __shfl_down_sync(0xffffffffu, L.cs, 1);
+        ce = lane < 31 ? next : re;
     }
 };
 
@@ -537,47 +515,31 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
     constexpr int NQ = 12;
     __shared__ float s_c[NQ][SC_STRIDE];               // [m, px, py] x corner, per cell
     __shared__ __align__(16) float s_row[TILE_CY][K1_NF][K1_ROW_P];  // staged particles of each cell row
-    __shared__ int s_cs[TILE_CY][33];
     __shared__ TileGeo G;
-    const int parity = (load_step(ctl) + k) & 1;
     const int tid = threadIdx.x, lx = tid & (TILE_CX - 1), ly = tid / TILE_CX;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
     const int ci = c0x + lx, cj = c0y + ly;
+    const TileLoads L = REC ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
+    const int parity = (load_step(ctl) + k) & 1;
     const float* __restrict__ rho = S.rho[parity];
     const bool node_ok = lx < TILE_NX && ly < TILE_NY && c0x + 1 + lx <= S.nx && c0y + 1 + ly <= S.ny;
     const int node = (c0y + 1 + ly) * (S.nx + 1) + c0x + 1 + lx;
     const uint16_t ncons = node_ok ? S.ncons[node] : 0;   // node-phase input, fetched early
-    const TileLoads L = REC ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
-    if (!__syncthreads_or(L.occ)) {
-        // no particle in the tile: every node is massless and keeps its
-        // velocity (the node phase below with all sums zero)
-        if (node_ok) {
-            float vx = flush(S.nvbx[node]), vy = flush(S.nvby[node]);
-            apply_constraint(S, ncons, vx, vy, nullptr, nullptr);
-            S.nm[node] = 0.0f;
-            S.nvax[node] = vx;
-            S.nvay[node] = vy;
-        }
-        return;
-    }
     build_geo(S, c0x, c0y, G);
-    #pragma unroll
-    for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
-    s_cs[ly][lx] = L.cs;
-    if (lx == 0) s_cs[ly][32] = L.cs32;
-    const bool slow = __syncthreads_or(L.drift) != 0;
+    // the row's particles are on their way before the drift flags are known
+    const RowRange R(L, lx);
+    const float* const src[K1_NF] = {S.x, S.y, S.vx, S.vy, REINIT ? rho : S.mass};
+    float (*buf)[K1_ROW_P] = s_row[ly];
+    row_issue16<K1_NF, K1_ROW_P>(buf, src, R.rb & ~3, R.re, lx);
+    const bool slow = __syncthreads_or(L.drift()) != 0;
 
     if (!slow) {
-        const int* cs = s_cs[ly];
-        const int cb = cs[lx], ce = cs[lx + 1];
         const CellGeo g = geo_of(G, lx + 1, ly + 1);
-        const float V0 = (REINIT && ce > cb) ? fdv(S.vol_el, (float)(ce - cb)) : 0.0f;
+        const float V0 = (REINIT && R.ce > R.cb) ? fdv(S.vol_el, (float)(R.ce - R.cb)) : 0.0f;
         float acc[NQ];
         #pragma unroll
         for (int k = 0; k < NQ; ++k) acc[k] = 0.0f;
-        const float* const src[K1_NF] = {S.x, S.y, S.vx, S.vy, REINIT ? rho : S.mass};
-        float (*buf)[K1_ROW_P] = s_row[ly];
-        row_pass16<K1_NF, K1_ROW_P>(buf, src, cs[0], cs[32], cb, ce, lx, [&](int, int j) {
+        row_pass16<K1_NF, K1_ROW_P, true>(buf, src, R.rb, R.re, R.cb, R.ce, lx, [&](int, int j) {
             const float m = REINIT ? fm(V0, buf[4][j]) : buf[4][j];
             float cc[NQ];
             mass_contrib(buf[0][j], buf[1][j], buf[2][j], buf[3][j], m, g.cx, g.rx, g.cy, g.ry, cc);
@@ -586,20 +548,25 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
         });
         #pragma unroll
         for (int k = 0; k < NQ; ++k) s_c[k][tid] = acc[k];
-    } else if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
-        const CellGeo g = geo_of(G, lx + 1, ly + 1);
-        float V0 = 0.0f;
-        if (REINIT) {
-            const int cnt = count_cell(S, ci, cj, g);
-            if (cnt) V0 = fdv(S.vol_el, (float)cnt);
+    } else {
+        cp_async_wait<0>();
+        #pragma unroll
+        for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
+        if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
+            const CellGeo g = geo_of(G, lx + 1, ly + 1);
+            float V0 = 0.0f;
+            if (REINIT) {
+                const int cnt = count_cell(S, ci, cj, g);
+                if (cnt) V0 = fdv(S.vol_el, (float)cnt);
+            }
+            visit_cell(S, ci, cj, g, [&](int q) {
+                const float m = REINIT ? fm(V0, rho[q]) : S.mass[q];
+                float cc[NQ];
+                mass_contrib(S.x[q], S.y[q], S.vx[q], S.vy[q], m, g.cx, g.rx, g.cy, g.ry, cc);
+                #pragma unroll
+                for (int k = 0; k < NQ; ++k) s_c[k][tid] = fa(s_c[k][tid], cc[k]);
+            });
         }
-        visit_cell(S, ci, cj, g, [&](int q) {
-            const float m = REINIT ? fm(V0, rho[q]) : S.mass[q];
-            float cc[NQ];
-            mass_contrib(S.x[q], S.y[q], S.vx[q], S.vy[q], m, g.cx, g.rx, g.cy, g.ry, cc);
-            #pragma unroll
-            for (int k = 0; k < NQ; ++k) s_c[k][tid] = fa(s_c[k][tid], cc[k]);
-        });
     }
     __syncthreads();
     if (node_ok) {
@@ -791,22 +758,22 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
     constexpr int NQ = 8;
     __shared__ __align__(16) ForceShared<MODE, NQ, USL, REINIT> sh;
     auto& s_c = sh.c;                                   // [f x, f y] x corner, per cell
-    __shared__ int s_cs[TILE_CY][33];
     __shared__ float2 s_v[NV_W * NV_H];   // nodal velocity after phase 1 of the tile's nodes
     __shared__ TileGeo G;
-    const int step = load_step(ctl) + k;
-    const int parity = step & 1;
-    const float t = step_time(step, S.dt);
     const int tid = threadIdx.x, lx = tid & (TILE_CX - 1), ly = tid / TILE_CX;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
     const int ci = c0x + lx, cj = c0y + ly;
+    const TileLoads L = VD ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
+    const int step = load_step(ctl) + k;
+    const int parity = step & 1;
+    const float t = step_time(step, S.dt);
     const bool node_ok = lx < TILE_NX && ly < TILE_NY && c0x + 1 + lx <= S.nx && c0y + 1 + ly <= S.ny;
     const int node = (c0y + 1 + ly) * (S.nx + 1) + c0x + 1 + lx;
     // node-phase inputs, fetched early
     const float nmass = node_ok ? S.nm[node] : 0.0f;
     const uint16_t ncons = node_ok ? S.ncons[node] : 0;
     // the node tile (two entries per thread at most) and the tile set-up in
-    // one round trip
+    // one round trip, the geometry meanwhile
     static_assert(NV_W * NV_H <= 2 * TILE_THREADS, "two node-tile entries per thread");
     float2 nv[2];
     #pragma unroll
@@ -819,25 +786,19 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
             nv[e] = make_float2(S.nvax[n], S.nvay[n]);
         }
     }
-    const TileLoads L = VD ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
-    if (!__syncthreads_or(L.occ)) {
-        // no particle in the tile: the nodal update with zero particle forces
-        if (node_ok) nodal_update<VD>(S, node, t, 0.0f, 0.0f, S.nvax[node], S.nvay[node], nmass, ncons);
-        return;
-    }
     build_geo(S, c0x, c0y, G);
+    if constexpr (MODE == FM_STAGED) staged_arrays<USL, REINIT, VD>(S, parity, tid, sh.src);
+    if constexpr (!USL) stage_materials<VD>(S);
     if constexpr (MODE != FM_STAGED) {
         #pragma unroll
         for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
     }
-    s_cs[ly][lx] = L.cs;
-    if (lx == 0) s_cs[ly][32] = L.cs32;
     #pragma unroll
     for (int e = 0; e < 2; ++e)
         if (tid + e * TILE_THREADS < NV_W * NV_H) s_v[tid + e * TILE_THREADS] = nv[e];
-    if constexpr (MODE == FM_STAGED) staged_arrays<USL, REINIT, VD>(S, parity, tid, sh.src);
-    if constexpr (!USL) stage_materials<VD>(S);
-    const bool slow = __syncthreads_or(L.drift) != 0;
+    const RowRange R(L, lx);
+    const int rb = R.rb, re = R.re, cb = R.cb, ce = R.ce;
+    const bool slow = __syncthreads_or(L.drift()) != 0;
 
     auto cell_velocities = [&](int li, int lj, float* vx, float* vy) {
         const int a = lj * NV_W + li;
@@ -856,8 +817,6 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
         float (*buf)[F::P] = sh.buf[ly];
         auto& s_cell = sh.cell;
         auto& s_cellv = sh.cellv;
-        const int* cs = s_cs[ly];
-        const int rb = cs[0], re = cs[32], cb = cs[lx], ce = cs[lx + 1];
         {
             float nvx[4], nvy[4], V0, size0, dvol;
             if (!USL) cell_velocities(lx, ly, nvx, nvy);
@@ -926,7 +885,6 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
         for (int q = 0; q < NQ; ++q) s_c[q][tid] = acc[q];
       } else if constexpr (MODE == FM_LPC) {
         if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
-            const int cb = s_cs[ly][lx], ce = s_cs[ly][lx + 1];
             const CellGeo g = geo_of(G, lx + 1, ly + 1);
             float nvx[4], nvy[4], V0, size0, dvol;
             if (!USL) cell_velocities(lx, ly, nvx, nvy);
@@ -954,9 +912,6 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
         auto& s_slot = sh.rows.slot;
         auto& s_cell = sh.rows.cell;
         auto& s_cellv = sh.rows.cellv;
-        const int* cs = s_cs[ly];
-        const int rb = cs[0], re = cs[32];
-        const int cb = cs[lx], ce = cs[lx + 1];
         {
             float nvx[4], nvy[4], V0, size0, dvol;
             if (!USL) cell_velocities(lx, ly, nvx, nvy);
@@ -1224,28 +1179,39 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
     __shared__ int s_flag[TILE_CY][32];   // drift flag after this step
     __shared__ int s_status;
     __shared__ TileGeo G;
-    const int step = load_step(ctl) + k;
-    const int parity = step & 1, next = parity ^ 1;
     const int tid = threadIdx.x, lane = tid & 31, w = tid / 32;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
     // row w + 1 of the tile: owned sort-cells c0x+1 .. c0x+31 -> starts cs[0..31]
     const int sj = c0y + 1 + w;
     const bool row_ok = w < TILE_NY && sj < S.ny;
-    int rb = 0, re = 0;
-    unsigned sfmask = 0;   // bit l: sort-cell c0x + 1 + l had a drifted particle at the step start
-    if (row_ok) {
-        // (a batched tile's row starts come with its record: row w + 1,
-        // column lane + 1 of the record's table)
-        const int col = min(c0x + 1 + lane, S.nx);
-        s_cs[w][lane] = REC ? rec->cs[w + 1][lane + 1] : S.cstart[sj * S.nx + col];
-        sfmask = __ballot_sync(0xffffffffu, col < S.nx && S.cflag[sj * S.nx + col] != 0);
+    const int col = min(c0x + 1 + lane, S.nx);
+    // (a batched tile's row starts come with its record: row w + 1,
+    // column lane + 1 of the record's table)
+    const int cs_l = row_ok ? (REC ? rec->cs[w + 1][lane + 1] : S.cstart[sj * S.nx + col]) : 0;
+    const uint8_t fl = row_ok && col < S.nx ? S.cflag[sj * S.nx + col] : 0;
+    // the node tile, both entries of a thread in flight together and with the
+    // row starts and the rows' first chunks
+    static_assert(G_W * G_H <= 2 * TILE_THREADS, "two node-tile entries per thread");
+    float4 nd[2];
+    #pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int idx = tid + e * TILE_THREADS;
+        const int I = c0x + idx % G_W, J = c0y + idx / G_W;
+        nd[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (idx < G_W * G_H && I >= 0 && I <= S.nx && J >= 0 && J <= S.ny) {
+            const int n = J * (S.nx + 1) + I;
+            nd[e] = make_float4(S.nvbx[n], S.nvby[n], S.nax[n], S.nay[n]);
+        }
     }
+    const int step = load_step(ctl) + k;
+    const int parity = step & 1, next = parity ^ 1;
+    if (tid == 0) s_status = 0;
     s_flag[w][lane] = 0;
+    s_cs[w][lane] = cs_l;
+    // bit l: sort-cell c0x + 1 + l had a drifted particle at the step start
+    const unsigned sfmask = __ballot_sync(0xffffffffu, fl != 0);
+    const int rb = __shfl_sync(0xffffffffu, cs_l, 0), re = __shfl_sync(0xffffffffu, cs_l, 31);
     __syncwarp();
-    if (row_ok) {
-        rb = s_cs[w][0];
-        re = s_cs[w][31];
-    }
     const float* src[NF] = {S.x, S.y, S.vx, S.vy};
     if constexpr (USL) {
         src[GF_SXX] = S.sxx[parity];
@@ -1262,33 +1228,11 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
     RowStage16<NF, DEPTH> st(&s_stage[w][0][0][0], src, rb, re, lane);
     const int rb4 = st.rb4;
     st.prime();
+    build_geo(S, c0x, c0y, G);
     if constexpr (USL) stage_materials<false>(S);
-    if (!__syncthreads_or(re > rb)) {
-        // no particle stored in the tile's sort-cells: their drift flags clear
-        if (row_ok && lane < TILE_NX && c0x + 1 + lane < S.nx) S.cflag[sj * S.nx + c0x + 1 + lane] = 0;
-        return;
-    }
-    if (tid == 0) s_status = 0;
-    {
-        // the node tile, both entries of a thread in flight together (and in
-        // flight with the rows' first chunks)
-        static_assert(G_W * G_H <= 2 * TILE_THREADS, "two node-tile entries per thread");
-        float4 nd[2];
-        #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int idx = tid + e * TILE_THREADS;
-            const int I = c0x + idx % G_W, J = c0y + idx / G_W;
-            nd[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (idx < G_W * G_H && I >= 0 && I <= S.nx && J >= 0 && J <= S.ny) {
-                const int n = J * (S.nx + 1) + I;
-                nd[e] = make_float4(S.nvbx[n], S.nvby[n], S.nax[n], S.nay[n]);
-            }
-        }
-        build_geo(S, c0x, c0y, G);
-        #pragma unroll
-        for (int e = 0; e < 2; ++e)
-            if (tid + e * TILE_THREADS < G_W * G_H) s_nd[tid + e * TILE_THREADS] = nd[e];
-    }
+    #pragma unroll
+    for (int e = 0; e < 2; ++e)
+        if (tid + e * TILE_THREADS < G_W * G_H) s_nd[tid + e * TILE_THREADS] = nd[e];
     if (row_ok && lane < TILE_NX) {
         // storage index rb + j of the row holds a particle of sort-cell s_map[j]
         const int lo = s_cs[w][lane] - rb, hi = min(s_cs[w][lane + 1] - rb, G2P_MAP);
