@@ -263,7 +263,8 @@ int launch_phase(MpmHandle* h, int phase, int k, cudaStream_t s) {
     const StepConfig c = step_config(h);
     cudaError_t e = cudaSuccess;
     if (phase == 0) {
-        CK(h, launch_empty_nodes(h->hs, h->d_empty, h->nemp, h->ctl, k, s));
+        if (empty_nodes_due(k, h->hs.cnf_ptr != nullptr))
+            CK(h, launch_empty_nodes(h->hs, h->d_empty, h->nemp, h->ctl, k, s));
         e = launch_nodal_kinematics(c, h->hs, h->step_tiles, h->nact, h->ctl, k, s);
     } else if (phase == 1) {
         e = launch_forces(c, h->hs, h->step_tiles, h->nact, h->ctl, k, s);

@@ -73,8 +73,10 @@ int prepare_tiles(MpmBatch* b, cudaStream_t s) {
 }
 
 int launch_batch_steps(MpmBatch* b, int n, cudaStream_t s) {
+    bool forces = false;
+    for (const MpmHandle* h : b->sims) forces = forces || h->hs.cnf_ptr;
     for (int i = 0; i < n; ++i) {
-        BCK(b, launch_empty_nodes_batch(b->d_edescs, b->nemp, i, s));
+        if (empty_nodes_due(i, forces)) BCK(b, launch_empty_nodes_batch(b->d_edescs, b->nemp, i, s));
         BCK(b, launch_nodal_kinematics_batch(b->cfg, b->d_tdescs, b->nact, i, s));
         BCK(b, launch_forces_batch(b->cfg, b->d_tdescs, b->nact, i, s));
         BCK(b, launch_particle_kinematics_batch(b->cfg, b->d_tdescs, b->nact, i, s));

@@ -57,7 +57,7 @@ int check_ready(MpmBatch* b);
 // not inside a stream capture.
 int prepare_tiles(MpmBatch* b, cudaStream_t s);
 // n steps of every simulation as 3n batched launches over the active tiles
-// plus one over the empty tiles per step (no status handling).
+// plus those over the empty tiles that are due (no status handling).
 int launch_batch_steps(MpmBatch* b, int n, cudaStream_t s);
 // Copy a host argument table into b->d_table (valid until the next upload on
 // the stream).
