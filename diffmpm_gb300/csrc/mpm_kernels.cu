@@ -112,40 +112,6 @@ cudaError_t launch_advance_step(Control* ctl, int by, cudaStream_t s) {
 }
 
 
-// Visit, in a fixed order, the particles whose current cell is (ci, cj):
-// sort-cells (ci+di, cj+dj) row by row; a neighbour is scanned only when its
-// drift flag is set, and particles of a flagged sort-cell are tested.
-template <class F>
-__device__ __forceinline__ void visit_cell(const SimDev& S, int ci, int cj, const CellGeo& g,
-                                           F&& f) {
-    const int nx = S.nx, ny = S.ny;
-    #pragma unroll 1
-    for (int dj = -1; dj <= 1; ++dj) {
-        const int sj = cj + dj;
-        if (sj < 0 || sj >= ny) continue;
-        #pragma unroll 1
-        for (int di = -1; di <= 1; ++di) {
-            const int si = ci + di;
-            if (si < 0 || si >= nx) continue;
-            const int s = sj * nx + si;
-            const bool flagged = S.cflag[s] != 0;
-            if (!(di == 0 && dj == 0) && !flagged) continue;
-            const int b = S.cstart[s], e = S.cstart[s + 1];
-            #pragma unroll 1
-            for (int q = b; q < e; ++q) {
-                if (flagged && !in_cell(g, S.x[q], S.y[q])) continue;
-                f(q);
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ int count_cell(const SimDev& S, int ci, int cj, const CellGeo& g) {
-    int n = 0;
-    visit_cell(S, ci, cj, g, [&](int) { ++n; });
-    return n;
-}
-
 __device__ __forceinline__ void cell_nodes(const SimDev& S, int ci, int cj, int ids[4]) {
     const int ll = cj * (S.nx + 1) + ci;
     ids[0] = ll;
@@ -309,6 +275,78 @@ struct RowRange {
         ce = lane < 31 ? next : re;
     }
 };
+
+// The gathering path's shared memory: the drift flags and storage starts of the
+// sort-cells [c0x-1, c0x+33) x [c0y-1, c0y+17), and per cell of the tile the
+// storage slots of the particles found in it.  A cell's particles are found
+// twice (their count sets the cell's volume, then they contribute); with the
+// flags, starts and slots in global memory each visit was a chain of some
+// twenty dependent loads (a thrown block of 38k particles: nodal kinematics
+// 16.1 us and forces 16.7 us a step, where undrifted tiles take 6 and 10).
+constexpr int GATHER_SLOTS = 12;
+struct GatherTile {
+    uint8_t flag[HALO_H][HALO_W];
+    int start[HALO_H][HALO_W + 1];
+    int slot[GATHER_SLOTS][TILE_THREADS];
+};
+
+__device__ __forceinline__ void gather_setup(const SimDev& S, int c0x, int c0y, const TileLoads& L,
+                                             GatherTile& W) {
+    #pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int idx = threadIdx.x + e * TILE_THREADS;
+        if (idx < HALO_W * HALO_H) (&W.flag[0][0])[idx] = e ? L.f1 : L.f0;
+    }
+    for (int idx = threadIdx.x; idx < HALO_H * (HALO_W + 1); idx += TILE_THREADS) {
+        const int r = idx / (HALO_W + 1), sj = c0y - 1 + r, si = c0x - 1 + idx - r * (HALO_W + 1);
+        W.start[r][si - c0x + 1] = sj >= 0 && sj < S.ny ? S.cstart[sj * S.nx + min(max(si, 0), S.nx)] : 0;
+    }
+    __syncthreads();
+}
+
+// Visit, in a fixed order, the particles whose current cell is the tile's cell
+// (lx, ly), geometry g: the sort-cells around it row by row; a neighbour is
+// scanned only when its drift flag is set, and particles of a flagged
+// sort-cell are tested.  (Sort-cells off the mesh are never flagged.)
+template <class F>
+__device__ __forceinline__ void visit_cell(const SimDev& S, const GatherTile& W, int lx, int ly,
+                                           const CellGeo& g, F&& f) {
+    #pragma unroll 1
+    for (int r = ly; r < ly + 3; ++r) {
+        #pragma unroll 1
+        for (int c = lx; c < lx + 3; ++c) {
+            const bool flagged = W.flag[r][c] != 0;
+            if (!(r == ly + 1 && c == lx + 1) && !flagged) continue;
+            const int b = W.start[r][c], e = W.start[r][c + 1];
+            #pragma unroll 1
+            for (int q = b; q < e; ++q) {
+                if (flagged && !in_cell(g, S.x[q], S.y[q])) continue;
+                f(q);
+            }
+        }
+    }
+}
+
+// The number of those particles, with the first GATHER_SLOTS slots kept ...
+__device__ __forceinline__ int gather_cell(const SimDev& S, GatherTile& W, int lx, int ly, const CellGeo& g) {
+    int n = 0;
+    visit_cell(S, W, lx, ly, g, [&](int q) {
+        if (n < GATHER_SLOTS) W.slot[n][threadIdx.x] = q;
+        ++n;
+    });
+    return n;
+}
+// ... and f of each of the n, in the same order.
+template <class F>
+__device__ __forceinline__ void for_gathered(const SimDev& S, const GatherTile& W, int lx, int ly,
+                                             const CellGeo& g, int n, F&& f) {
+    if (n > GATHER_SLOTS) {
+        visit_cell(S, W, lx, ly, g, f);
+    } else {
+        #pragma unroll 1
+        for (int i = 0; i < n; ++i) f(W.slot[i][threadIdx.x]);
+    }
+}
 
 // Per-particle contributions of phase 1 to the 4 corners of its cell:
 // [m N_k, N_k (m vx), N_k (m vy)] (element.py:138-152, 170-189).  `m` is the
@@ -514,7 +552,10 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
                                                       const TileDesc* rec = nullptr) {
     constexpr int NQ = 12;
     __shared__ float s_c[NQ][SC_STRIDE];               // [m, px, py] x corner, per cell
-    __shared__ __align__(16) float s_row[TILE_CY][K1_NF][K1_ROW_P];  // staged particles of each cell row
+    __shared__ union {
+        __align__(16) float row[TILE_CY][K1_NF][K1_ROW_P];   // staged particles of each cell row
+        GatherTile gather;
+    } sh;
     __shared__ TileGeo G;
     const int tid = threadIdx.x, lx = tid & (TILE_CX - 1), ly = tid / TILE_CX;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
@@ -529,7 +570,7 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
     // the row's particles are on their way before the drift flags are known
     const RowRange R(L, lx);
     const float* const src[K1_NF] = {S.x, S.y, S.vx, S.vy, REINIT ? rho : S.mass};
-    float (*buf)[K1_ROW_P] = s_row[ly];
+    float (*buf)[K1_ROW_P] = sh.row[ly];
     row_issue16<K1_NF, K1_ROW_P>(buf, src, R.rb & ~3, R.re, lx);
     const bool slow = __syncthreads_or(L.drift()) != 0;
 
@@ -550,16 +591,15 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
         for (int k = 0; k < NQ; ++k) s_c[k][tid] = acc[k];
     } else {
         cp_async_wait<0>();
+        __syncthreads();   // the staged rows are dropped
+        gather_setup(S, c0x, c0y, L, sh.gather);
         #pragma unroll
         for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
         if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
             const CellGeo g = geo_of(G, lx + 1, ly + 1);
-            float V0 = 0.0f;
-            if (REINIT) {
-                const int cnt = count_cell(S, ci, cj, g);
-                if (cnt) V0 = fdv(S.vol_el, (float)cnt);
-            }
-            visit_cell(S, ci, cj, g, [&](int q) {
+            const int cnt = gather_cell(S, sh.gather, lx, ly, g);
+            const float V0 = REINIT && cnt ? fdv(S.vol_el, (float)cnt) : 0.0f;
+            for_gathered(S, sh.gather, lx, ly, g, cnt, [&](int q) {
                 const float m = REINIT ? fm(V0, rho[q]) : S.mass[q];
                 float cc[NQ];
                 mass_contrib(S.x[q], S.y[q], S.vx[q], S.vy[q], m, g.cx, g.rx, g.cy, g.ry, cc);
@@ -697,22 +737,30 @@ struct StagedFields {
     static constexpr int P = 132;
 };
 
-// Shared memory of forces_tile by mode.  FM_STAGED overlays the per-cell
-// corner sums on the staged rows (they are formed after every row is done).
+// Shared memory of forces_tile by mode; the gathering path's tables overlay the
+// row buffers.  FM_STAGED overlays the per-cell corner sums on the staged rows
+// (they are formed after every row is done).
 template <int MODE, int NQ, bool USL, bool REINIT>
 struct ForceShared {
     float c[NQ][SC_STRIDE];
-    ForceRows<NQ> rows;
+    union {
+        ForceRows<NQ> rows;
+        GatherTile gather;
+    };
 };
 template <int NQ, bool USL, bool REINIT>
 struct ForceShared<FM_LPC, NQ, USL, REINIT> {
     float c[NQ][SC_STRIDE];
+    GatherTile gather;
 };
 template <int NQ, bool USL, bool REINIT>
 struct ForceShared<FM_STAGED, NQ, USL, REINIT> {
     using F = StagedFields<USL, REINIT>;
     union {
-        float c[NQ][SC_STRIDE];
+        struct {
+            float c[NQ][SC_STRIDE];
+            GatherTile gather;
+        };
         __align__(16) float buf[TILE_CY][F::NBUF][F::P];
     };
     unsigned char cell[TILE_CY][F::P];   // a staged particle's cell within the row
@@ -956,18 +1004,19 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
         for (int k = 0; k < NQ; ++k) s_c[k][tid] = acc[k];
       }
     } else {
+        gather_setup(S, c0x, c0y, L, sh.gather);
         if constexpr (MODE == FM_STAGED) {
             #pragma unroll
             for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
         }
         if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
             const CellGeo g = geo_of(G, lx + 1, ly + 1);
-            const int cnt = REINIT ? count_cell(S, ci, cj, g) : 0;
+            const int cnt = gather_cell(S, sh.gather, lx, ly, g);
             float nvx[4], nvy[4], V0, size0, dvol;
             if (!USL) cell_velocities(lx, ly, nvx, nvy);
             force_cell_values<USL, REINIT, VD, TRAC>(S, cnt, g, nvx, nvy, V0, size0, dvol);
             const bool own = lx >= 1 && ly >= 1;
-            visit_cell(S, ci, cj, g, [&](int q) {
+            for_gathered(S, sh.gather, lx, ly, g, cnt, [&](int q) {
                 float cc[NQ];
                 force_contrib<USL, REINIT, TRAC, VD>(S, q, force_in_global<VD>(S, q, parity, REINIT), g.cx,
                                                  g.rx, g.cy, g.ry, V0, size0, nvx, nvy, dvol, parity,
