@@ -64,6 +64,7 @@ void bind_particles(MpmHandle* h) {
     SimDev& s = h->hs;
     s.np = (int)h->np;
     s.x = p.x; s.y = p.y; s.vx = p.vx; s.vy = p.vy;
+    s.xo = p.x; s.yo = p.y; s.vxo = p.vx; s.vyo = p.vy;
     for (int k = 0; k < 2; ++k) {
         s.sxx[k] = p.sxx[k]; s.syy[k] = p.syy[k]; s.szz[k] = p.szz[k]; s.sxy[k] = p.sxy[k];
         s.rho[k] = p.rho[k]; s.vsc[k] = p.vsc[k]; s.vol[k] = p.vol[k];
@@ -79,7 +80,7 @@ void bind_particles(MpmHandle* h) {
     s.pvc_vel = h->d_pvc_vel;
     s.pid = p.pid;
     s.cstart = h->cstart[h->cs_cur];
-    s.cflag = h->cflag;
+    s.cflag = s.cflago = h->cflag;
 }
 
 int parity(const MpmHandle* h) { return (int)(h->step & 1); }
@@ -258,18 +259,19 @@ StepKey step_key(const MpmHandle* h) {
 
 // One phase of step (ctl->step + k) over the active tiles (the empty tiles'
 // nodes are updated with the nodal kinematics); phase 2 ends the step, whose
-// counter the caller advances.
-int launch_phase(MpmHandle* h, int phase, int k, cudaStream_t s) {
+// counter the caller advances.  S is the handle's descriptor, or one that
+// points at tape slots (the empty tiles' nodes are always the handle's).
+int launch_phase(MpmHandle* h, const SimDev& S, int phase, int k, cudaStream_t s) {
     const StepConfig c = step_config(h);
     cudaError_t e = cudaSuccess;
     if (phase == 0) {
         if (empty_nodes_due(k, h->hs.cnf_ptr != nullptr))
             CK(h, launch_empty_nodes(h->hs, h->d_empty, h->nemp, h->ctl, k, s));
-        e = launch_nodal_kinematics(c, h->hs, h->step_tiles, h->nact, h->ctl, k, s);
+        e = launch_nodal_kinematics(c, S, h->step_tiles, h->nact, h->ctl, k, s);
     } else if (phase == 1) {
-        e = launch_forces(c, h->hs, h->step_tiles, h->nact, h->ctl, k, s);
+        e = launch_forces(c, S, h->step_tiles, h->nact, h->ctl, k, s);
     } else {
-        e = launch_particle_kinematics(c, h->hs, h->step_tiles, h->nact, h->ctl, k, s);
+        e = launch_particle_kinematics(c, S, h->step_tiles, h->nact, h->ctl, k, s);
     }
     CK(h, e);
     return MPM_OK;
@@ -277,7 +279,7 @@ int launch_phase(MpmHandle* h, int phase, int k, cudaStream_t s) {
 
 int launch_steps(MpmHandle* h, int n, cudaStream_t s) {
     for (int i = 0; i < n; ++i)
-        for (int p = 0; p < 3; ++p) TRY(launch_phase(h, p, i, s));
+        for (int p = 0; p < 3; ++p) TRY(launch_phase(h, h->hs, p, i, s));
     CK(h, launch_advance_step(h->ctl, n, s));
     return MPM_OK;
 }
@@ -746,7 +748,8 @@ int mpm_create(const MpmDesc* d, MpmHandle** out) {
     s.cnf_ptr = h->d_cnf_ptr; s.cnf_dir = h->d_cnf_dir; s.cnf_val = h->d_cnf_val; s.cnf_fn = h->d_cnf_fn;
     s.nfn = h->nfn; s.fn_off = h->d_fn_off; s.fn_x = h->d_fn_x; s.fn_y = h->d_fn_y;
     s.nmat = h->nmat; s.mats = h->d_mats;
-    s.cstart = h->cstart[0]; s.cflag = h->cflag;
+    s.cstart = h->cstart[0]; s.cflag = s.cflago = h->cflag;
+    s.nvpx = h->nvbx; s.nvpy = h->nvby;
     if (upload_desc(h) != MPM_OK) {
         g_create_error = h->err;
         return bail(MPM_ERR_CUDA);
@@ -1186,7 +1189,7 @@ int mpm_run_phase(MpmHandle* h, int phase, void* stream) {
     cudaStream_t s = S(stream);
     if (phase == 0 && h->needs_resort) TRY(resort(h, s));
     if (phase == 0) TRY(classify_tiles(h, s));
-    TRY(launch_phase(h, phase, 0, s));
+    TRY(launch_phase(h, h->hs, phase, 0, s));
     if (phase == 2) {
         CK(h, launch_advance_step(h->ctl, 1, s));
         h->step++;
@@ -1273,7 +1276,7 @@ int mpm_time_phases(MpmHandle* h, int nsteps, float* ms_out, void* stream) {
     CK(h, cudaEventRecord(ev[0], s));
     for (int i = 0; i < nsteps && r == MPM_OK; ++i)
         for (int p = 0; p < 3 && r == MPM_OK; ++p) {
-            r = launch_phase(h, p, 0, s);
+            r = launch_phase(h, h->hs, p, 0, s);
             if (r == MPM_OK && p == 2) CK(h, launch_advance_step(h->ctl, 1, s));
             if (r == MPM_OK) CK(h, cudaEventRecord(ev[3 * i + p + 1], s));
         }
@@ -1331,6 +1334,12 @@ int mpm_set_empty_split(MpmHandle* h, int min_empty) {
     if (!h) return MPM_ERR_INVALID;
     if (min_empty < 0) return fail(h, MPM_ERR_INVALID, "min_empty is negative");
     h->empty_split_min = min_empty;   // applies from the next classification
+    return MPM_OK;
+}
+
+int mpm_set_tape_limit(MpmHandle* h, int64_t bytes) {
+    if (!h) return MPM_ERR_INVALID;
+    h->tape_limit = bytes;   // applies from the next mpm_record
     return MPM_OK;
 }
 

@@ -1,34 +1,41 @@
-// Differentiation of the explicit step: a checkpointed forward run
-// (mpm_record) and the hand-written discrete adjoint (mpm_adjoint).
+// Differentiation of the explicit step: a recorded forward run (mpm_record) and
+// the hand-written discrete adjoint (mpm_adjoint).
 //
-// mpm_record advances like mpm_step and keeps a full copy of the simulation
-// state at the start of every segment of K steps (and at the end), plus the
-// steps before which the particles were re-sorted.  mpm_adjoint walks the
-// segments backwards: it restores the segment's checkpoint, re-runs its K
-// steps while copying each step's start state and nodal results into a tape
-// (re-sorting at the recorded steps, so the storage order of every step
-// matches the recorded run), then runs the four reverse passes of
-// mpm_adjoint.h for each step from the last to the first.  A segment without
-// a re-sort re-runs and reverses as two cached CUDA graphs; one with a
-// re-sort goes step by step.  The adjoint arrays
-// follow the storage order of the step being reversed; where a re-sort
-// separates two steps they are permuted through the original particle order,
-// and after a segment they are left in the order of its checkpoint, which is
-// the order the re-run of the previous segment ends in (the re-run is checked
-// to reproduce the recorded state bit for bit).
-// Memory: one checkpoint per segment (the particle state, cell starts and
-// persistent nodal velocity) and a tape of K steps (9 floats per particle, 7
-// per node and 1 byte per cell per step; one more float per particle for the
-// volume under solve semantics and one for the volumetric strain of a run
-// with Newtonian particles).
+// The tape holds, for a run of consecutive steps, each step's start state and
+// nodal results.  Taped steps write it as they go: a step's kernels read the
+// particles from its slot and write them to the next one, and write the nodal
+// results to its slot, so a tape costs no copies but the first slot of a block
+// and the nodes of its last (as copies around every step it was a third of the
+// forward time).  The last step of a block writes the handle's own arrays,
+// where re-sorts, snapshots and reads find the state.
+//
+// mpm_record tapes the whole run when that fits a bounded share of the device
+// memory; mpm_adjoint then only runs the reverse passes of mpm_adjoint.h from
+// the last step to the first.  A longer run is cut into segments of K steps,
+// with a full copy of the state at the start of every segment (and at the
+// end) and the steps before which the particles were re-sorted: record tapes
+// the last segment, and mpm_adjoint restores each earlier one's checkpoint,
+// re-runs its steps with the tape (re-sorting at the recorded steps, so the
+// storage order of every step matches the recorded run, and checking that it
+// ends bit for bit in the next checkpoint) and reverses it.
+// The adjoint arrays follow the storage order of the step being reversed;
+// where a re-sort separates two steps they are permuted through the original
+// particle order, and after a segment they are left in the order of its
+// checkpoint, which is the order the previous segment ends in.
+// Memory: per taped step 9 floats per particle, 7 per node and 1 byte per cell
+// (one more float per particle for the volume under solve semantics and one
+// for the volumetric strain of a run with Newtonian particles), the material
+// ids, moduli and cell starts of each sort, and one checkpoint per segment when
+// there are several.
 //
 // mpm_batch_record / mpm_batch_adjoint do the same for every simulation of a
-// batch in lockstep: each re-run step, tape copy and reverse pass is one
-// launch for all simulations (segmented copies with a slot offset, and the
-// reverse passes over a table of per-simulation arguments).
+// batch in lockstep: each step and reverse pass is one launch for all
+// simulations (the tile records carry the tape, and the reverse passes work
+// over a table of per-simulation arguments).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <map>
 #include <vector>
 
@@ -64,22 +71,30 @@ struct Epoch {               // arrays of one sort epoch inside a segment
 
 }  // namespace
 
-// The segment graphs of one configuration of the step launches: the re-run
-// with its tape copies (keyed by 2 * length + start parity) and the reverse
-// steps (keyed by length).
+using GraphKey = std::array<int64_t, 4>;
+// Executable graphs by what varies between them; a null entry has run once
+// without a graph (the second time captures it: a run that happens once does
+// not pay for capturing).
+using GraphMap = std::map<GraphKey, cudaGraphExec_t>;
+
+// The graphs of one configuration of the step launches: taped runs of steps
+// (first slot, length, parity) and reverse runs (first and last slot, sort
+// epoch, tiles), with the copy tables of the handle's buffers.
 struct AdjGraphs {
     StepKey key;
-    std::map<int64_t, cudaGraphExec_t> rerun, rev;
-    SegBuf tp[2], tn;          // tape copy tables of the re-run graphs
+    GraphMap fwd, rev;
+    SegBuf tp[2], tn;          // slot copies of the start state (by parity) and of the nodal results
 };
 
 struct AdjointState {
-    int K = 0, nseg = 0;
+    int interval = 0;          // the checkpoint interval asked for
+    int K = 0, nseg = 0;       // the segments kept: K steps each, nseg of them
     int64_t step0 = 0, nsteps = 0;
     uint64_t gen = 0;
     bool valid = false, recording = false;
     std::vector<int64_t> resort_steps;
-    std::vector<Checkpoint> ck;   // ck[s]: start of segment s; ck[nseg]: end state
+    std::vector<Checkpoint> ck;   // ck[s]: start of segment s; ck[nseg]: end state (several segments)
+    int tape_seg = -1;         // the segment whose steps the tape holds, or -1
     // sized for np_alloc particles and tape_slots steps
     int64_t np_alloc = -1;
     int tape_slots = 0;
@@ -91,7 +106,13 @@ struct AdjointState {
     std::vector<Epoch> epochs;
     std::vector<int> epoch_of;
     int nep = 0;               // epochs captured in the current segment
-    int64_t seg_first = 0;     // first step of the segment being reversed
+    int64_t seg_first = 0;     // first step of the taped segment
+    // the tiles with particles in any sort of the taped segment (the reverse
+    // node passes' list), valid while every run had its empty tiles apart
+    int* tile_union = nullptr;
+    int4 *rtiles = nullptr, *rempty = nullptr;
+    int nrtiles = -1;          // grid over rtiles; -1: not formed since the segment was taped
+    bool all_tiles = false;
     float* lam[NLAM] = {};
     float* lam_tmp = nullptr;
     float* pscr[NPS] = {};
@@ -99,34 +120,43 @@ struct AdjointState {
     int* cnt = nullptr;
     int* mismatch = nullptr;   // device counter of the re-run check
     int* h_mismatch = nullptr; // pinned
-    // CUDA graphs of whole segments without a re-sort, for the most recently
-    // used configurations first; dropped whenever a buffer here is
-    // (re)allocated.
+    // for the most recently used configurations first; dropped whenever a
+    // buffer here is (re)allocated
     std::vector<AdjGraphs> graphs;
 };
 
-// Scratch of a batched adjoint (owned by the batch).
+// Scratch of a batched record and adjoint (owned by the batch).
 struct BatchAdjoint {
     AdjStep* d_bases = nullptr;
     AdjStep* d_table = nullptr;
     std::vector<AdjStep> bases;
     int2* part_blocks = nullptr;
     int n_part_blocks = 0;
-    SegBuf tape_p[2], tape_n, misc;
+    TapeDev* d_tapes = nullptr;
+    SegBuf misc;
     int* mismatch = nullptr;
     int* h_mismatch = nullptr;
-    // graphs of one-epoch segments: the re-run (keyed by length and tile
-    // counts) and the reverse steps (length, tiles, particle blocks); valid
-    // for the buffers and kernel builds in `gsig`
-    std::map<int64_t, cudaGraphExec_t> g_rerun, g_rev;
+    // the tiles with particles in any sort of the taped segment
+    int* tile_union = nullptr;
+    int4 *rtiles = nullptr, *rempty = nullptr;
+    int nrtiles = -1;
+    // graphs of the reverse steps (first and last slot, tiles, particle
+    // blocks), valid for the buffers in `gsig`
+    GraphMap g_rev;
     std::vector<uintptr_t> gsig;
 };
 
 namespace {
 
+void free_graphs(GraphMap& m) {
+    for (auto& kv : m)
+        if (kv.second) cudaGraphExecDestroy(kv.second);
+    m.clear();
+}
+
 void free_adj_graphs(AdjGraphs& g) {
-    for (auto& kv : g.rerun) cudaGraphExecDestroy(kv.second);
-    for (auto& kv : g.rev) cudaGraphExecDestroy(kv.second);
+    free_graphs(g.fwd);
+    free_graphs(g.rev);
     for (SegBuf& b : g.tp) segbuf_free(b);
     segbuf_free(g.tn);
 }
@@ -136,10 +166,8 @@ void drop_adj_graphs(AdjointState* a) {
     a->graphs.clear();
 }
 
-void free_buffers(MpmHandle* h, AdjointState* a) {
+void free_tape(MpmHandle* h, AdjointState* a) {
     drop_adj_graphs(a);
-    for (auto& c : a->ck) checkpoint_free(h, c);
-    a->ck.clear();
     for (float*& p : a->tp) { dfree(h, p); p = nullptr; }
     for (float*& p : a->tn) { dfree(h, p); p = nullptr; }
     dfree(h, a->tvol);
@@ -149,6 +177,18 @@ void free_buffers(MpmHandle* h, AdjointState* a) {
     dfree(h, a->tflag);
     a->tflag = nullptr;
     a->tape_slots = 0;
+    a->tape_seg = -1;
+}
+
+void free_buffers(MpmHandle* h, AdjointState* a) {
+    free_tape(h, a);
+    for (auto& c : a->ck) checkpoint_free(h, c);
+    a->ck.clear();
+    dfree(h, a->tile_union);
+    dfree(h, a->rtiles);
+    dfree(h, a->rempty);
+    a->tile_union = nullptr;
+    a->rtiles = a->rempty = nullptr;
     for (Epoch& e : a->epochs) {
         dfree(h, e.pid);
         dfree(h, e.mat);
@@ -202,31 +242,39 @@ int restore_checkpoint(MpmHandle* h, Checkpoint& c, cudaStream_t s) {
 // Particle slots between consecutive tape slots (np rounded up to 4).
 size_t tape_stride(const MpmHandle* h) { return ((size_t)h->np + 3) & ~(size_t)3; }
 
-int ensure_adjoint_buffers(MpmHandle* h, AdjointState* a, int slots, cudaStream_t s) {
-    // particle arrays and tape slots hold a multiple of 4 slots, so that every
-    // slot starts on a 16-byte boundary for the reverse node passes' 16-byte
-    // row staging (which may read up to 3 slots past a row's end)
-    const size_t np = ((size_t)h->np + 3) & ~(size_t)3, nn = (size_t)h->nn;
-    bool newtonian = false;
-    for (const MatDev& m : h->mats) newtonian = newtonian || m.type == MAT_NEWTONIAN;
-    if (a->tape_slots < slots || (!h->reinit && !a->tvol) || (newtonian && !a->tvsc)) {
-        drop_adj_graphs(a);
-        for (float*& p : a->tp) { dfree(h, p); p = nullptr; }
-        dfree(h, a->tvol);
-        a->tvol = nullptr;
-        dfree(h, a->tvsc);
-        a->tvsc = nullptr;
-        for (float*& p : a->tn) { dfree(h, p); p = nullptr; }
-        dfree(h, a->tflag);
-        a->tflag = nullptr;
-        a->tape_slots = 0;
+bool newtonian(const MpmHandle* h) {
+    for (const MatDev& m : h->mats)
+        if (m.type == MAT_NEWTONIAN) return true;
+    return false;
+}
+
+// A tape of `slots` steps.  Particle arrays and tape slots hold a multiple of
+// 4 slots, so that every slot starts on a 16-byte boundary for the row staging
+// of the step kernels and the reverse node passes (which may read up to 3
+// slots past a row's end).
+int ensure_tape(MpmHandle* h, AdjointState* a, int slots) {
+    const size_t np = tape_stride(h), nn = (size_t)h->nn;
+    if (a->tape_slots >= slots && (h->reinit || a->tvol) && (!newtonian(h) || a->tvsc)) return MPM_OK;
+    free_tape(h, a);
+    auto alloc = [&]() -> int {
         for (float*& p : a->tp) TRY(dalloc(h, &p, np * slots));
         if (!h->reinit) TRY(dalloc(h, &a->tvol, np * slots));
-        if (newtonian) TRY(dalloc(h, &a->tvsc, np * slots));
+        if (newtonian(h)) TRY(dalloc(h, &a->tvsc, np * slots));
         for (float*& p : a->tn) TRY(dalloc(h, &p, nn * slots));
-        TRY(dalloc(h, &a->tflag, (size_t)h->ncell * slots));
-        a->tape_slots = slots;
+        return dalloc(h, &a->tflag, (size_t)h->ncell * slots);
+    };
+    const int r = alloc();
+    if (r != MPM_OK) {
+        cudaGetLastError();
+        free_tape(h, a);
+        return r;
     }
+    a->tape_slots = slots;
+    return MPM_OK;
+}
+
+int ensure_adjoint_buffers(MpmHandle* h, AdjointState* a) {
+    const size_t np = tape_stride(h), nn = (size_t)h->nn;
     if (!a->lam[0]) {
         drop_adj_graphs(a);
         for (float*& p : a->lam) TRY(dalloc(h, &p, np));
@@ -238,6 +286,29 @@ int ensure_adjoint_buffers(MpmHandle* h, AdjointState* a, int slots, cudaStream_
         CK(h, cudaMallocHost(&a->h_mismatch, sizeof(int)));
     }
     return MPM_OK;
+}
+
+// Bytes of a taped step, with a sort epoch of its own.
+size_t tape_step_bytes(const MpmHandle* h) {
+    const size_t np = tape_stride(h);
+    return np * (4 * (NTP + 2) + 9 + (h->has_trac ? 10 : 0) + (h->has_pvc ? 2 : 0) + (h->reinit ? 0 : 8)) +
+           (size_t)h->nn * 4 * NTN + (size_t)h->ncell * 5;
+}
+
+// Whether a run of nsteps steps of these bytes each is taped whole, however
+// short the segments asked for: it takes at most a tenth of the device's
+// memory and a quarter of what is free (`have`: tape bytes already held).
+// `limit`: the caller's bound in bytes, negative for none.
+bool tape_whole(size_t step_bytes, int nsteps, size_t have, int64_t limit) {
+    const size_t need = step_bytes * (size_t)nsteps;
+    if (limit >= 0 && need > (size_t)limit) return false;
+    if (need <= have) return true;
+    size_t free_b = 0, total = 0;
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return need <= total / 10 && need - have <= free_b / 4;
 }
 
 void add_seg(std::vector<CopySeg>& v, const void* src, void* dst, size_t bytes, size_t step) {
@@ -346,6 +417,7 @@ int prepare_adj_graphs(MpmHandle* h, AdjointState* a, cudaStream_t s) {
         return MPM_OK;
     }
     if (a->graphs.size() == KEEP) {
+        TRY(sync(h, s));       // none of its graphs is running
         free_adj_graphs(a->graphs.back());
         a->graphs.pop_back();
     }
@@ -361,13 +433,22 @@ int prepare_adj_graphs(MpmHandle* h, AdjointState* a, cudaStream_t s) {
     return upload_segments(h, g.tn, vn, s);
 }
 
-// Capture the launches that `body` issues on the handle's capture stream
-// into an executable graph stored at map[key] (if absent), then launch it.
+// Launch what `body` issues: directly the first time, as a graph captured on
+// the handle's capture stream and kept at map[key] after that (at most
+// GRAPHS_KEPT of them).
+constexpr size_t GRAPHS_KEPT = 64;
 template <class F>
-int run_cached_graph(MpmHandle* h, std::map<int64_t, cudaGraphExec_t>& map, int64_t key, cudaStream_t s,
-                     F&& body) {
+int run_cached_graph(MpmHandle* h, GraphMap& map, const GraphKey& key, cudaStream_t s, F&& body) {
     auto it = map.find(key);
     if (it == map.end()) {
+        if (map.size() >= GRAPHS_KEPT) {
+            TRY(sync(h, s));   // none of them is running
+            free_graphs(map);
+        }
+        map.emplace(key, nullptr);
+        return body(s);
+    }
+    if (!it->second) {
         cudaGraph_t g = nullptr;
         CK(h, cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
         const int r = body(h->cap);
@@ -381,31 +462,137 @@ int run_cached_graph(MpmHandle* h, std::map<int64_t, cudaGraphExec_t>& map, int6
         const cudaError_t ei = cudaGraphInstantiate(&ex, g, 0);
         cudaGraphDestroy(g);
         CK(h, ei);
-        it = map.emplace(key, ex).first;
+        it->second = ex;
     }
     CK(h, cudaGraphLaunch(it->second, s));
     return MPM_OK;
 }
 
-// Re-run of a segment of `len` steps without a re-sort as one graph: per
-// step the tape copy of the start state, the step's kernels (at step offset
-// t) and the tape copy of the nodal results; the step counter advances once.
-int rerun_graph(MpmHandle* h, AdjointState* a, int len, cudaStream_t s) {
-    TRY(classify_tiles(h, s));   // the restored checkpoint's sort
+// The handle's descriptor for step k of a taped run of len steps from slot
+// `slot` (ping-pong parity par at the run's start).
+SimDev slot_desc(MpmHandle* h, AdjointState* a, int slot, int k, int len, int par) {
+    SimDev S = h->hs;
+    const size_t sp = tape_stride(h), nn = (size_t)h->nn, nc = (size_t)h->ncell, i = (size_t)(slot + k);
+    const int p = (par + k) & 1;
+    const bool last = k == len - 1;
+    float** in[4] = {&S.x, &S.y, &S.vx, &S.vy};
+    float** to[4] = {&S.xo, &S.yo, &S.vxo, &S.vyo};
+    for (int f = 0; f < 4; ++f) {
+        *in[f] = a->tp[f] + i * sp;
+        if (!last) *to[f] = a->tp[f] + (i + 1) * sp;
+    }
+    float** pair[TAPE_P - 4] = {S.sxx, S.syy, S.szz, S.sxy, S.rho, S.vol, S.vsc};
+    float* tape[TAPE_P - 4] = {a->tp[4], a->tp[5], a->tp[6], a->tp[7], a->tp[8], h->reinit ? nullptr : a->tvol,
+                               a->tvsc};
+    for (int f = 0; f < TAPE_P - 4; ++f) {
+        if (!tape[f]) continue;
+        pair[f][p] = tape[f] + i * sp;
+        if (!last) pair[f][p ^ 1] = tape[f] + (i + 1) * sp;
+    }
+    float** node[NTN] = {&S.nm, &S.nvax, &S.nvay, &S.nvbx, &S.nvby, &S.nax, &S.nay};
+    if (!last)
+        for (int f = 0; f < NTN; ++f) *node[f] = a->tn[f] + i * nn;
+    if (k > 0) {
+        S.nvpx = a->tn[3] + (i - 1) * nn;
+        S.nvpy = a->tn[4] + (i - 1) * nn;
+    }
+    S.cflag = a->tflag + i * nc;
+    if (!last) S.cflago = a->tflag + (i + 1) * nc;
+    return S;
+}
+
+// The taped segment starts: its first epoch and its tile set are the current
+// sort's.
+int tape_begin(MpmHandle* h, AdjointState* a, int len, cudaStream_t s, bool capture = true) {
+    if (!a->tile_union) {
+        TRY(dalloc(h, &a->tile_union, (size_t)h->ntiles));
+        TRY(dalloc(h, &a->rtiles, (size_t)h->ntiles));
+        TRY(dalloc(h, &a->rempty, (size_t)h->ntiles));
+    }
+    CK(h, cudaMemsetAsync(a->tile_union, 0, sizeof(int) * (size_t)h->ntiles, s));
+    a->nrtiles = -1;
+    a->all_tiles = false;
+    a->tape_seg = -1;
+    a->seg_first = h->step;
+    a->epoch_of.assign(len, 0);
+    a->nep = 0;
+    return capture ? capture_epoch(h, a, s) : MPM_OK;
+}
+
+// Advance len steps within one sort, tape slots slot .. slot + len - 1.
+int run_taped(MpmHandle* h, AdjointState* a, int slot, int len, cudaStream_t s) {
+    TRY(classify_tiles(h, s));
+    if (h->step_tiles == h->d_active) CK(h, launch_or_flags(a->tile_union, h->d_tile_flags, h->ntiles, s));
+    else a->all_tiles = true;
     TRY(prepare_adj_graphs(h, a, s));
     AdjGraphs& g = a->graphs[0];
-    const int par0 = parity(h);
-    TRY(run_cached_graph(h, g.rerun, 2 * len + par0, s, [&](cudaStream_t c) -> int {
-        for (int t = 0; t < len; ++t) {
-            const SegBuf& tp = g.tp[(par0 + t) & 1];
-            CK(h, launch_copy_segments(tp.blk, tp.nblocks, t, c));
-            for (int p = 0; p < 3; ++p) TRY(launch_phase(h, p, t, c));
-            CK(h, launch_copy_segments(g.tn.blk, g.tn.nblocks, t, c));
+    const int par = parity(h);
+    auto body = [&](cudaStream_t c) -> int {
+        CK(h, launch_copy_segments(g.tp[par].blk, g.tp[par].nblocks, slot, c));
+        for (int k = 0; k < len; ++k) {
+            const SimDev S = slot_desc(h, a, slot, k, len, par);
+            for (int p = 0; p < 3; ++p) TRY(launch_phase(h, S, p, k, c));
         }
         CK(h, launch_advance_step(h->ctl, len, c));
+        CK(h, launch_copy_segments(g.tn.blk, g.tn.nblocks, slot + len - 1, c));
         return MPM_OK;
-    }));
+    };
+    if (len < GRAPH_STEPS) TRY(body(s));
+    else TRY(run_cached_graph(h, g.fwd, GraphKey{slot, len, par, 0}, s, body));
+    for (int k = 0; k < len; ++k) a->epoch_of[slot + k] = a->nep - 1;
     h->step += len;
+    return MPM_OK;
+}
+
+// replay_block with the tape: the block's B steps from slot `slot`.
+int replay_taped(MpmHandle* h, AdjointState* a, int64_t step0, int slot, int B, int& st, cudaStream_t s) {
+    h->rollbacks++;
+    TRY(restore_snapshot(h, step0, s));
+    st = 0;
+    for (int i = 0; i < B; ++i) {
+        if (st & ST_DRIFTED) {
+            TRY(resort(h, s));
+            TRY(capture_epoch(h, a, s));
+        }
+        TRY(run_taped(h, a, slot + i, 1, s));
+        TRY(read_ctl(h, s));
+        TRY(check_status(h, st));
+        if (st & ST_DRIFT_VIOLATION)
+            return fail(h, MPM_ERR_CFL, "a particle crossed more than one cell in one step (step %lld)",
+                        (long long)h->step - 1);
+        TRY(clear_status(h, s));
+    }
+    return MPM_OK;
+}
+
+// Steps of the block at step `done` of a recorded run: blocks end at multiples
+// of the checkpoint interval however the run is kept, so that its re-sorts,
+// and with them the last bits of its sums, do not depend on that.
+int block_length(const AdjointState* a, int done, int n, int block_steps) {
+    return std::min({n - done, block_steps, a->interval - done % a->interval});
+}
+
+// mpm_step of the n steps of the segment being taped, the same blocks.
+int taped_steps(MpmHandle* h, AdjointState* a, int n, cudaStream_t s) {
+    h->gen++;
+    TRY(tape_begin(h, a, n, s));
+    for (int slot = 0; slot < n;) {
+        const int B = block_length(a, slot, n, h->block_steps);
+        if (h->needs_resort) {
+            TRY(resort(h, s));
+            TRY(capture_epoch(h, a, s));
+        }
+        const int64_t step0 = h->step;
+        TRY(take_snapshot(h, s));
+        TRY(run_taped(h, a, slot, B, s));
+        TRY(read_ctl(h, s));
+        int st = h->h_ctl->status;
+        if (st & ST_DRIFT_VIOLATION) TRY(replay_taped(h, a, step0, slot, B, st, s));
+        else TRY(check_status(h, st));
+        h->needs_resort = (st & ST_DRIFTED) != 0;
+        TRY(clear_status(h, s));
+        slot += B;
+    }
     return MPM_OK;
 }
 
@@ -414,58 +601,25 @@ int rerun_graph(MpmHandle* h, AdjointState* a, int len, cudaStream_t s) {
 int recompute_segment(MpmHandle* h, AdjointState* a, int seg, int len, cudaStream_t s) {
     TRY(restore_checkpoint(h, a->ck[seg], s));
     const int64_t first = a->ck[seg].step;
-    a->seg_first = first;
-    a->epoch_of.assign(len, 0);
-    a->nep = 0;
-    TRY(capture_epoch(h, a, s));
-    bool resorts = false;
-    for (int t = 0; t < len; ++t) resorts = resorts || resorts_at(a, first + t);
-    SegBuf& tp = h->segbuf;
-    int tp_par = -1;
-    SegBuf tn;
-    std::vector<CopySeg> vn;
-    tape_node_segments(h, a, vn);
-    if (resorts) TRY(upload_segments(h, tn, vn, s));
-    int r = resorts ? MPM_OK : rerun_graph(h, a, len, s);
-    for (int t = 0; t < len && r == MPM_OK && resorts; ++t) {
+    TRY(tape_begin(h, a, len, s));
+    for (int t = 0; t < len;) {
         if (resorts_at(a, first + t)) {
-            r = resort(h, s);
-            if (r == MPM_OK) r = capture_epoch(h, a, s);
-            tp_par = -1;
-            if (r != MPM_OK) break;
+            TRY(resort(h, s));
+            TRY(capture_epoch(h, a, s));
         }
-        const int par = parity(h);
-        if (par != tp_par) {
-            std::vector<CopySeg> v;
-            tape_particle_segments(h, a, par, v);
-            r = upload_segments(h, tp, v, s);
-            if (r != MPM_OK) break;
-            tp_par = par;
-        }
-        if (t == 0 || resorts_at(a, first + t)) {   // the sort of the step (restored or re-sorted)
-            r = classify_tiles(h, s);
-            if (r != MPM_OK) break;
-        }
-        cudaError_t e = launch_copy_segments(tp.blk, tp.nblocks, t, s);
-        if (e == cudaSuccess) {
-            r = launch_steps(h, 1, s);
-            h->step++;
-        }
-        if (e == cudaSuccess && r == MPM_OK)
-            e = launch_copy_segments(tn.blk, tn.nblocks, t, s);
-        if (e != cudaSuccess) r = fail(h, MPM_ERR_CUDA, "tape copy: %s", cudaGetErrorString(e));
-        a->epoch_of[t] = a->nep - 1;
+        int t1 = t + 1;
+        while (t1 < len && !resorts_at(a, first + t1)) ++t1;
+        TRY(run_taped(h, a, t, t1 - t, s));
+        t = t1;
     }
-    if (r == MPM_OK) r = read_ctl(h, s);
-    segbuf_free(tn);
-    TRY(r);
+    TRY(read_ctl(h, s));
     int st = 0;
     TRY(check_status(h, st));
     // the re-run must end bit for bit in the recorded state of the next checkpoint
     std::vector<CopySeg> vc;
     check_segments(h, a, seg, vc);
     SegBuf cb;
-    r = upload_segments(h, cb, vc, s);
+    int r = upload_segments(h, cb, vc, s);
     if (r == MPM_OK) {
         cudaError_t e = cudaMemsetAsync(a->mismatch, 0, sizeof(int), s);
         if (e == cudaSuccess) e = launch_compare_segments(cb.blk, cb.nblocks, a->mismatch, s);
@@ -480,6 +634,7 @@ int recompute_segment(MpmHandle* h, AdjointState* a, int seg, int len, cudaStrea
         return fail(h, MPM_ERR_STATE,
                     "re-run of steps %lld..%lld did not reproduce the recorded run (%d words differ)",
                     (long long)first, (long long)(first + len - 1), *a->h_mismatch);
+    a->tape_seg = seg;
     return clear_status(h, s);
 }
 
@@ -556,21 +711,27 @@ AdjStep base_args(MpmHandle* h, AdjointState* a, int epoch) {
     return A;
 }
 
-// The tiles the reverse node passes visit: the forward step kernels' tiles of
-// the segment's sort when the segment is one sort epoch (the classification
-// of its re-run holds for every step; an empty tile's node adjoints and cell
-// counts are read by no particle), else every tile.
-void reverse_tiles(MpmHandle* h, AdjointState* a, const int4*& tiles, int& ntiles) {
-    if (a->nep == 1) {
-        tiles = h->step_tiles;
-        ntiles = h->nact;
-    } else {
+// The tiles the reverse node passes visit: those with particles in some sort
+// of the taped segment (an empty tile's node adjoints and cell counts are
+// read by no particle), or every tile.
+int reverse_tiles(MpmHandle* h, AdjointState* a, const int4*& tiles, int& ntiles, cudaStream_t s) {
+    if (a->all_tiles) {
         tiles = h->dtiles;
         ntiles = h->ntiles;
+        return MPM_OK;
     }
+    if (a->nrtiles < 0) {
+        CK(h, launch_compact_tiles(a->tile_union, h->dtiles, h->ntiles, a->rtiles, a->rempty, h->d_tile_counts, s));
+        CK(h, cudaMemcpyAsync(h->h_tile_counts, h->d_tile_counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        TRY(sync(h, s));
+        a->nrtiles = tile_grid(h->h_tile_counts[0], h->ntiles);
+    }
+    tiles = a->rtiles;
+    ntiles = a->nrtiles;
+    return MPM_OK;
 }
 
-int reverse_step(MpmHandle* h, AdjointState* a, int t, cudaStream_t s) {
+int reverse_step(MpmHandle* h, AdjointState* a, int t, const int4* tiles, int ntiles, cudaStream_t s) {
     AdjStep A = base_args(h, a, a->epoch_of[t]);
     const size_t op = (size_t)t * A.sp, on = (size_t)t * A.sn, oc = (size_t)t * A.sc;
     A.x += op; A.y += op; A.vx += op; A.vy += op;
@@ -580,21 +741,24 @@ int reverse_step(MpmHandle* h, AdjointState* a, int t, cudaStream_t s) {
     A.cflag += oc;
     A.nm += on; A.nvax += on; A.nvay += on; A.nvbx += on; A.nvby += on; A.nax += on; A.nay += on;
     A.step += t;
-    const int4* tiles;
-    int ntiles;
-    reverse_tiles(h, a, tiles, ntiles);
     CK(h, launch_rev_step(A, h->usl, h->has_trac, tiles, ntiles, s));
     return MPM_OK;
 }
 
-// The reverse steps of a segment of `len` steps in one sort epoch as one
-// graph (for the step configuration of its re-run).
-int reverse_graph(MpmHandle* h, AdjointState* a, int len, cudaStream_t s) {
-    TRY(prepare_adj_graphs(h, a, s));
-    return run_cached_graph(h, a->graphs[0].rev, len, s, [&](cudaStream_t c) -> int {
-        for (int t = len - 1; t >= 0; --t) TRY(reverse_step(h, a, t, c));
+// The reverse steps t1 .. t0, of one sort epoch (tractions need the step
+// number, which a graph would hold by value).
+int reverse_run(MpmHandle* h, AdjointState* a, int t0, int t1, cudaStream_t s) {
+    const int4* tiles;
+    int ntiles;
+    TRY(reverse_tiles(h, a, tiles, ntiles, s));
+    auto body = [&](cudaStream_t c) -> int {
+        for (int t = t1; t >= t0; --t) TRY(reverse_step(h, a, t, tiles, ntiles, c));
         return MPM_OK;
-    });
+    };
+    if (h->has_trac || t1 - t0 + 1 < GRAPH_STEPS) return body(s);
+    TRY(prepare_adj_graphs(h, a, s));
+    const int64_t grid = (int64_t)ntiles * 2 + (tiles == a->rtiles);
+    return run_cached_graph(h, a->graphs[0].rev, GraphKey{t0, t1, a->epoch_of[t0], grid}, s, body);
 }
 
 // Zero the adjoint arrays; particle (n, 2) seeds in original order -> lam[0..3]
@@ -642,6 +806,12 @@ int check_supported(MpmHandle* h) {
     return MPM_OK;
 }
 
+// Record the run in segments of K steps.
+void record_segments(AdjointState* a, int K) {
+    a->K = K;
+    a->nseg = (int)((a->nsteps + K - 1) / K);
+}
+
 // Start a recording on h: checks, state and bookkeeping.
 int record_begin(MpmHandle* h, int nsteps, int K) {
     if (!h->initialized) return fail(h, MPM_ERR_STATE, "initialize first");
@@ -652,11 +822,12 @@ int record_begin(MpmHandle* h, int nsteps, int K) {
     AdjointState* a = h->adj;
     fit(h, a);
     a->valid = false;
+    a->tape_seg = -1;
     a->resort_steps.clear();
     a->step0 = h->step;
-    a->K = K;
     a->nsteps = nsteps;
-    a->nseg = (nsteps + K - 1) / K;
+    a->interval = K;
+    record_segments(a, K);
     a->recording = true;
     return MPM_OK;
 }
@@ -692,26 +863,14 @@ void adjoint_free(MpmHandle* h) {
     h->adj = nullptr;
 }
 
-void drop_batch_adj_graphs(BatchAdjoint* x) {
-    for (auto& kv : x->g_rerun) cudaGraphExecDestroy(kv.second);
-    for (auto& kv : x->g_rev) cudaGraphExecDestroy(kv.second);
-    x->g_rerun.clear();
-    x->g_rev.clear();
-}
-
-// The buffers and kernel builds the batched adjoint's graphs hold; the
-// cached graphs are dropped when any of them changed.
+// The buffers the batched reverse graphs hold; the cached graphs are dropped
+// when any of them changed.
 void check_batch_adj_graphs(MpmBatch* b, BatchAdjoint* x) {
-    const std::vector<uintptr_t> sig = {
-        (uintptr_t)x->tape_p[0].segs, (uintptr_t)x->tape_p[0].blk, x->tape_p[0].nblocks,
-        (uintptr_t)x->tape_p[1].segs, (uintptr_t)x->tape_p[1].blk, x->tape_p[1].nblocks,
-        (uintptr_t)x->tape_n.segs, (uintptr_t)x->tape_n.blk, x->tape_n.nblocks,
-        (uintptr_t)x->d_bases, (uintptr_t)x->d_table, (uintptr_t)x->part_blocks,
-        (uintptr_t)x->n_part_blocks, (uintptr_t)b->d_tdescs, (uintptr_t)b->d_edescs,
-        (uintptr_t)b->d_act_list, (uintptr_t)b->d_tiles, (uintptr_t)b->d_ctls,
-        (uintptr_t)b->cfg.nk_ctas, (uintptr_t)b->cfg.g2p_ctas, (uintptr_t)b->cfg.forces_lpc};
+    const std::vector<uintptr_t> sig = {(uintptr_t)x->d_bases, (uintptr_t)x->d_table, (uintptr_t)x->part_blocks,
+                                        (uintptr_t)x->n_part_blocks, (uintptr_t)x->rtiles,
+                                        (uintptr_t)b->sims.size()};
     if (sig != x->gsig) {
-        drop_batch_adj_graphs(x);
+        free_graphs(x->g_rev);
         x->gsig = sig;
     }
 }
@@ -719,15 +878,16 @@ void check_batch_adj_graphs(MpmBatch* b, BatchAdjoint* x) {
 void batch_adjoint_free(MpmBatch* b) {
     BatchAdjoint* x = b->badj;
     if (!x) return;
-    drop_batch_adj_graphs(x);
+    free_graphs(x->g_rev);
+    cudaFree(x->d_tapes);
+    cudaFree(x->tile_union);
+    cudaFree(x->rtiles);
+    cudaFree(x->rempty);
     cudaFree(x->d_bases);
     cudaFree(x->d_table);
     cudaFree(x->part_blocks);
     cudaFree(x->mismatch);
     if (x->h_mismatch) cudaFreeHost(x->h_mismatch);
-    segbuf_free(x->tape_p[0]);
-    segbuf_free(x->tape_p[1]);
-    segbuf_free(x->tape_n);
     segbuf_free(x->misc);
     delete x;
     b->badj = nullptr;
@@ -739,6 +899,132 @@ using namespace mpm::batch;
 
 namespace {
 
+int ensure_batch_tape(MpmBatch* b) {
+    if (!b->badj) b->badj = new BatchAdjoint();
+    BatchAdjoint* x = b->badj;
+    const size_t nt = (size_t)b->ntiles;
+    if (!x->tile_union) BCK(b, cudaMalloc(&x->tile_union, sizeof(int) * nt));
+    if (!x->rtiles) BCK(b, cudaMalloc(&x->rtiles, sizeof(int4) * nt));
+    if (!x->rempty) BCK(b, cudaMalloc(&x->rempty, sizeof(int4) * nt));
+    if (!x->d_tapes) BCK(b, cudaMalloc(&x->d_tapes, sizeof(TapeDev) * b->sims.size()));
+    return MPM_OK;
+}
+
+// Capture the current sort of the listed members as their next epoch.
+int capture_epochs(MpmBatch* b, BatchAdjoint* x, const std::vector<int>& members, cudaStream_t s) {
+    std::vector<CopySeg> v;
+    for (int i : members) {
+        AdjointState* a = b->sims[i]->adj;
+        BTRY(b, i, epoch_segments(b->sims[i], a, (size_t)a->nep, v));
+        a->nep++;
+    }
+    BTRY(b, 0, run_segments(b->sims[0], x->misc, v, s));
+    return MPM_OK;
+}
+
+// tape_begin for every member.
+int batch_tape_begin(MpmBatch* b, BatchAdjoint* x, int len, cudaStream_t s) {
+    std::vector<int> every;
+    BCK(b, cudaMemsetAsync(x->tile_union, 0, sizeof(int) * (size_t)b->ntiles, s));
+    x->nrtiles = -1;
+    for (int i = 0; i < (int)b->sims.size(); ++i) {
+        BTRY(b, i, tape_begin(b->sims[i], b->sims[i]->adj, len, s, false));
+        every.push_back(i);
+    }
+    return capture_epochs(b, x, every, s);
+}
+
+// run_taped for every member (slots slot .. slot + len - 1 of each).
+int batch_run_taped(MpmBatch* b, BatchAdjoint* x, int slot, int len, cudaStream_t s) {
+    const int n = (int)b->sims.size();
+    std::vector<TapeDev> tapes(n);
+    std::vector<CopySeg> v;
+    for (int i = 0; i < n; ++i) {
+        MpmHandle* h = b->sims[i];
+        AdjointState* a = h->adj;
+        TapeDev& T = tapes[i];
+        for (int k = 0; k < NTP; ++k) T.p[k] = a->tp[k];
+        T.p[NTP] = h->reinit ? nullptr : a->tvol;
+        T.p[NTP + 1] = a->tvsc;
+        for (int k = 0; k < NTN; ++k) T.n[k] = a->tn[k];
+        T.cflag = a->tflag;
+        T.sp = (long long)tape_stride(h);
+        T.sn = h->nn;
+        T.sc = h->ncell;
+        T.step0 = (int)a->seg_first;
+        T.first = (int)h->step;
+        T.last = (int)h->step + len - 1;
+        T.pad = 0;
+        tape_particle_segments(h, a, parity(h), v);
+    }
+    BCK(b, cudaMemcpyAsync(x->d_tapes, tapes.data(), sizeof(TapeDev) * n, cudaMemcpyHostToDevice, s));
+    BTRY(b, 0, upload_segments(b->sims[0], x->misc, v, s));
+    BCK(b, launch_copy_segments(x->misc.blk, x->misc.nblocks, slot, s));
+    int r = prepare_tiles(b, s, x->d_tapes);
+    if (r != MPM_OK) return r;
+    BCK(b, launch_or_flags(x->tile_union, b->d_tflags, b->ntiles, s));
+    r = run_batch_steps(b, len, s);
+    if (r != MPM_OK) return r;
+    v.clear();
+    for (MpmHandle* h : b->sims) tape_node_segments(h, h->adj, v);
+    BTRY(b, 0, upload_segments(b->sims[0], x->misc, v, s));
+    BCK(b, launch_copy_segments(x->misc.blk, x->misc.nblocks, slot + len - 1, s));
+    for (MpmHandle* h : b->sims) {
+        for (int k = 0; k < len; ++k) h->adj->epoch_of[slot + k] = h->adj->nep - 1;
+        h->step += len;
+    }
+    return MPM_OK;
+}
+
+// batch_steps of the n steps of the segment being taped, the same blocks.
+int batch_taped_steps(MpmBatch* b, BatchAdjoint* x, int n, cudaStream_t s) {
+    int r = batch_tape_begin(b, x, n, s);
+    for (int slot = 0; slot < n && r == MPM_OK;) {
+        const int B = block_length(b->sims[0]->adj, slot, n, b->block_steps);
+        std::vector<int> resorted;
+        r = block_resorts(b, resorted, s);
+        if (r == MPM_OK && !resorted.empty()) r = capture_epochs(b, x, resorted, s);
+        if (r == MPM_OK) r = snapshot_all(b, s);
+        if (r != MPM_OK) break;
+        std::vector<int64_t> step0;
+        for (MpmHandle* h : b->sims) step0.push_back(h->step);
+        r = batch_run_taped(b, x, slot, B, s);
+        if (r == MPM_OK) r = read_statuses(b, s);
+        for (int i = 0; i < (int)b->sims.size() && r == MPM_OK; ++i) {
+            MpmHandle* h = b->sims[i];
+            h->gen++;
+            int st = b->h_status[i].status;
+            if (st & ST_DRIFT_VIOLATION) {
+                BTRY(b, i, replay_taped(h, h->adj, step0[i], slot, B, st, s));
+                x->nrtiles = -2;   // the replay's sorts are not in the batch's tile set
+            } else if (st & ST_OUT_OF_MESH) {
+                return bfail(b, MPM_ERR_OUT_OF_MESH, "simulation %d: a particle left the mesh", i);
+            }
+            h->needs_resort = (st & ST_DRIFTED) != 0;
+        }
+        slot += B;
+    }
+    return r;
+}
+
+// The tiles of the batched reverse node passes (reverse_tiles).
+int batch_reverse_tiles(MpmBatch* b, BatchAdjoint* x, const int4*& tiles, int& ntiles, cudaStream_t s) {
+    if (x->nrtiles == -2) {
+        tiles = b->d_tiles;
+        ntiles = b->ntiles;
+        return MPM_OK;
+    }
+    if (x->nrtiles < 0) {
+        BCK(b, launch_compact_tiles(x->tile_union, b->d_tiles, b->ntiles, x->rtiles, x->rempty, b->d_tcounts, s));
+        BCK(b, cudaMemcpyAsync(b->h_tcounts, b->d_tcounts, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        BCK(b, cudaStreamSynchronize(s));
+        x->nrtiles = tile_grid(b->h_tcounts[0], b->ntiles);
+    }
+    tiles = x->rtiles;
+    ntiles = x->nrtiles;
+    return MPM_OK;
+}
+
 // Batched re-run of segment `seg` of every simulation (tape slots 0..len-1),
 // with the bitwise check against the next checkpoints.
 int batch_recompute(MpmBatch* b, BatchAdjoint* x, int seg, int len, cudaStream_t s) {
@@ -747,89 +1033,29 @@ int batch_recompute(MpmBatch* b, BatchAdjoint* x, int seg, int len, cudaStream_t
     for (int i = 0; i < n; ++i) checkpoint_segments(b->sims[i], b->sims[i]->adj->ck[seg], false, v);
     BTRY(b, 0, run_segments(b->sims[0], x->misc, v, s));
     int r = read_statuses(b, s);   // (clears the restored status words)
+    if (r == MPM_OK) r = batch_tape_begin(b, x, len, s);
     if (r != MPM_OK) return r;
-    v.clear();
-    for (int i = 0; i < n; ++i) {
-        AdjointState* a = b->sims[i]->adj;
-        a->epoch_of.assign(len, 0);
-        a->nep = 0;
-        BTRY(b, i, epoch_segments(b->sims[i], a, 0, v));
-        a->nep = 1;
-    }
-    BTRY(b, 0, run_segments(b->sims[0], x->misc, v, s));
-    // tape tables: particle copies for even and odd t (each simulation's own
-    // parity), nodal copies
-    auto build_particle_tables = [&]() -> int {
-        for (int q = 0; q < 2; ++q) {
-            std::vector<CopySeg> w;
-            for (MpmHandle* h : b->sims)
-                tape_particle_segments(h, h->adj, (int)((h->step + q) & 1), w);
-            BTRY(b, 0, upload_segments(b->sims[0], x->tape_p[q], w, s));
-        }
-        return MPM_OK;
-    };
-    // (the parity of slot t is that of the segment's first step plus t)
     std::vector<int64_t> first(n);
-    for (int i = 0; i < n; ++i) {
-        first[i] = b->sims[i]->step;
-        b->sims[i]->adj->seg_first = first[i];
-    }
-    r = build_particle_tables();
-    if (r != MPM_OK) return r;
-    v.clear();
-    for (MpmHandle* h : b->sims) tape_node_segments(h, h->adj, v);
-    BTRY(b, 0, upload_segments(b->sims[0], x->tape_n, v, s));
-    bool resorts = false;
-    for (int i = 0; i < n && !resorts; ++i)
-        for (int t = 0; t < len && !resorts; ++t) resorts = resorts_at(b->sims[i]->adj, first[i] + t);
-    if (!resorts) {
-        // one sort epoch for every simulation: the segment's steps with their
-        // tape copies as one graph (the same launches as the loop below)
-        r = prepare_tiles(b, s);
-        if (r != MPM_OK) return r;
-        check_batch_adj_graphs(b, x);
-        const int64_t key = (int64_t)len | ((int64_t)b->nact << 20) | ((int64_t)b->nemp << 42);
-        BTRY(b, 0, run_cached_graph(b->sims[0], x->g_rerun, key, s, [&](cudaStream_t c) -> int {
-            for (int t = 0; t < len; ++t) {
-                const SegBuf& tp = x->tape_p[t & 1];
-                CK(b->sims[0], launch_copy_segments(tp.blk, tp.nblocks, t, c));
-                const int rr = launch_batch_steps(b, 1, c);
-                if (rr != MPM_OK) return fail(b->sims[0], MPM_ERR_CUDA, "%s", b->err.c_str());
-                CK(b->sims[0], launch_copy_segments(x->tape_n.blk, x->tape_n.nblocks, t, c));
-            }
-            return MPM_OK;
-        }));
-        for (MpmHandle* h : b->sims) h->step += len;
-    }
-    for (int t = 0; t < len && resorts; ++t) {
-        bool resorted = false;
-        for (int i = 0; i < n; ++i) {
-            MpmHandle* h = b->sims[i];
-            if (!resorts_at(h->adj, first[i] + t)) continue;
-            BTRY(b, i, resort(h, s));
-            BTRY(b, i, capture_epoch(h, h->adj, s));
-            resorted = true;
-        }
-        if (resorted) {
-            // tables are built for the parity at t = 0: shift the simulations' steps back
-            for (int i = 0; i < n; ++i) b->sims[i]->step -= t;
-            r = build_particle_tables();
-            for (int i = 0; i < n; ++i) b->sims[i]->step += t;
+    for (int i = 0; i < n; ++i) first[i] = b->sims[i]->step;
+    for (int t = 0; t < len;) {
+        std::vector<int> due;
+        for (int i = 0; i < n; ++i)
+            if (resorts_at(b->sims[i]->adj, first[i] + t)) due.push_back(i);
+        if (!due.empty()) {
+            r = resort_many(b, due, s);
+            if (r == MPM_OK) r = capture_epochs(b, x, due, s);
             if (r != MPM_OK) return r;
         }
-        const SegBuf& tp = x->tape_p[t & 1];
-        BCK(b, launch_copy_segments(tp.blk, tp.nblocks, t, s));
-        // the tile records hold the sort: refreshed at the segment start and
-        // after a re-sort only
-        if (t == 0 || resorted) {
-            r = prepare_tiles(b, s);
-            if (r != MPM_OK) return r;
-        }
-        r = launch_batch_steps(b, 1, s);
+        int t1 = t + 1;
+        auto any_due = [&](int u) {
+            for (int i = 0; i < n; ++i)
+                if (resorts_at(b->sims[i]->adj, first[i] + u)) return true;
+            return false;
+        };
+        while (t1 < len && !any_due(t1)) ++t1;
+        r = batch_run_taped(b, x, t, t1 - t, s);
         if (r != MPM_OK) return r;
-        for (MpmHandle* h : b->sims) h->step++;
-        BCK(b, launch_copy_segments(x->tape_n.blk, x->tape_n.nblocks, t, s));
-        for (MpmHandle* h : b->sims) h->adj->epoch_of[t] = h->adj->nep - 1;
+        t = t1;
     }
     r = read_statuses(b, s);
     if (r != MPM_OK) return r;
@@ -852,17 +1078,19 @@ int batch_recompute(MpmBatch* b, BatchAdjoint* x, int seg, int len, cudaStream_t
     if (*x->h_mismatch != 0)
         return bfail(b, MPM_ERR_STATE, "re-run of segment %d did not reproduce the recorded run "
                      "(%d words differ)", seg, *x->h_mismatch);
+    for (MpmHandle* h : b->sims) h->adj->tape_seg = seg;
     return MPM_OK;
 }
 
 // seed() for every member, one launch per seed array.  A host seed is staged in
 // its member's own staging buffer; the second seed's copy follows the first
 // one's transfer on the stream.
-int batch_seed(MpmBatch* b, const float* const* dl_dloc, const float* const* dl_dvel, int on_device,
+int batch_seed(MpmBatch* b, const float* const* dl_dloc, const float* const* dl_dvel, int len, int on_device,
                cudaStream_t s) {
     const int n = (int)b->sims.size();
     std::vector<FieldMap> maps;
-    for (MpmHandle* h : b->sims) maps.push_back(lam_map(h, h->adj, 0, NLAM, h->ps[h->pcur].pid, nullptr));
+    auto order = [&](MpmHandle* h) { return h->adj->epochs[h->adj->epoch_of[len - 1]].pid; };
+    for (MpmHandle* h : b->sims) maps.push_back(lam_map(h, h->adj, 0, NLAM, order(h), nullptr));
     int r = fields_many(b, maps, true, s);
     const float* const* src[2] = {dl_dloc, dl_dvel};
     for (int k = 0; k < 2 && r == MPM_OK; ++k) {
@@ -873,7 +1101,7 @@ int batch_seed(MpmBatch* b, const float* const* dl_dloc, const float* const* dl_
             if (!src[k][i]) continue;
             const void* d = nullptr;
             BTRY(b, i, to_device(h, src[k][i], sizeof(float) * 2 * h->np, on_device, s, &d));
-            maps.push_back(lam_map(h, h->adj, 2 * k, 2, h->ps[h->pcur].pid, static_cast<const float*>(d)));
+            maps.push_back(lam_map(h, h->adj, 2 * k, 2, order(h), static_cast<const float*>(d)));
         }
         r = fields_many(b, maps, true, s);
     }
@@ -940,20 +1168,29 @@ int mpm_record(MpmHandle* h, int nsteps, int checkpoint_steps, void* stream) {
     TRY(record_begin(h, nsteps, checkpoint_steps));
     cudaStream_t s = S(stream);
     AdjointState* a = h->adj;
+    if (tape_whole(tape_step_bytes(h), nsteps, tape_step_bytes(h) * (size_t)a->tape_slots, h->tape_limit))
+        record_segments(a, nsteps);
+    bool taped = ensure_tape(h, a, std::min(a->K, nsteps)) == MPM_OK;
+    if (!taped && a->K > checkpoint_steps) {
+        record_segments(a, checkpoint_steps);
+        taped = ensure_tape(h, a, std::min(a->K, nsteps)) == MPM_OK;
+    }
+    // (without memory for a tape the run keeps checkpoints only)
+    const bool checkpoints = !taped || a->nseg > 1;
     int r = MPM_OK;
-    for (int seg = 0; seg < a->nseg && r == MPM_OK; ++seg) {
-        std::vector<CopySeg> v;
-        r = save_checkpoint(h, a, seg, v);
-        if (r == MPM_OK) r = run_segments(h, h->segbuf, v, s);
-        const int len = std::min(checkpoint_steps, nsteps - seg * checkpoint_steps);
-        if (r == MPM_OK) r = mpm_step(h, len, stream);
+    for (int seg = 0; seg <= a->nseg && r == MPM_OK; ++seg) {
+        if (checkpoints) {
+            std::vector<CopySeg> v;
+            r = save_checkpoint(h, a, seg, v);
+            if (r == MPM_OK) r = run_segments(h, h->segbuf, v, s);
+        }
+        if (r != MPM_OK || seg == a->nseg) break;
+        const int len = std::min(a->K, nsteps - seg * a->K);
+        if (taped && seg == a->nseg - 1) r = taped_steps(h, a, len, s);
+        else r = mpm_step(h, len, stream);
     }
-    if (r == MPM_OK) {
-        std::vector<CopySeg> v;
-        r = save_checkpoint(h, a, a->nseg, v);
-        if (r == MPM_OK) r = run_segments(h, h->segbuf, v, s);
-        if (r == MPM_OK) r = sync(h, s);
-    }
+    if (r == MPM_OK) r = sync(h, s);
+    if (r == MPM_OK && taped) a->tape_seg = a->nseg - 1;
     record_end(h, r == MPM_OK);
     return r;
 }
@@ -967,31 +1204,33 @@ int mpm_adjoint(MpmHandle* h, const float* dl_dloc, const float* dl_dvel, float*
     if (!dl_dloc) return fail(h, MPM_ERR_INVALID, "dl_dloc is null");
     AdjointState* a = h->adj;
     cudaStream_t s = S(stream);
-    const int K = a->K;
-    TRY(ensure_adjoint_buffers(h, a, K, s));
-    // the seeds are in the order of the recorded end state (the current one)
-    TRY(seed(h, a, dl_dloc, dl_dvel, h->ps[h->pcur].pid, on_device, s));
+    TRY(ensure_adjoint_buffers(h, a));
+    TRY(ensure_tape(h, a, (int)std::min<int64_t>(a->K, a->nsteps)));
     int r = MPM_OK;
+    bool moved = false;
     for (int seg = a->nseg - 1; seg >= 0 && r == MPM_OK; --seg) {
-        const int len = (int)std::min<int64_t>(K, a->nsteps - (int64_t)seg * K);
-        r = recompute_segment(h, a, seg, len, s);
-        // one sort epoch: the segment's reverse steps as a graph (tractions
-        // need the step number, which the graph would hold by value)
-        if (r == MPM_OK && a->nep == 1 && !h->has_trac) {
-            r = reverse_graph(h, a, len, s);
-            continue;
+        const int len = (int)std::min<int64_t>(a->K, a->nsteps - (int64_t)seg * a->K);
+        if (a->tape_seg != seg) {
+            moved = true;
+            r = recompute_segment(h, a, seg, len, s);
         }
-        for (int t = len - 1; t >= 0 && r == MPM_OK; --t) {
-            if (t < len - 1 && a->epoch_of[t] != a->epoch_of[t + 1])
-                r = permute(h, a, a->epochs[a->epoch_of[t + 1]].pid, a->epochs[a->epoch_of[t]].pid, s);
-            if (r == MPM_OK) r = reverse_step(h, a, t, s);
+        // the seeds go to the order of the last step, the recorded end state's
+        if (r == MPM_OK && seg == a->nseg - 1)
+            r = seed(h, a, dl_dloc, dl_dvel, a->epochs[a->epoch_of[len - 1]].pid, on_device, s);
+        for (int t1 = len - 1; t1 >= 0 && r == MPM_OK;) {
+            const int e = a->epoch_of[t1];
+            if (t1 < len - 1) r = permute(h, a, a->epochs[a->epoch_of[t1 + 1]].pid, a->epochs[e].pid, s);
+            int t0 = t1;
+            while (t0 > 0 && a->epoch_of[t0 - 1] == e) --t0;
+            if (r == MPM_OK) r = reverse_run(h, a, t0, t1, s);
+            t1 = t0 - 1;
         }
         if (r == MPM_OK && a->epoch_of[0] != 0)
             r = permute(h, a, a->epochs[a->epoch_of[0]].pid, a->epochs[0].pid, s);
     }
     if (r == MPM_OK) r = emit_all(h, a, dl_dE, dl_dloc0, dl_dvel0, on_device, s);
-    // leave the handle at the recorded end state
-    const int r2 = restore_checkpoint(h, a->ck[a->nseg], s);
+    // leave the handle at the recorded end state (where the re-runs moved it)
+    const int r2 = moved ? restore_checkpoint(h, a->ck[a->nseg], s) : sync(h, s);
     TRY(r);
     return r2;
 }
@@ -1003,19 +1242,51 @@ int mpm_batch_record(MpmBatch* b, int nsteps, int checkpoint_steps, void* stream
     const int n = (int)b->sims.size();
     for (int i = 0; i < n; ++i) BTRY(b, i, record_begin(b->sims[i], nsteps, checkpoint_steps));
     cudaStream_t s = S(stream);
-    const int nseg = b->sims[0]->adj->nseg;
-    for (int seg = 0; seg <= nseg && r == MPM_OK; ++seg) {
-        std::vector<CopySeg> v;
-        for (int i = 0; i < n && r == MPM_OK; ++i) {
-            r = save_checkpoint(b->sims[i], b->sims[i]->adj, seg, v);
-            if (r != MPM_OK) r = from_sim(b, i, r);
+    size_t step_bytes = 0, have = 0;
+    for (MpmHandle* h : b->sims) {
+        step_bytes += tape_step_bytes(h);
+        have += tape_step_bytes(h) * (size_t)h->adj->tape_slots;
+    }
+    int64_t limit = -1;   // of the whole batch: the least of its members' bounds
+    for (MpmHandle* h : b->sims)
+        if (h->tape_limit >= 0 && (limit < 0 || h->tape_limit < limit)) limit = h->tape_limit;
+    auto ensure_tapes = [&](int K) {
+        for (MpmHandle* h : b->sims) {
+            record_segments(h->adj, K);
+            if (ensure_tape(h, h->adj, std::min(K, nsteps)) != MPM_OK) return false;
         }
-        if (r == MPM_OK && run_segments(b->sims[0], b->segbuf, v, s) != MPM_OK) r = from_sim(b, 0, MPM_ERR_CUDA);
-        if (r == MPM_OK && seg < nseg)
-            r = batch_steps(b, std::min(checkpoint_steps, nsteps - seg * checkpoint_steps), s);
+        return true;
+    };
+    const bool whole = tape_whole(step_bytes, nsteps, have, limit);
+    bool taped = ensure_batch_tape(b) == MPM_OK && ensure_tapes(whole ? nsteps : checkpoint_steps);
+    if (!taped && whole) {
+        for (MpmHandle* h : b->sims) free_tape(h, h->adj);
+        taped = ensure_batch_tape(b) == MPM_OK && ensure_tapes(checkpoint_steps);
+    }
+    // (without memory for the tapes the run keeps checkpoints only)
+    for (MpmHandle* h : b->sims)
+        if (!taped) record_segments(h->adj, checkpoint_steps);
+    const int K = b->sims[0]->adj->K, nseg = b->sims[0]->adj->nseg;
+    const bool checkpoints = !taped || nseg > 1;
+    for (int seg = 0; seg <= nseg && r == MPM_OK; ++seg) {
+        if (checkpoints) {
+            std::vector<CopySeg> v;
+            for (int i = 0; i < n && r == MPM_OK; ++i) {
+                r = save_checkpoint(b->sims[i], b->sims[i]->adj, seg, v);
+                if (r != MPM_OK) r = from_sim(b, i, r);
+            }
+            if (r == MPM_OK && run_segments(b->sims[0], b->segbuf, v, s) != MPM_OK)
+                r = from_sim(b, 0, MPM_ERR_CUDA);
+        }
+        if (r != MPM_OK || seg == nseg) break;
+        const int len = std::min(K, nsteps - seg * K);
+        r = taped && seg == nseg - 1 ? batch_taped_steps(b, b->badj, len, s) : batch_steps(b, len, s);
     }
     if (r == MPM_OK && cudaStreamSynchronize(s) != cudaSuccess) r = bfail(b, MPM_ERR_CUDA, "synchronise");
-    for (MpmHandle* h : b->sims) record_end(h, r == MPM_OK);
+    for (MpmHandle* h : b->sims) {
+        if (r == MPM_OK && taped) h->adj->tape_seg = nseg - 1;
+        record_end(h, r == MPM_OK);
+    }
     return r;
 }
 
@@ -1038,71 +1309,82 @@ int mpm_batch_adjoint(MpmBatch* b, const float* const* dl_dloc, const float* con
     int r = ensure_batch_adjoint(b, s);
     if (r != MPM_OK) return r;
     BatchAdjoint* x = b->badj;
-    for (int i = 0; i < n; ++i) BTRY(b, i, ensure_adjoint_buffers(b->sims[i], b->sims[i]->adj, K, s));
-    r = batch_seed(b, dl_dloc, dl_dvel, on_device, s);
-    if (r != MPM_OK) {
-        cudaStreamSynchronize(s);   // seeds already in flight
-        return r;
+    r = ensure_batch_tape(b);
+    if (r != MPM_OK) return r;
+    for (int i = 0; i < n; ++i) {
+        MpmHandle* h = b->sims[i];
+        BTRY(b, i, ensure_adjoint_buffers(h, h->adj));
+        BTRY(b, i, ensure_tape(h, h->adj, (int)std::min<int64_t>(K, nsteps)));
     }
-    x->bases.assign(n, AdjStep{});
-    std::vector<int> cur(n, -1);   // epoch whose pointers bases[i] holds
-    bool any_pvc = false, any_newt = false;
+    bool any_pvc = false, any_newt = false, moved = false;
     for (MpmHandle* h : b->sims) {
         any_pvc = any_pvc || h->has_pvc;
         any_newt = any_newt || h->adj->tvsc != nullptr;
     }
+    std::vector<int> cur(n, -1);   // epoch whose order the member's adjoint arrays are in
     for (int seg = nseg - 1; seg >= 0 && r == MPM_OK; --seg) {
         const int len = (int)std::min<int64_t>(K, nsteps - (int64_t)seg * K);
-        r = batch_recompute(b, x, seg, len, s);
-        if (r != MPM_OK) break;
-        for (int i = 0; i < n; ++i) {
-            AdjointState* a = b->sims[i]->adj;
-            x->bases[i] = base_args(b->sims[i], a, a->epoch_of[len - 1]);
-            cur[i] = a->epoch_of[len - 1];
+        bool have = true;
+        for (MpmHandle* h : b->sims) have = have && h->adj->tape_seg == seg;
+        if (!have) {
+            moved = true;
+            r = batch_recompute(b, x, seg, len, s);
+            if (r != MPM_OK) break;
         }
-        BCK(b, cudaMemcpyAsync(x->d_bases, x->bases.data(), sizeof(AdjStep) * n, cudaMemcpyHostToDevice, s));
-        // the reverse node passes visit the active tiles of the re-run's
-        // classification when no simulation re-sorted in the segment (see
-        // reverse_tiles), else every tile
-        bool one_epoch = true;
-        for (MpmHandle* h : b->sims) one_epoch = one_epoch && h->adj->nep == 1;
-        const int4* rtiles = one_epoch ? b->d_act_list : b->d_tiles;
-        const int nrtiles = one_epoch ? b->nact : b->ntiles;
-        if (one_epoch) {
-            // no permutation between steps: the segment's reverse steps as one graph
-            check_batch_adj_graphs(b, x);
-            const int64_t key = (int64_t)len | ((int64_t)nrtiles << 20) | ((int64_t)x->n_part_blocks << 42);
-            r = run_cached_graph(b->sims[0], x->g_rev, key, s, [&](cudaStream_t c) -> int {
-                for (int t = len - 1; t >= 0; --t) {
+        for (int i = 0; i < n; ++i) cur[i] = b->sims[i]->adj->epoch_of[len - 1];
+        if (seg == nseg - 1) {
+            r = batch_seed(b, dl_dloc, dl_dvel, len, on_device, s);
+            if (r != MPM_OK) break;
+        }
+        const int4* rtiles = nullptr;
+        int nrtiles = 0;
+        r = batch_reverse_tiles(b, x, rtiles, nrtiles, s);
+        if (r != MPM_OK) break;
+        x->bases.assign(n, AdjStep{});
+        for (int t1 = len - 1; t1 >= 0 && r == MPM_OK;) {
+            // the steps down to t0 keep every member's sort
+            for (int i = 0; i < n && r == MPM_OK; ++i) {
+                MpmHandle* h = b->sims[i];
+                AdjointState* a = h->adj;
+                const int e = a->epoch_of[t1];
+                if (e != cur[i]) r = permute(h, a, a->epochs[cur[i]].pid, a->epochs[e].pid, s);
+                if (r != MPM_OK) {
+                    r = from_sim(b, i, r);
+                    break;
+                }
+                cur[i] = e;
+                x->bases[i] = base_args(h, a, e);
+            }
+            if (r != MPM_OK) break;
+            BCK(b, cudaMemcpyAsync(x->d_bases, x->bases.data(), sizeof(AdjStep) * n, cudaMemcpyHostToDevice, s));
+            int t0 = t1;
+            auto same = [&](int t) {
+                for (int i = 0; i < n; ++i)
+                    if (b->sims[i]->adj->epoch_of[t] != cur[i]) return false;
+                return true;
+            };
+            while (t0 > 0 && same(t0 - 1)) --t0;
+            auto body = [&](cudaStream_t c) -> int {
+                for (int t = t1; t >= t0; --t) {
                     CK(b->sims[0], launch_adj_table(x->d_bases, n, t, x->d_table, c));
                     CK(b->sims[0], launch_rev_batch(x->d_table, b->cfg.usl, b->cfg.traction, any_pvc,
                                                     b->cfg.reinit, any_newt, rtiles, nrtiles, x->part_blocks,
                                                     x->n_part_blocks, c));
                 }
                 return MPM_OK;
-            });
-            if (r != MPM_OK) r = from_sim(b, 0, r);
-        }
-        for (int t = len - 1; t >= 0 && r == MPM_OK && !one_epoch; --t) {
-            for (int i = 0; i < n && r == MPM_OK; ++i) {
-                MpmHandle* h = b->sims[i];
-                AdjointState* a = h->adj;
-                if (a->epoch_of[t] == cur[i]) continue;
-                r = permute(h, a, a->epochs[cur[i]].pid, a->epochs[a->epoch_of[t]].pid, s);
-                if (r != MPM_OK) {
-                    r = from_sim(b, i, r);
-                    break;
-                }
-                cur[i] = a->epoch_of[t];
-                x->bases[i] = base_args(h, a, cur[i]);
-                if (cudaMemcpyAsync(x->d_bases + i, &x->bases[i], sizeof(AdjStep), cudaMemcpyHostToDevice,
-                                    s) != cudaSuccess)
-                    r = bfail(b, MPM_ERR_CUDA, "argument upload");
+            };
+            if (t1 - t0 + 1 < GRAPH_STEPS) {
+                r = body(s);
+            } else {
+                check_batch_adj_graphs(b, x);
+                const int64_t grid = (int64_t)nrtiles * 2 + (rtiles == x->rtiles);
+                const int64_t opts = (int64_t)x->n_part_blocks * 4 + any_pvc * 2 + any_newt;
+                r = run_cached_graph(b->sims[0], x->g_rev, GraphKey{t0, t1, grid, opts}, s, body);
             }
-            if (r != MPM_OK) break;
-            BCK(b, launch_adj_table(x->d_bases, n, t, x->d_table, s));
-            BCK(b, launch_rev_batch(x->d_table, b->cfg.usl, b->cfg.traction, any_pvc, b->cfg.reinit,
-                                    any_newt, rtiles, nrtiles, x->part_blocks, x->n_part_blocks, s));
+            if (r != MPM_OK) r = from_sim(b, 0, r);
+            t1 = t0 - 1;
+            // (the host copy of the arguments must outlive the upload)
+            if (r == MPM_OK && cudaStreamSynchronize(s) != cudaSuccess) r = bfail(b, MPM_ERR_CUDA, "synchronise");
         }
         for (int i = 0; i < n && r == MPM_OK; ++i) {
             MpmHandle* h = b->sims[i];
@@ -1112,25 +1394,22 @@ int mpm_batch_adjoint(MpmBatch* b, const float* const* dl_dloc, const float* con
                 if (e != MPM_OK) r = from_sim(b, i, e);
             }
         }
-        // (the host copy of the arguments must outlive the uploads)
-        if (r == MPM_OK && cudaStreamSynchronize(s) != cudaSuccess) r = bfail(b, MPM_ERR_CUDA, "synchronise");
     }
     if (r == MPM_OK && dl_dE) r = batch_emit(b, dl_dE, 9, 1, on_device, s);
     if (r == MPM_OK && dl_dloc0) r = batch_emit(b, dl_dloc0, 0, 2, on_device, s);
     if (r == MPM_OK && dl_dvel0) r = batch_emit(b, dl_dvel0, 2, 2, on_device, s);
-    // leave every simulation at the recorded end state (read_statuses
-    // synchronises the stream: the gradients' copies are complete on return)
-    std::vector<CopySeg> v;
-    for (MpmHandle* h : b->sims) checkpoint_segments(h, h->adj->ck[nseg], false, v);
-    int r2 = run_segments(b->sims[0], x->misc, v, s);
-    if (r2 == MPM_OK) {
-        r2 = read_statuses(b, s);
-    } else {
-        cudaStreamSynchronize(s);
-        r2 = from_sim(b, 0, r2);
+    // leave every simulation at the recorded end state, where the re-runs moved
+    // it (the wait also completes the gradients' copies)
+    int r2 = MPM_OK;
+    if (moved) {
+        std::vector<CopySeg> v;
+        for (MpmHandle* h : b->sims) checkpoint_segments(h, h->adj->ck[nseg], false, v);
+        r2 = run_segments(b->sims[0], x->misc, v, s);
+        if (r2 == MPM_OK) r2 = read_statuses(b, s);
+        else r2 = from_sim(b, 0, r2);
     }
-    if (r != MPM_OK) return r;
-    return r2;
+    if (cudaStreamSynchronize(s) != cudaSuccess && r2 == MPM_OK) r2 = bfail(b, MPM_ERR_CUDA, "synchronise");
+    return r != MPM_OK ? r : r2;
 }
 
 }  // extern "C"

@@ -57,14 +57,14 @@ void drop_batch_graphs(MpmBatch* b) {
     b->graphs.clear();
 }
 
-int prepare_tiles(MpmBatch* b, cudaStream_t s) {
+int prepare_tiles(MpmBatch* b, cudaStream_t s, const TapeDev* tapes) {
     // the descriptors and row starts change only between step blocks
     // (re-sorts, set-up calls): one record per tile and block lets a CTA fetch
     // its tile, descriptor, control pointer and row starts in one read
     BCK(b, launch_classify_tiles_batch(b->d_sims, b->d_tiles, b->ntiles, b->d_tflags, b->d_act_list,
                                        b->d_emp_list, b->d_tcounts, s));
-    BCK(b, launch_gather_tiles(b->d_sims, b->d_ctls, b->d_act_list, b->ntiles, b->d_tdescs, s));
-    BCK(b, launch_gather_tiles(b->d_sims, b->d_ctls, b->d_emp_list, b->ntiles, b->d_edescs, s));
+    BCK(b, launch_gather_tiles(b->d_sims, b->d_ctls, tapes, b->d_act_list, b->ntiles, b->d_tdescs, s));
+    BCK(b, launch_gather_tiles(b->d_sims, b->d_ctls, nullptr, b->d_emp_list, b->ntiles, b->d_edescs, s));
     BCK(b, cudaMemcpyAsync(b->h_tcounts, b->d_tcounts, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     BCK(b, cudaStreamSynchronize(s));
     b->nact = tile_grid(b->h_tcounts[0], b->ntiles);
@@ -85,10 +85,7 @@ int launch_batch_steps(MpmBatch* b, int n, cudaStream_t s) {
     return MPM_OK;
 }
 
-// n steps: whole graphs of GRAPH_STEPS steps, then the rest as launches.
 int run_batch_steps(MpmBatch* b, int n, cudaStream_t s) {
-    const int r0 = prepare_tiles(b, s);
-    if (r0 != MPM_OK) return r0;
     if (n >= GRAPH_STEPS) {
         const int64_t key = (int64_t)b->nact | ((int64_t)b->nemp << 32);
         auto it = b->graphs.find(key);
@@ -189,11 +186,10 @@ int resort_many(MpmBatch* b, const std::vector<int>& members, cudaStream_t s) {
     return MPM_OK;
 }
 
-// One block of B steps for every simulation (see the file comment).
-int batch_block(MpmBatch* b, int B, cudaStream_t s) {
+int block_resorts(MpmBatch* b, std::vector<int>& resorted, cudaStream_t s) {
     const int n = (int)b->sims.size();
     if ((int)b->since_resort.size() != n) b->since_resort.assign(n, 0);
-    std::vector<int> drifted;
+    resorted.clear();
     for (int i = 0; i < n; ++i) {
         // a drifted simulation keeps its sort for resort_every - 1 more blocks
         // (its drifted cells take the gathering path); a two-cell drift
@@ -201,18 +197,31 @@ int batch_block(MpmBatch* b, int B, cudaStream_t s) {
         if (!b->sims[i]->needs_resort) {
             b->since_resort[i] = 0;
         } else if (++b->since_resort[i] >= b->resort_every) {
-            drifted.push_back(i);
+            resorted.push_back(i);
             b->since_resort[i] = 0;
         }
     }
-    int r = resort_many(b, drifted, s);
-    if (r != MPM_OK) return r;
+    return resort_many(b, resorted, s);
+}
+
+int snapshot_all(MpmBatch* b, cudaStream_t s) {
     std::vector<CopySeg> v;
     for (MpmHandle* h : b->sims) snapshot_segments(h, true, v);
     BTRY(b, 0, run_segments(b->sims[0], b->segbuf, v, s));
+    return MPM_OK;
+}
+
+// One block of B steps for every simulation (see the file comment).
+int batch_block(MpmBatch* b, int B, cudaStream_t s) {
+    const int n = (int)b->sims.size();
+    std::vector<int> resorted;
+    int r = block_resorts(b, resorted, s);
+    if (r == MPM_OK) r = snapshot_all(b, s);
+    if (r != MPM_OK) return r;
     std::vector<int64_t> step0(n);
     for (int i = 0; i < n; ++i) step0[i] = b->sims[i]->step;
-    r = run_batch_steps(b, B, s);
+    r = prepare_tiles(b, s);
+    if (r == MPM_OK) r = run_batch_steps(b, B, s);
     if (r != MPM_OK) return r;
     for (MpmHandle* h : b->sims) {
         h->step += B;

@@ -54,11 +54,16 @@ int check_ready(MpmBatch* b);
 // Split the batch's tiles into active and empty ones and write their records
 // (descriptor, row starts, occupancy) for the current descriptors and sorts;
 // needed whenever a descriptor or a sort changed.  Waits for the counts, so
-// not inside a stream capture.
-int prepare_tiles(MpmBatch* b, cudaStream_t s);
-// n steps of every simulation as 3n batched launches over the active tiles
-// plus those over the empty tiles that are due (no status handling).
-int launch_batch_steps(MpmBatch* b, int n, cudaStream_t s);
+// not inside a stream capture.  With `tapes` (one per simulation, on the
+// device) the steps over these records are taped.
+int prepare_tiles(MpmBatch* b, cudaStream_t s, const TapeDev* tapes = nullptr);
+// n steps over the prepared records: whole graphs of GRAPH_STEPS steps, then
+// the rest as launches.
+int run_batch_steps(MpmBatch* b, int n, cudaStream_t s);
+// What starts a step block: the re-sorts that are due (their members in
+// `resorted`), and a snapshot of every member.
+int block_resorts(MpmBatch* b, std::vector<int>& resorted, cudaStream_t s);
+int snapshot_all(MpmBatch* b, cudaStream_t s);
 // Copy a host argument table into b->d_table (valid until the next upload on
 // the stream).
 int upload_table(MpmBatch* b, const void* src, size_t bytes, cudaStream_t s);

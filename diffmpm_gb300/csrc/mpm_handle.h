@@ -164,6 +164,7 @@ struct MpmHandle {
     int forces_lpc = 0;
     int empty_split_min = mpm::EMPTY_SPLIT_MIN;   // mpm_set_empty_split
     int64_t resorts = 0, rollbacks = 0;
+    int64_t tape_limit = -1;           // mpm_set_tape_limit
     // differentiation (null until mpm_record); gen counts state changes
     mpm::AdjointState* adj = nullptr;
     mpm::LineAdjoint* line_adj = nullptr;   // 1-D recording (mpm_line_adjoint.cu)
@@ -226,8 +227,9 @@ void sort_done(MpmHandle* h);
 FieldMap field_map(MpmHandle* h, int field, const float* aos);
 // n steps from ctl->step (the tiles classified for the current sort).
 int launch_steps(MpmHandle* h, int n, cudaStream_t s);
-// Phase `phase` (0 nodal kinematics, 1 forces, 2 G2P) of step ctl->step + k.
-int launch_phase(MpmHandle* h, int phase, int k, cudaStream_t s);
+// Phase `phase` (0 nodal kinematics, 1 forces, 2 G2P) of step ctl->step + k
+// with descriptor S (the handle's own, or one of a taped step).
+int launch_phase(MpmHandle* h, const SimDev& S, int phase, int k, cudaStream_t s);
 // The step kernels' tile list and grids (step_tiles, nact, nemp) for the
 // current sort; call before a sequence of launch_phase (it waits for the
 // counts, so not inside a stream capture).
@@ -235,6 +237,7 @@ int classify_tiles(MpmHandle* h, cudaStream_t s);
 StepKey step_key(const MpmHandle* h);
 int check_status(MpmHandle* h, int& st);
 int take_snapshot(MpmHandle* h, cudaStream_t s);
+int restore_snapshot(MpmHandle* h, int64_t step0, cudaStream_t s);
 int replay_block(MpmHandle* h, int64_t step0, int B, int& st, cudaStream_t s);
 // Where a recorded 1-D step copies its start state (x, v, sxx, syy, szz, sxy,
 // rho, volume, centroid volumetric strain in storage order, the storage ->

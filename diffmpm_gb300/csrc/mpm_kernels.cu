@@ -34,7 +34,8 @@ __device__ __forceinline__ int load_step(const Control* ctl) { return __ldg(&ctl
 // simulation's descriptor and control pointer, the storage starts of its
 // cell rows and its occupancy (one warp per record).
 __global__ void k_gather_tiles(const SimDev* const* __restrict__ sims, Control* const* __restrict__ ctls,
-                               const int4* __restrict__ tiles, int ntiles, TileDesc* __restrict__ out) {
+                               const TapeDev* __restrict__ tapes, const int4* __restrict__ tiles, int ntiles,
+                               TileDesc* __restrict__ out) {
     const int t = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
     if (t >= ntiles) return;
     const int4 T = tiles[t];
@@ -52,6 +53,9 @@ __global__ void k_gather_tiles(const SimDev* const* __restrict__ sims, Control* 
     const int* a = reinterpret_cast<const int*>(sd);
     int* b = reinterpret_cast<int*>(&d.S);
     for (int i = lane; i < (int)(sizeof(SimDev) / 4); i += 32) b[i] = a[i];
+    const int* c = reinterpret_cast<const int*>(tapes + T.x);
+    int* e = reinterpret_cast<int*>(&d.tape);
+    for (int i = lane; i < (int)(sizeof(TapeDev) / 4); i += 32) e[i] = tapes ? c[i] : 0;
     const int nx = sd->nx, ny = sd->ny;
     const int* __restrict__ cstart = sd->cstart;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
@@ -74,18 +78,48 @@ __global__ void k_gather_tiles(const SimDev* const* __restrict__ sims, Control* 
     }
 }
 
-cudaError_t launch_gather_tiles(const SimDev* const* sims, Control* const* ctls, const int4* tiles,
-                                int ntiles, TileDesc* out, cudaStream_t s) {
-    if (ntiles > 0) k_gather_tiles<<<(ntiles + 7) / 8, 256, 0, s>>>(sims, ctls, tiles, ntiles, out);
+cudaError_t launch_gather_tiles(const SimDev* const* sims, Control* const* ctls, const TapeDev* tapes,
+                                const int4* tiles, int ntiles, TileDesc* out, cudaStream_t s) {
+    if (ntiles > 0) k_gather_tiles<<<(ntiles + 7) / 8, 256, 0, s>>>(sims, ctls, tapes, tiles, ntiles, out);
     return cudaGetLastError();
 }
 
 // A batched CTA copies its tile record (tile, control pointer, descriptor,
-// row starts) into shared memory, 16 bytes per thread.
-__device__ __forceinline__ void load_tile(const TileDesc* __restrict__ src, TileDesc& dst) {
+// row starts) into shared memory, 16 bytes per thread, and points the
+// descriptor of a taped step at its slots.
+static_assert(offsetof(SimDev, vy) == offsetof(SimDev, x) + 3 * sizeof(float*) &&
+              offsetof(SimDev, vyo) == offsetof(SimDev, xo) + 3 * sizeof(float*) &&
+              offsetof(SimDev, sxy) == offsetof(SimDev, sxx) + 6 * sizeof(float*) &&
+              offsetof(SimDev, nay) == offsetof(SimDev, nm) + 6 * sizeof(float*), "members load_tile indexes");
+__device__ __forceinline__ void load_tile(const TileDesc* __restrict__ src, TileDesc& dst, int k) {
     const int4* a = reinterpret_cast<const int4*>(src);
     int4* b = reinterpret_cast<int4*>(&dst);
     for (int i = threadIdx.x; i < (int)(sizeof(TileDesc) / 16); i += blockDim.x) b[i] = a[i];
+    __syncthreads();
+    if (dst.T.x < 0 || !dst.tape.p[0]) return;
+    const TapeDev& tp = dst.tape;
+    SimDev& S = dst.S;
+    const int i = threadIdx.x, step = load_step(dst.ctl) + k, par = step & 1;
+    const long long slot = step - tp.step0;
+    const bool last = step == tp.last, first = step == tp.first;
+    if (i < 4) {                              // x, y, vx, vy (consecutive members, as below)
+        (&S.x)[i] = tp.p[i] + slot * tp.sp;
+        if (!last) (&S.xo)[i] = tp.p[i] + (slot + 1) * tp.sp;
+    } else if (i < TAPE_P) {                  // the ping-pong pairs
+        float** pair = i < 8 ? S.sxx + 2 * (i - 4) : i == 8 ? S.rho : i == 9 ? S.vol : S.vsc;
+        if (tp.p[i]) {
+            pair[par] = tp.p[i] + slot * tp.sp;
+            if (!last) pair[par ^ 1] = tp.p[i] + (slot + 1) * tp.sp;
+        }
+    } else if (i >= 32 && i < 32 + TAPE_N) {  // m, vA, vB, aB
+        if (!last) (&S.nm)[i - 32] = tp.n[i - 32] + slot * tp.sn;
+    } else if (i == 64) {
+        S.cflag = tp.cflag + slot * tp.sc;
+        if (!last) S.cflago = tp.cflag + (slot + 1) * tp.sc;
+    } else if (i == 96 && !first) {
+        S.nvpx = tp.n[3] + (slot - 1) * tp.sn;
+        S.nvpy = tp.n[4] + (slot - 1) * tp.sn;
+    }
     __syncthreads();
 }
 
@@ -615,8 +649,8 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
         const float pyn = flush(node_sum(s_c + 8, tid));
         float vx, vy;
         if (mass == 0.0f) {
-            vx = S.nvbx[node];
-            vy = S.nvby[node];
+            vx = S.nvpx[node];
+            vy = S.nvpy[node];
         } else {
             vx = fdv(pxn, mass);
             vy = fdv(pyn, mass);
@@ -643,7 +677,7 @@ template <bool REINIT, int MINB = TILE_CTAS_LIGHT>
 __global__ void __launch_bounds__(TILE_THREADS, MINB)
 k_nodal_kinematics_batch(const TileDesc* __restrict__ td, int k) {
     __shared__ TileDesc sT;
-    load_tile(td + blockIdx.x, sT);
+    load_tile(td + blockIdx.x, sT, k);
     if (sT.T.x < 0) return;   // past the listed tiles
     nodal_kinematics_tile<REINIT, true>(sT.S, sT.T, sT.ctl, k, &sT);
 }
@@ -1047,7 +1081,7 @@ template <bool USL, bool REINIT, bool TRAC, int MODE = FM_ROW>
 __global__ void __launch_bounds__(TILE_THREADS, TILE_MIN_CTAS)
 k_forces_batch(const TileDesc* __restrict__ td, int k) {
     __shared__ TileDesc sT;
-    load_tile(td + blockIdx.x, sT);
+    load_tile(td + blockIdx.x, sT, k);
     if (sT.T.x < 0) return;   // past the listed tiles
     forces_tile<USL, REINIT, TRAC, true, MODE>(sT.S, sT.T, sT.ctl, k, &sT);
 }
@@ -1177,10 +1211,10 @@ __device__ __forceinline__ float2 g2p_particle(const SimDev& S, int q, const flo
         if (c.y) vy = S.pvc_vel[c.y - 1];
     }
     const float xn = fa(x, fm(vhx, dt)), yn = fa(y, fm(vhy, dt));
-    S.x[q] = xn;
-    S.y[q] = yn;
-    S.vx[q] = vx;
-    S.vy[q] = vy;
+    S.xo[q] = xn;
+    S.yo[q] = yn;
+    S.vxo[q] = vx;
+    S.vyo[q] = vy;
     if constexpr (USL) {
         float Gcx[4], Gcy[4], c0, c1, c3;
         dshape4(0.0f, 0.0f, g.rx, g.ry, Gcx, Gcy);
@@ -1376,7 +1410,7 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
         const int si = c0x + 1 + lane;
         if (si < S.nx) {
             const int f = s_flag[w][lane];
-            S.cflag[sj * S.nx + si] = (uint8_t)f;
+            S.cflago[sj * S.nx + si] = (uint8_t)f;
             if (f) status |= ST_DRIFTED;
         }
     }
@@ -1400,7 +1434,7 @@ template <bool USL, bool REINIT, int MINB = (USL ? TILE_MIN_CTAS : TILE_CTAS_LIG
 __global__ void __launch_bounds__(TILE_THREADS, MINB)
 k_particle_kinematics_batch(const TileDesc* __restrict__ td, int k) {
     __shared__ TileDesc sT;
-    load_tile(td + blockIdx.x, sT);
+    load_tile(td + blockIdx.x, sT, k);
     if (sT.T.x < 0) return;   // past the listed tiles
     // no particle stored in the tile's sort-cells or around them: nothing
     // moves, and the sort-cells' drift flags are already clear (a flag is set
@@ -1632,6 +1666,23 @@ k_compact_tiles(const int* __restrict__ flags, const int4* __restrict__ tiles, i
         counts[0] = base[0];
         counts[1] = base[1];
     }
+}
+
+// flags[t] |= more[t]
+__global__ void k_or_flags(int* __restrict__ flags, const int* __restrict__ more, int n) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) flags[t] |= more[t];
+}
+
+cudaError_t launch_or_flags(int* flags, const int* more, int n, cudaStream_t s) {
+    if (n > 0) k_or_flags<<<(n + 255) / 256, 256, 0, s>>>(flags, more, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_compact_tiles(const int* flags, const int4* tiles, int ntiles, int4* active, int4* empty,
+                                 int* counts, cudaStream_t s) {
+    if (ntiles > 0) k_compact_tiles<<<1, 1024, 0, s>>>(flags, tiles, ntiles, active, empty, counts);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_classify_tiles(const SimDev& S, const int4* tiles, int ntiles, int* flags, int4* active,

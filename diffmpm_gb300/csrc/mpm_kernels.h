@@ -52,6 +52,11 @@ cudaError_t launch_particle_kinematics(const StepConfig& c, const SimDev& S, con
 // ints of scratch.  Valid until the sort changes.
 cudaError_t launch_classify_tiles(const SimDev& S, const int4* tiles, int ntiles, int* flags, int4* active,
                                   int4* empty, int* counts, cudaStream_t s);
+// The same split from flags alone, and flags[t] |= more[t] (the tiles that hold
+// particles in any of several sorts).
+cudaError_t launch_compact_tiles(const int* flags, const int4* tiles, int ntiles, int4* active, int4* empty,
+                                 int* counts, cudaStream_t s);
+cudaError_t launch_or_flags(int* flags, const int* more, int n, cudaStream_t s);
 // A single simulation launches its empty tiles apart only when it has at
 // least this many (mpm_set_empty_split changes it per handle).
 constexpr int EMPTY_SPLIT_MIN = 128;
@@ -94,9 +99,10 @@ cudaError_t launch_advance_steps(Control* const* ctls, int n, int by, cudaStream
 // t works on simulation tiles[t].x, whose descriptor is sims[tiles[t].x] and
 // whose step counter and status are in ctls[tiles[t].x].
 // out[t] = {tiles[t], ctls[tiles[t].x], *sims[tiles[t].x], row starts,
-// occupancy} for t < ntiles (only out[t].T for a tile (-1, ...)).
-cudaError_t launch_gather_tiles(const SimDev* const* sims, Control* const* ctls, const int4* tiles,
-                                int ntiles, TileDesc* out, cudaStream_t s);
+// occupancy, tapes[tiles[t].x] if any} for t < ntiles (only out[t].T for a
+// tile (-1, ...)).
+cudaError_t launch_gather_tiles(const SimDev* const* sims, Control* const* ctls, const TapeDev* tapes,
+                                const int4* tiles, int ntiles, TileDesc* out, cudaStream_t s);
 cudaError_t launch_nodal_kinematics_batch(const StepConfig& c, const TileDesc* td, int ntiles,
                                           int k, cudaStream_t s);
 cudaError_t launch_forces_batch(const StepConfig& c, const TileDesc* td, int ntiles, int k,

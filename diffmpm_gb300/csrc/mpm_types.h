@@ -69,10 +69,15 @@ struct SimDev {
     int *pid;              // storage index -> original particle index
     const uint8_t *pvc;    // [2 per particle] velocity constraint slot+1 per direction, or null
     const float *pvc_vel;  // particle velocity constraint table
+    // where G2P puts the moved particles (x, y, vx, vy again, or the next
+    // slot of the adjoint's tape)
+    float *xo, *yo, *vxo, *vyo;
     // cells
     int *cstart;
-    uint8_t *cflag;
+    uint8_t *cflag;        // at the step start ...
+    uint8_t *cflago;       // ... and after it (cflag again, or the next tape slot)
     // nodes
+    const float *nvpx, *nvpy;   // velocity of the previous step (nvb, or its tape slot)
     float *nm;
     float *nvax, *nvay;
     float *nvbx, *nvby;
@@ -94,6 +99,23 @@ struct SimDev {
 
 struct Control;
 
+// A simulation's tape (the adjoint's record of every step: particle state and
+// drift flags at the step start, nodal results) as a batched step writes it:
+// step s of the block reads its particles from slot s - step0 and writes them
+// to the next slot, so that the tape costs no copies.  The last step of the
+// block writes the simulation's own arrays, as its first step's nodal
+// velocities come from them.
+constexpr int TAPE_P = 11;   // x y vx vy sxx syy szz sxy rho (vol) (vsc)
+constexpr int TAPE_N = 7;    // m vAx vAy vBx vBy aBx aBy
+struct TapeDev {
+    float* p[TAPE_P];        // slot 0; p[0] null: the step is not taped
+    float* n[TAPE_N];
+    uint8_t* cflag;
+    long long sp, sn, sc;    // slot strides (particles, nodes, cells)
+    int step0, first, last;  // step of slot 0; first and last step of the block
+    int pad;
+};
+
 // One tile of a batched launch together with its simulation's descriptor and
 // control block, so that a CTA fetches everything it needs to start in one
 // contiguous read (refreshed before every step block).  The storage starts
@@ -110,6 +132,7 @@ struct alignas(16) TileDesc {
     int occ;               // a particle is stored in sort-cells [c0x-1, c0x+33) x [c0y-1, c0y+17)
     int pad2[3];
     int cs[TILE_CY][33];   // storage start of cell (c0x + l, c0y + r), l clamped to [0, nx]; 0 off the mesh
+    TapeDev tape;
 };
 static_assert(sizeof(TileDesc) % 16 == 0, "tile records are copied in 16-byte pieces");
 

@@ -407,9 +407,15 @@ class Simulation:
         return {"resorts": a.value, "rollbacks": b.value}
 
     # ------------------------------------------------------------------
+    def set_tape_limit(self, nbytes):
+        """Bound the memory of a run that :meth:`record` keeps whole (0: always
+        checkpoints, negative: the default bound); the same gradients."""
+        self._ok(self._lib.mpm_set_tape_limit(self._h, int(nbytes)))
+
     def record(self, nsteps, checkpoint_steps=100, stream=None):
-        """Advance ``nsteps`` steps keeping a checkpoint every
-        ``checkpoint_steps`` steps for :meth:`adjoint`."""
+        """Advance ``nsteps`` steps keeping what :meth:`adjoint` needs: every
+        step's start state when that fits a bounded share of the device
+        memory, else a checkpoint every ``checkpoint_steps`` steps."""
         self._ok(self._lib.mpm_record(self._h, int(nsteps), int(checkpoint_steps), stream))
 
     def adjoint(self, dl_dloc, dl_dvel=None, *, want=("youngs_modulus", "loc", "velocity")):

@@ -257,11 +257,20 @@ int mpm_get_counters(const MpmHandle* h, int64_t* resorts, int64_t* rollbacks);
  * or USL, with or without the per-step volume set-up, particle tractions and
  * particle velocity constraints.
  *
- * mpm_record advances `nsteps` steps like mpm_step and keeps a checkpoint of
- * the full state every `checkpoint_steps` steps (and at the end); on a
- * Linear1D mesh it keeps every step's start state instead (checkpoint_steps
- * is not used). */
+ * mpm_record advances `nsteps` steps like mpm_step and keeps every step's start
+ * state and nodal results (the tape) when they take at most a tenth of the
+ * device's memory and a quarter of what is free (mpm_set_tape_limit lowers
+ * that).  Otherwise it keeps a checkpoint of the full state every
+ * `checkpoint_steps` steps (and at the end) and the tape of the last
+ * checkpoint_steps steps.  A Linear1D mesh always keeps the tape.  The
+ * gradients are the same bits either way. */
 int mpm_record(MpmHandle* h, int nsteps, int checkpoint_steps, void* stream);
+
+/* Bound, in bytes, on the tape of a run that mpm_record keeps whole (0: always
+ * checkpoints; negative, the default: the bound above).  In a batch the least
+ * of the members' bounds holds for the whole batch.  Applies from the next
+ * record.  No counterpart in the reference. */
+int mpm_set_tape_limit(MpmHandle* h, int64_t bytes);
 
 /* Gradient of a loss L(x_end, v_end) through the steps of the last
  * mpm_record, given dL/dx_end (n, ndim) and dL/dv_end (n, ndim; NULL = zero) in
@@ -269,7 +278,7 @@ int mpm_record(MpmHandle* h, int nsteps, int checkpoint_steps, void* stream);
  * dL/dE (n; per-particle Young's modulus, or the material's modulus counted
  * per particle: the sum over a material's particles is dL/dE of that
  * material), dL/dx_0 (n, ndim) and dL/dv_0 (n, ndim) at the recorded start; NULL
- * outputs are skipped.  Each segment between checkpoints is re-run to rebuild
+ * outputs are skipped.  Each segment that is not on the tape is re-run to rebuild
  * its per-step tape.  The handle is left at the recorded end state, so the
  * call may be repeated with other seeds; any call that changes the state
  * (step, write, set) in between makes it return MPM_ERR_STATE. */
