@@ -855,8 +855,8 @@ int mpm_write_field(MpmHandle* h, int field, const void* src, int on_device, voi
         return sync(h, s);
     }
     if (field == MPM_FIELD_YOUNGS_MODULUS && !h->has_E) {
-        TRY(dalloc(h, &h->ps[0].E, n));
-        TRY(dalloc(h, &h->ps[1].E, n));
+        for (PSet& q : h->ps)   // (kept when the particles are set again)
+            if (!q.E) TRY(dalloc(h, &q.E, n));
         h->has_E = true;
         bind_particles(h);
         TRY(upload_desc(h));

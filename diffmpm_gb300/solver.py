@@ -132,8 +132,8 @@ class MPMExplicit:
         sets, mats, mat_index, offsets = self._population()
         ndim = sim.ndim
         loc = np.concatenate([p.loc.reshape(len(p), ndim) for p in sets])
-        mids = np.concatenate([np.asarray([mat_index[id(p.materials[k])] for k in p.material_ids],
-                                          dtype=np.int32).reshape(-1) for p in sets])
+        mids = np.concatenate([np.asarray([mat_index[id(m)] for m in p.materials],
+                                          dtype=np.int32)[p.material_ids] for p in sets])
         sim.set_particles(loc, mids)
         sim.write("velocity", np.concatenate([p.velocity.reshape(len(p), ndim) for p in sets]))
         sim.write("stress", np.concatenate([p.stress.reshape(len(p), 6) for p in sets]))
