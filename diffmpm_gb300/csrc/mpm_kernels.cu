@@ -200,81 +200,6 @@ __device__ __forceinline__ void apply_constraint(const SimDev& S, uint16_t code,
 // (storage order within the cell), so on an undrifted tile they give bitwise
 // the same partials.
 // ---------------------------------------------------------------------------
-constexpr int HALO_W = TILE_CX + 2;   // sort-cells checked for drift: [c0x-1, c0x+33)
-constexpr int HALO_H = TILE_CY + 2;   //                               [c0y-1, c0y+17)
-constexpr int GEO_C = TILE_CX + 3;    // geometry table columns k <-> cell c0x - 1 + k
-constexpr int GEO_R = TILE_CY + 3;    // geometry table rows    k <-> cell c0y - 1 + k
-
-// Per-tile cell geometry: bounds, centre and 2/width of columns and rows, formed
-// exactly as cell_geo forms them, one 16-byte entry per column and per row.
-struct TileGeo {
-    float4 col[GEO_C];   // (x0, x1, cx, rx) of cell column c0x - 1 + k
-    float4 row[GEO_R];   // (y0, y1, cy, ry) of cell row    c0y - 1 + k
-};
-
-__device__ __forceinline__ float4 axis_geo(int i, float h) {
-    const float a = node_coord(i, h), b = node_coord(i + 1, h);
-    return make_float4(a, b, fm(fa(a, b), 0.5f), fdv(2.0f, fs(b, a)));
-}
-
-__device__ __forceinline__ void build_geo(const SimDev& S, int c0x, int c0y, TileGeo& G) {
-    const int t = threadIdx.x;
-    if (t < GEO_C) G.col[t] = axis_geo(c0x - 1 + t, S.hx);
-    else if (t >= 64 && t < 64 + GEO_R) G.row[t - 64] = axis_geo(c0y - 1 + (t - 64), S.hy);
-}
-
-__device__ __forceinline__ CellGeo geo_of(const TileGeo& G, int kc, int kr) {
-    const float4 c = G.col[kc], r = G.row[kr];
-    CellGeo g;
-    g.x0 = c.x;
-    g.x1 = c.y;
-    g.cx = c.z;
-    g.rx = c.w;
-    g.y0 = r.x;
-    g.y1 = r.y;
-    g.cy = r.z;
-    g.ry = r.w;
-    return g;
-}
-
-
-// The cell l in [0, last] whose range [cs[l], cs[l+1]) holds storage index q
-// (the last l with cs[l] <= q; q lies in [cs[0], cs[last+1])).
-__device__ __forceinline__ int cell_of(const int* cs, int last, int q) {
-    int lo = 0, hi = last;
-    #pragma unroll 1
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cs[mid] <= q) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// The tile set-up loads, returned unconsumed so that they stay in flight
-// behind the work that needs none of them: the storage starts of the tile's
-// cell row cj (lane l: column c0x + l, lane 0 also column c0x + 32) and this
-// thread's drift flags of the sort-cells [c0x-1, c0x+33) x [c0y-1, c0y+17)
-// (a particle is at most one cell from its sort-cell; when one of them is set
-// the tile takes the gathering path).
-struct TileLoads {
-    int cs, cs32;          // row starts
-    uint8_t f0, f1;        // drift flags
-    __device__ __forceinline__ int drift() const { return f0 | f1; }
-};
-
-__device__ __forceinline__ void drift_loads(const SimDev& S, int c0x, int c0y, TileLoads& L) {
-    static_assert(HALO_W * HALO_H <= 2 * TILE_THREADS, "two flags per thread");
-    L.f0 = L.f1 = 0;
-    #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int idx = threadIdx.x + e * TILE_THREADS;
-        const int si = c0x - 1 + idx % HALO_W, sj = c0y - 1 + idx / HALO_W;
-        if (idx < HALO_W * HALO_H && si >= 0 && si < S.nx && sj >= 0 && sj < S.ny)
-            (e ? L.f1 : L.f0) = S.cflag[sj * S.nx + si];
-    }
-}
-
 // tile_loads for a batched tile: the row starts come from its record (rec, in
 // shared memory); only the drift flags are loaded.
 __device__ __forceinline__ TileLoads record_loads(const SimDev& S, const TileDesc& rec, int c0x, int c0y,
@@ -285,30 +210,6 @@ __device__ __forceinline__ TileLoads record_loads(const SimDev& S, const TileDes
     drift_loads(S, c0x, c0y, L);
     return L;
 }
-
-__device__ __forceinline__ TileLoads tile_loads(const SimDev& S, int c0x, int c0y, int cj, int lane) {
-    TileLoads L;
-    L.cs = L.cs32 = 0;
-    if (cj >= 0 && cj < S.ny) {
-        const int base = cj * S.nx;
-        L.cs = S.cstart[base + min(max(c0x + lane, 0), S.nx)];
-        if (lane == 0) L.cs32 = S.cstart[base + min(max(c0x + 32, 0), S.nx)];
-    }
-    drift_loads(S, c0x, c0y, L);
-    return L;
-}
-
-// Storage range [rb, re) of the warp's cell row and [cb, ce) of the lane's cell.
-struct RowRange {
-    int rb, re, cb, ce;
-    __device__ __forceinline__ RowRange(const TileLoads& L, int lane) {
-        rb = __shfl_sync(0xffffffffu, L.cs, 0);
-        re = __shfl_sync(0xffffffffu, L.cs32, 0);
-        cb = L.cs;
-        const int next = __shfl_down_sync(0xffffffffu, L.cs, 1);
-        ce = lane < 31 ? next : re;
-    }
-};
 
 // The gathering path's shared memory: the drift flags and storage starts of the
 // sort-cells [c0x-1, c0x+33) x [c0y-1, c0y+17), and per cell of the tile the
@@ -1096,10 +997,6 @@ k_forces_batch(const TileDesc* __restrict__ td, int k) {
 // acceleration, and records per sort-cell whether a particle now lies in
 // another cell (the drift flags).
 // ---------------------------------------------------------------------------
-constexpr int G_W = TILE_CX + 2;   // node tile [c0x, c0x+34) x [c0y, c0y+18)
-constexpr int G_H = TILE_CY + 2;
-constexpr int G2P_MAP = 160;        // particles of a row whose sort-cell is looked up in a map
-
 // New cell along one axis for a coordinate that was in table column k (cell
 // c = base + k): same, or a neighbour by one, decided against the tabulated
 // bounds; otherwise a full locate.
@@ -1119,60 +1016,6 @@ template <bool USL>
 struct G2PStage {
     static constexpr int NF = USL ? GF_N : 4;
     static constexpr int DEPTH = USL ? 2 : 4;
-};
-
-// Per-warp staging of a row's particles in chunks of 32 storage slots that
-// start on 16-byte boundaries: chunk c holds slots rb4 + 32c + [0, 32) with
-// rb4 = rb rounded down to a multiple of 4, copied as 16-byte cp.async pieces
-// (8 per field; NF = 4 fields is one piece per lane).  Pieces wholly past the
-// row end re are skipped; the last piece may read up to 3 slots past re,
-// which the particle arrays' padding (a multiple of 4 slots) covers.  Slot q
-// of chunk c lands in buf[c % DEPTH][f][q - rb4 - 32c].
-template <int NF, int DEPTH>
-struct RowStage16 {
-    static constexpr int NP = (NF * 8 + 31) / 32;   // pieces per lane per chunk
-    float* buf;                 // [DEPTH][NF][32]
-    const float* lp[NP];        // this lane's source array for its piece j (null: none)
-    int doff[NP];               // and its offset in a chunk's [NF][32] block
-    int lo, rb4, re, nch;
-
-    // src: the NF source arrays (null entries are not staged)
-    __device__ __forceinline__ RowStage16(float* b, const float* const* src, int rb, int re_, int lane)
-        : buf(b), lo((lane & 7) * 4), rb4(rb & ~3), re(re_), nch(re_ > rb ? (re_ - (rb & ~3) + 31) / 32 : 0) {
-        #pragma unroll
-        for (int j = 0; j < NP; ++j) {
-            const int p = 32 * j + lane, f = p >> 3;
-            // select the field without indexing src by a runtime value
-            const float* ptr = nullptr;
-            #pragma unroll
-            for (int g = 4 * j; g < 4 * j + 4 && g < NF; ++g)
-                if (f == g) ptr = src[g];
-            lp[j] = p < NF * 8 ? ptr : nullptr;
-            doff[j] = f * 32 + lo;
-        }
-    }
-    __device__ __forceinline__ void issue(int c) {
-        if (c < nch) {
-            const int base = rb4 + 32 * c + lo;
-            float* dst = buf + (c % DEPTH) * (NF * 32);
-            #pragma unroll
-            for (int j = 0; j < NP; ++j)
-                if (lp[j] && base < re) cp_async16(dst + doff[j], lp[j] + base);
-        }
-        cp_async_commit();
-    }
-    __device__ __forceinline__ void prime() {
-        #pragma unroll
-        for (int c = 0; c < DEPTH - 1; ++c) issue(c);
-    }
-    // Issue chunk c + DEPTH - 1 and wait until chunk c has landed (visible to
-    // the whole warp).
-    __device__ __forceinline__ const float (*advance(int c))[32] {
-        issue(c + DEPTH - 1);
-        cp_async_wait<DEPTH - 1>();
-        __syncwarp();
-        return reinterpret_cast<const float (*)[32]>(buf + (c % DEPTH) * (NF * 32));
-    }
 };
 
 // G2P of one particle (storage slot q, staged inputs b[.][lane]) in cell

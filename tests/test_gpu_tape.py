@@ -134,3 +134,20 @@ def test_batched_tape_equals_single(built, names):
                 for k in r:
                     assert np.array_equal(g[k], r[k]), (limit, again, k)
         batch.close()
+
+
+# 20 x 34 listed tiles: the particle passes of the reverse steps go by tile,
+# where the small mesh's go by particle (the mesh around the block does not
+# enter its particles' results)
+@pytest.mark.parametrize("name", list(CASES))
+def test_reverse_by_tile_equals_by_particle(built, name):
+    got = []
+    for nx, ny in ((70, 50), (600, 500)):
+        case = dict(CASES[name], nx=nx, ny=ny, split=1 << 30)
+        if case.pop("loads", False):
+            case.update(newtonian=True)     # (node ids differ between the meshes)
+        sim, _, w = make(**case)
+        sim.record(45, 45)
+        got.append({**{f: sim.read(f) for f in FIELDS[:6]}, **sim.adjoint(w[0], w[1])})
+    for k in got[0]:
+        assert np.array_equal(got[0][k], got[1][k]), k
