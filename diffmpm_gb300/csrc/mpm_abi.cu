@@ -55,7 +55,15 @@ void dfree(MpmHandle* h, void* p) {
 }
 
 int upload_desc(MpmHandle* h) {
+    h->desc_dirty = false;
     CK(h, cudaMemcpy(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice));
+    return MPM_OK;
+}
+
+int flush_desc(MpmHandle* h, cudaStream_t s) {
+    if (!h->desc_dirty) return MPM_OK;
+    CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
+    h->desc_dirty = false;
     return MPM_OK;
 }
 
@@ -123,6 +131,11 @@ int read_ctl(MpmHandle* h, cudaStream_t s) {
     return sync(h, s);
 }
 
+int take_ctl(MpmHandle* h, cudaStream_t s) {
+    CK(h, launch_take_control(h->ctl, h->h_ctl, s));
+    return sync(h, s);
+}
+
 int clear_status(MpmHandle* h, cudaStream_t s) {
     CK(h, cudaMemsetAsync(&h->ctl->status, 0, sizeof(int), s));
     return MPM_OK;
@@ -169,9 +182,10 @@ SortJob sort_job(MpmHandle* h) {
     return J;
 }
 
-// The sorted buffers become the current ones (the device descriptor is the
-// caller's to update).
+// The sorted buffers become the current ones (the device copy of the descriptor
+// is updated when something reads it: flush_desc).
 void sort_done(MpmHandle* h) {
+    h->desc_dirty = true;
     h->pcur ^= 1;
     h->cs_cur ^= 1;
     bind_particles(h);
@@ -193,7 +207,6 @@ int resort(MpmHandle* h, cudaStream_t s) {
     CK(h, launch_sort_move(J, s));
     if (line) CK(h, launch_line_eid(J.start, h->nx, h->line_eid, s));
     sort_done(h);
-    CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
     return MPM_OK;
 }
 
@@ -230,7 +243,7 @@ StepConfig step_config(const MpmHandle* h) {
 int classify_tiles(MpmHandle* h, cudaStream_t s) {
     if (h->ntiles < h->empty_split_min) {   // never enough empty tiles to launch apart
         h->step_tiles = h->dtiles;
-        h->nact = h->ntiles;
+        h->nact = h->nlist = h->ntiles;
         h->nemp = 0;
         return MPM_OK;
     }
@@ -238,15 +251,19 @@ int classify_tiles(MpmHandle* h, cudaStream_t s) {
                                 h->d_tile_counts, s));
     CK(h, cudaMemcpyAsync(h->h_tile_counts, h->d_tile_counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(h, cudaStreamSynchronize(s));
-    if (h->h_tile_counts[1] < h->empty_split_min) {
+    // (also apart when only the active tiles fit the SMs, one each: see resident)
+    const bool fit = h->ntiles > h->sm_count && h->h_tile_counts[0] <= h->sm_count && !h->hs.cnf_ptr &&
+                     h->empty_split_min == EMPTY_SPLIT_MIN;
+    if (h->h_tile_counts[1] < h->empty_split_min && !fit) {
         // too few empty tiles to pay for a launch of their own: the step
         // kernels take every tile (an empty one costs a CTA that only
         // updates its nodes, in a grid that is often under one wave)
         h->step_tiles = h->dtiles;
-        h->nact = h->ntiles;
+        h->nact = h->nlist = h->ntiles;
         h->nemp = 0;
     } else {
         h->step_tiles = h->d_active;
+        h->nlist = h->h_tile_counts[0];
         h->nact = tile_grid(h->h_tile_counts[0], h->ntiles);
         h->nemp = tile_grid(h->h_tile_counts[1], h->ntiles);
     }
@@ -277,7 +294,7 @@ int launch_phase(MpmHandle* h, const SimDev& S, int phase, int k, cudaStream_t s
     return MPM_OK;
 }
 
-int launch_steps(MpmHandle* h, int n, cudaStream_t s) {
+static int launch_steps(MpmHandle* h, int n, cudaStream_t s) {
     for (int i = 0; i < n; ++i)
         for (int p = 0; p < 3; ++p) TRY(launch_phase(h, h->hs, p, i, s));
     CK(h, launch_advance_step(h->ctl, n, s));
@@ -286,11 +303,24 @@ int launch_steps(MpmHandle* h, int n, cudaStream_t s) {
 
 
 
-// n steps: whole graphs of GRAPH_STEPS steps (of the most recently used
-// GRAPH_CACHE configurations), then the rest as launches.
+// Whether the run's steps go in one cooperative launch (see k_steps_resident):
+// a CTA per listed tile fits the SMs, the forces path is the default one and
+// no empty tile's nodes change from step to step.
+bool resident(const MpmHandle* h) {
+    return h->nlist > 0 && h->nlist <= h->sm_count && h->forces_lpc == (h->usl ? 1 : 0) &&
+           !(h->nemp > 0 && h->hs.cnf_ptr);
+}
+
+// n steps: in one resident launch, or as whole graphs of GRAPH_STEPS steps (of
+// the most recently used GRAPH_CACHE configurations) and the rest as launches.
 int run_steps(MpmHandle* h, int n, cudaStream_t s) {
     constexpr size_t GRAPH_CACHE = 8;
     TRY(classify_tiles(h, s));
+    if (n >= RESIDENT_STEPS && resident(h)) {
+        CK(h, launch_empty_nodes(h->hs, h->d_empty, h->nemp, h->ctl, 0, s));
+        CK(h, launch_steps_resident(step_config(h), h->hs, h->step_tiles, h->nlist, h->ctl, h->d_arrived, n, s));
+        return MPM_OK;
+    }
     if (n >= GRAPH_STEPS) {
         const StepKey key = step_key(h);
         size_t at = 0;
@@ -324,6 +354,7 @@ int run_steps(MpmHandle* h, int n, cudaStream_t s) {
 
 int check_status(MpmHandle* h, int& st) {
     st = h->h_ctl->status;
+    if (st & ST_STALLED) return fail(h, MPM_ERR_CUDA, "a wait between the CTAs of a step launch ran out");
     if (st & ST_OUT_OF_MESH)
         return fail(h, MPM_ERR_OUT_OF_MESH,
                     "a particle left the mesh (the reference would give it a wrapped element id)");
@@ -474,15 +505,13 @@ int replay_block(MpmHandle* h, int64_t step0, int B, int& st, cudaStream_t s) {
     st = 0;
     for (int i = 0; i < B; ++i) {
         if (st & ST_DRIFTED) TRY(resort(h, s));
-        TRY(classify_tiles(h, s));
-        TRY(launch_steps(h, 1, s));
+        TRY(run_steps(h, 1, s));
         h->step++;
-        TRY(read_ctl(h, s));
+        TRY(take_ctl(h, s));
         TRY(check_status(h, st));
         if (st & ST_DRIFT_VIOLATION)
             return fail(h, MPM_ERR_CFL, "a particle crossed more than one cell in one step (step %lld)",
                         (long long)h->step - 1);
-        TRY(clear_status(h, s));
     }
     return MPM_OK;
 }
@@ -522,6 +551,7 @@ int mpm_create(const MpmDesc* d, MpmHandle** out) {
 
     MpmHandle* h = new MpmHandle();
     cudaGetDevice(&h->device);
+    cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device);
     // a 1-D mesh sorts its particles as one row of cells (y = 0, hy = 1)
     h->ndim = d->ndim;
     h->nx = d->nelements[0];
@@ -679,6 +709,7 @@ int mpm_create(const MpmDesc* d, MpmHandle** out) {
     A(&h->snap_ctl, 1);
     A(&h->ds, 1);
     A(&h->ctl, 1);
+    A(&h->d_arrived, 1);
 #undef A
     cudaError_t e = cudaMallocHost(&h->h_ctl, sizeof(Control));
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_tile_counts, 2 * sizeof(int));
@@ -922,6 +953,7 @@ int gather_field(MpmHandle* h, int field, void* d, cudaStream_t s) {
         int what = field == MPM_FIELD_ELEMENT_ID ? 0 : field == MPM_FIELD_VOLUME ? 1 : field == MPM_FIELD_MASS ? 2 : 3;
         if (!h->initialized && (what == 1 || what == 2))
             return fail(h, MPM_ERR_STATE, "initialize first");
+        TRY(flush_desc(h, s));
         CK(h, launch_derived_out(h->ds, h->ndim, (int)n, parity(h), h->reinit, what, h->ps[h->pcur].pid, d, s));
     } else if (field == MPM_FIELD_MATERIAL_ID) {
         CK(h, launch_scatter_out_u8(p.mat, p.pid, (int)n, static_cast<int32_t*>(d), s));
@@ -1069,7 +1101,7 @@ int mpm_set_tractions(MpmHandle* h, int n, const int64_t* pid, const int32_t* di
     CK(h, launch_gather_pairs(reinterpret_cast<const uint16_t*>(st8), reinterpret_cast<uint16_t*>(p.tr_fn), p.pid, (int)np, s));
     h->has_trac = true;
     bind_particles(h);
-    CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
+    h->desc_dirty = true;
     return sync(h, s);
 }
 
@@ -1115,7 +1147,7 @@ int mpm_set_particle_velocity_constraints(MpmHandle* h, int n, const int64_t* pi
     CK(h, launch_gather_pairs(static_cast<const uint16_t*>(h->stage), reinterpret_cast<uint16_t*>(p.pvc), p.pid, (int)np, s));
     h->has_pvc = true;
     bind_particles(h);
-    CK(h, cudaMemcpyAsync(h->ds, &h->hs, sizeof(SimDev), cudaMemcpyHostToDevice, s));
+    h->desc_dirty = true;
     return sync(h, s);
 }
 
@@ -1171,7 +1203,10 @@ int mpm_initialize(MpmHandle* h, void* stream) {
     TRY(resort(h, s));
     if (!h->reinit && h->np > 0) {
         if (h->ndim == 1) TRY(line_setup_volume(h, s));
-        else CK(h, launch_setup_volume(h->ds, (int)h->np, parity(h), s));
+        else {
+            TRY(flush_desc(h, s));
+            CK(h, launch_setup_volume(h->ds, (int)h->np, parity(h), s));
+        }
     }
     TRY(read_ctl(h, s));
     int st = 0;
@@ -1233,17 +1268,17 @@ int mpm_step(MpmHandle* h, int nsteps, void* stream) {
         TRY(take_snapshot(h, s));
         TRY(run_steps(h, B, s));
         h->step += B;
-        TRY(read_ctl(h, s));
+        TRY(take_ctl(h, s));
         // a two-cell drift corrupts the rest of the block (a particle may even be
         // thrown out of the mesh by it): roll back before judging anything else
         int st = h->h_ctl->status;
+        if (st & ST_STALLED) TRY(check_status(h, st));
         if (st & ST_DRIFT_VIOLATION) TRY(replay_block(h, step0, B, st, s));
         else TRY(check_status(h, st));
         h->needs_resort = (st & ST_DRIFTED) != 0;
-        TRY(clear_status(h, s));
         nsteps -= B;
     }
-    return sync(h, s);
+    return MPM_OK;   // (every block ends with a wait)
 }
 
 int mpm_get_step(const MpmHandle* h, int64_t* step) {

@@ -555,12 +555,11 @@ int replay_taped(MpmHandle* h, AdjointState* a, int64_t step0, int slot, int B, 
             TRY(capture_epoch(h, a, s));
         }
         TRY(run_taped(h, a, slot + i, 1, s));
-        TRY(read_ctl(h, s));
+        TRY(take_ctl(h, s));
         TRY(check_status(h, st));
         if (st & ST_DRIFT_VIOLATION)
             return fail(h, MPM_ERR_CFL, "a particle crossed more than one cell in one step (step %lld)",
                         (long long)h->step - 1);
-        TRY(clear_status(h, s));
     }
     return MPM_OK;
 }
@@ -585,12 +584,11 @@ int taped_steps(MpmHandle* h, AdjointState* a, int n, cudaStream_t s) {
         const int64_t step0 = h->step;
         TRY(take_snapshot(h, s));
         TRY(run_taped(h, a, slot, B, s));
-        TRY(read_ctl(h, s));
+        TRY(take_ctl(h, s));
         int st = h->h_ctl->status;
         if (st & ST_DRIFT_VIOLATION) TRY(replay_taped(h, a, step0, slot, B, st, s));
         else TRY(check_status(h, st));
         h->needs_resort = (st & ST_DRIFTED) != 0;
-        TRY(clear_status(h, s));
         slot += B;
     }
     return MPM_OK;

@@ -58,6 +58,7 @@ void drop_batch_graphs(MpmBatch* b) {
 }
 
 int prepare_tiles(MpmBatch* b, cudaStream_t s, const TapeDev* tapes) {
+    for (int i = 0; i < (int)b->sims.size(); ++i) BTRY(b, i, flush_desc(b->sims[i], s));
     // the descriptors and row starts change only between step blocks
     // (re-sorts, set-up calls): one record per tile and block lets a CTA fetch
     // its tile, descriptor, control pointer and row starts in one read
@@ -178,6 +179,7 @@ int resort_many(MpmBatch* b, const std::vector<int>& members, cudaStream_t s) {
         sort_done(h);
         puts[k].dst = h->ds;
         puts[k].S = h->hs;
+        h->desc_dirty = false;
     }
     const int r = upload_table(b, table.data(), table.size(), s);
     if (r != MPM_OK) return r;
@@ -499,7 +501,10 @@ int mpm_batch_restart(MpmBatch* b, void* stream) {
     int r = resort_many(b, every, s);
     if (r != MPM_OK) return r;
     for (MpmHandle* h : b->sims) {
-        if (!h->reinit) BCK(b, launch_setup_volume(h->ds, (int)h->np, parity(h), s));
+        if (!h->reinit) {
+            if (flush_desc(h, s) != MPM_OK) return bfail(b, MPM_ERR_CUDA, "%s", h->err.c_str());
+            BCK(b, launch_setup_volume(h->ds, (int)h->np, parity(h), s));
+        }
         h->initialized = true;
     }
     r = read_statuses(b, s);

@@ -127,6 +127,7 @@ struct MpmHandle {
     // descriptors
     mpm::SimDev hs{};
     mpm::SimDev* ds = nullptr;
+    bool desc_dirty = false;         // ds is behind hs (a re-sort swapped the buffers)
     mpm::Control* ctl = nullptr;
     mpm::Control* h_ctl = nullptr;   // pinned mirror
     int4* dtiles = nullptr;
@@ -140,6 +141,9 @@ struct MpmHandle {
     int* d_tile_counts = nullptr;    // [active, empty]
     int* h_tile_counts = nullptr;    // pinned mirror
     int nact = 0, nemp = 0;          // the step kernels' and the empty-node kernel's grids
+    int nlist = 0;                   // tiles on the step kernels' list (nact without its rounding)
+    int sm_count = 0;
+    unsigned* d_arrived = nullptr;   // barrier word of resident steps
     const int4* step_tiles = nullptr; // the step kernels' list: d_active after a split, else dtiles
     int64_t step = 0;
     // staging and pointer tables
@@ -218,6 +222,10 @@ std::vector<float**> movable_f32(MpmHandle* h, PSet& p, bool for_snapshot);
 int ensure_stage(MpmHandle* h, size_t bytes);
 int sync(MpmHandle* h, cudaStream_t s);
 int read_ctl(MpmHandle* h, cudaStream_t s);
+// read_ctl, then clear the drift bit: one launch and a wait.
+int take_ctl(MpmHandle* h, cudaStream_t s);
+// Bring h->ds, the device copy of the descriptor, up to date.
+int flush_desc(MpmHandle* h, cudaStream_t s);
 int clear_status(MpmHandle* h, cudaStream_t s);
 int resort(MpmHandle* h, cudaStream_t s);
 // The parts of a re-sort, for launches over many simulations.
@@ -225,8 +233,8 @@ SortJob sort_job(MpmHandle* h);
 void sort_done(MpmHandle* h);
 // A field of h against the original-order array `aos` (ncomp 0: not a stored field).
 FieldMap field_map(MpmHandle* h, int field, const float* aos);
-// n steps from ctl->step (the tiles classified for the current sort).
-int launch_steps(MpmHandle* h, int n, cudaStream_t s);
+// n steps from ctl->step (classifies the tiles for the current sort).
+int run_steps(MpmHandle* h, int n, cudaStream_t s);
 // Phase `phase` (0 nodal kinematics, 1 forces, 2 G2P) of step ctl->step + k
 // with descriptor S (the handle's own, or one of a taped step).
 int launch_phase(MpmHandle* h, const SimDev& S, int phase, int k, cudaStream_t s);

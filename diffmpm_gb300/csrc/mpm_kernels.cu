@@ -497,7 +497,7 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
     const int ci = c0x + lx, cj = c0y + ly;
     const TileLoads L = REC ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
     const int parity = (load_step(ctl) + k) & 1;
-    const float* __restrict__ rho = S.rho[parity];
+    const float* rho = S.rho[parity];
     const bool node_ok = lx < TILE_NX && ly < TILE_NY && c0x + 1 + lx <= S.nx && c0y + 1 + ly <= S.ny;
     const int node = (c0y + 1 + ly) * (S.nx + 1) + c0x + 1 + lx;
     const uint16_t ncons = node_ok ? S.ncons[node] : 0;   // node-phase input, fetched early
@@ -1287,6 +1287,62 @@ k_particle_kinematics_batch(const TileDesc* __restrict__ td, int k) {
 }
 
 // ---------------------------------------------------------------------------
+// Resident steps: n whole steps in one cooperative launch of a CTA per tile,
+// for runs whose tiles are all resident at once (at most one per SM).  The
+// phases are the tile functions above with a grid barrier between them; each
+// kernel of a step costs such a run 2 to 3 us of launch, block scheduling and
+// drain around a CTA's own 3 to 5 us (144 particles, one tile: 14.1 -> 10.1 us
+// a step; 17k particles, 20 tiles: 22 -> 19).  Every wait is bounded: a CTA that gives
+// up sets ST_STALLED and returns, and so do the others in turn.
+// ---------------------------------------------------------------------------
+constexpr unsigned BARRIER_POLLS = 1u << 22;
+
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, Control* ctl) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (gridDim.x == 1) return true;
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(arrived, 1u);
+        bool ok = false;
+        for (unsigned i = 0; i < BARRIER_POLLS && !ok; ++i) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+            ok = (int)(v - target) >= 0;
+        }
+        __threadfence();
+        s_ok = ok;
+        if (!ok) atomicOr(&ctl->status, ST_STALLED);
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+template <bool USL, bool REINIT, bool TRAC>
+__global__ void __launch_bounds__(TILE_THREADS, 1)
+k_steps_resident(const __grid_constant__ SimDev S, const int4* __restrict__ tiles, Control* ctl,
+                 unsigned* arrived, int n) {
+    const int4 T = tiles[blockIdx.x];
+    unsigned target = 0;
+    #pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        nodal_kinematics_tile<REINIT>(S, T, ctl, k);
+        if (!grid_barrier(arrived, target, ctl)) return;
+        forces_tile<USL, REINIT, TRAC, false, USL ? FM_LPC : FM_ROW>(S, T, ctl, k);
+        if (!grid_barrier(arrived, target, ctl)) return;
+        particle_kinematics_tile<USL, REINIT>(S, T, ctl, k);
+        if (!grid_barrier(arrived, target, ctl)) return;
+        // a two-cell drift: the sequence will be rolled back (every CTA reads
+        // the same bit, which this step's G2P was the last to set)
+        if (__syncthreads_or(threadIdx.x == 0 &&
+                             (*reinterpret_cast<volatile int*>(&ctl->status) & ST_DRIFT_VIOLATION)))
+            return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->step += n;
+}
+
+// ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
 // The step kernels use 50-110 KB of shared memory per CTA and are sized for two
@@ -1299,6 +1355,28 @@ static void prefer_shared(K kernel) {
                              (int)cudaSharedmemCarveoutMaxShared);
         done = true;
     }
+}
+
+template <bool USL, bool REINIT, bool TRAC>
+static cudaError_t steps_resident(const SimDev& S, const int4* tiles, int ntiles, Control* ctl, unsigned* arrived,
+                                  int n, cudaStream_t s) {
+    prefer_shared(k_steps_resident<USL, REINIT, TRAC>);
+    void* args[] = {const_cast<SimDev*>(&S), &tiles, &ctl, &arrived, &n};
+    cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_steps_resident<USL, REINIT, TRAC>), dim3(ntiles),
+                                       dim3(TILE_THREADS), args, 0, s);
+}
+
+cudaError_t launch_steps_resident(const StepConfig& c, const SimDev& S, const int4* tiles, int ntiles, Control* ctl,
+                                  unsigned* arrived, int n, cudaStream_t s) {
+    using Fn = cudaError_t (*)(const SimDev&, const int4*, int, Control*, unsigned*, int, cudaStream_t);
+    static constexpr Fn fns[8] = {
+        steps_resident<false, false, false>, steps_resident<false, false, true>,
+        steps_resident<false, true, false>,  steps_resident<false, true, true>,
+        steps_resident<true, false, false>,  steps_resident<true, false, true>,
+        steps_resident<true, true, false>,   steps_resident<true, true, true>};
+    return fns[c.usl * 4 + c.reinit * 2 + c.traction](S, tiles, ntiles, ctl, arrived, n, s);
 }
 
 // The nodal kinematics and USF G2P kernels come in two builds: 40 registers
@@ -1932,6 +2010,18 @@ __global__ void k_zero_controls(Control* const* __restrict__ ctls, int n) {
 
 cudaError_t launch_zero_controls(Control* const* ctls, int n, cudaStream_t s) {
     if (n > 0) k_zero_controls<<<(n + 127) / 128, 128, 0, s>>>(ctls, n);
+    return cudaGetLastError();
+}
+
+__global__ void k_take_control(Control* ctl, Control* host) {
+    if (threadIdx.x == 0) {
+        *host = *ctl;
+        ctl->status &= ~ST_DRIFTED;
+    }
+}
+
+cudaError_t launch_take_control(Control* ctl, Control* host, cudaStream_t s) {
+    k_take_control<<<1, 32, 0, s>>>(ctl, host);
     return cudaGetLastError();
 }
 

@@ -45,6 +45,15 @@ cudaError_t launch_forces(const StepConfig& c, const SimDev& S, const int4* tile
                           Control* ctl, int k, cudaStream_t s);
 cudaError_t launch_particle_kinematics(const StepConfig& c, const SimDev& S, const int4* tiles,
                                        int ntiles, Control* ctl, int k, cudaStream_t s);
+// n whole steps over at most one tile per SM in one cooperative launch, with
+// the default forces path; advances the step counter.  `arrived`: one word of
+// scratch.  ST_STALLED in the status means that a wait ran out.  A cooperative
+// launch costs about two steps of plain launches, so fewer than RESIDENT_STEPS
+// steps take those (a thrown block whose 200 steps are replayed one at a time:
+// 26.0 ms with one-step resident launches, 21 without).
+constexpr int RESIDENT_STEPS = 8;
+cudaError_t launch_steps_resident(const StepConfig& c, const SimDev& S, const int4* tiles, int ntiles, Control* ctl,
+                                  unsigned* arrived, int n, cudaStream_t s);
 // Split the tile list into active tiles (cells or their ring store a
 // particle; the step kernels' grid) and empty ones (node updates only,
 // k_empty_nodes), in tile order, both padded to ntiles entries with
@@ -224,6 +233,9 @@ cudaError_t launch_compare_segments(const CopyChunk* chunks, unsigned nchunks, i
 
 // *ctls[i] = 0 for i < n.
 cudaError_t launch_zero_controls(Control* const* ctls, int n, cudaStream_t s);
+// *host = *ctl (pinned host memory), then the drift bit of ctl->status is
+// cleared (the bits of errors stay).
+cudaError_t launch_take_control(Control* ctl, Control* host, cudaStream_t s);
 // out[i] = *ctls[i], then ctls[i]->status = 0, for i < n.
 cudaError_t launch_gather_status(Control* const* ctls, int n, Control* out, cudaStream_t s);
 

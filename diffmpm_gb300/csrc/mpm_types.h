@@ -30,7 +30,8 @@ enum StatusBits : int {
     ST_OUT_OF_MESH = 1,     // a particle left the mesh
     ST_DRIFT_VIOLATION = 2, // a particle is more than one cell from its sort-cell
     ST_DRIFTED = 4,         // some particle is in a cell other than its sort-cell
-    ST_TRACTION_CONFLICT = 8
+    ST_TRACTION_CONFLICT = 8,
+    ST_STALLED = 16         // a wait between the CTAs of a launch ran out
 };
 
 enum MatType : int { MAT_LINEAR_ELASTIC = 0, MAT_SIMPLE = 1, MAT_NEWTONIAN = 2 };
