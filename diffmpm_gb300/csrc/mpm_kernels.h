@@ -152,8 +152,8 @@ struct SortJob {
 // in storage order with `buckets`); the arrays' move is apart.
 cudaError_t launch_sort_order(const SortJob& J, int* block_sums, bool buckets, cudaStream_t s);
 cudaError_t launch_sort_move(const SortJob& J, cudaStream_t s);
-// All of it for n simulations (device table), each of at most SORT_MANY_CELLS
-// cells: one CTA scans a simulation's counts.
+// Meshes of at most SORT_MANY_CELLS cells take one launch for the scan, and
+// several simulations (device table) are sorted together.
 constexpr int SORT_MANY_CELLS = 1 << 18;
 cudaError_t launch_sort_many(const SortJob* jobs, int n, int most_np, int most_cells, cudaStream_t s);
 // *puts[i].dst = puts[i].S

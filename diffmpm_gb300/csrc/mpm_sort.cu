@@ -159,37 +159,88 @@ __global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__
     if (i == n) out[n] = block_sums[gridDim.x];   // grand total
 }
 
-// The counts of one job by one CTA, 8 per thread and round.
-__device__ __forceinline__ void sort_scan(const SortJob& J) {
-    const int n = J.nx * J.ny + 1;
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    #pragma unroll 1
-    for (int base = 0; base < n; base += 8 * 1024) {
-        const int i0 = base + 8 * (int)threadIdx.x;
-        int v[8], sum = 0;
-        #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            v[k] = i0 + k < n ? J.count[i0 + k] : 0;
-            sum += v[k];
+// Chunk c of a job's counts by one CTA, start[n] with the last one: every CTA
+// adds up the counts before its chunk itself, so that one launch scans them all
+// (up to SORT_MANY_CELLS: the last chunk reads 1 MB of L2).  Bound by the two
+// round trips of loading and storing; 16-byte accesses, the loads of a thread's
+// four pieces in flight together (21k cells: 14.4 us by one CTA 8 counts a
+// thread and round, 3.5 so; a three-launch scan takes 8).
+constexpr int SCAN_PIECES = 4, SCAN_CHUNK = SCAN_PIECES * 4 * 1024;
+__device__ __forceinline__ void sort_scan(const SortJob& J, int c) {
+    const int n = J.nx * J.ny + 1, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int base = c * SCAN_CHUNK;
+    if (base >= n) return;
+    __shared__ int s_part[SCAN_PIECES * 32], s_before[32], s_carry;
+    const int4* __restrict__ in = reinterpret_cast<const int4*>(J.count);
+    int4 v[SCAN_PIECES];
+    #pragma unroll
+    for (int r = 0; r < SCAN_PIECES; ++r) {
+        const int i = base + 4 * (r * 1024 + t);
+        v[r] = make_int4(0, 0, 0, 0);
+        if (i + 4 <= n) {
+            v[r] = in[i >> 2];
+        } else {
+            if (i < n) v[r].x = J.count[i];
+            if (i + 1 < n) v[r].y = J.count[i + 1];
+            if (i + 2 < n) v[r].z = J.count[i + 2];
         }
-        int total;
-        int at = carry + block_exclusive_scan(sum, &total);
-        #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (i0 + k < n) J.start[i0 + k] = at;
-            at += v[k];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) carry += total;
-        __syncthreads();
     }
-    if (threadIdx.x == 0) J.start[n] = carry;
+    int before = 0;
+    #pragma unroll 8
+    for (int i = t; i < base / 4; i += 1024) {
+        const int4 w = in[i];
+        before += w.x + w.y + w.z + w.w;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) s_before[warp] = before;
+    int at[SCAN_PIECES];
+    #pragma unroll
+    for (int r = 0; r < SCAN_PIECES; ++r) {
+        const int own = v[r].x + v[r].y + v[r].z + v[r].w;
+        at[r] = own;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, at[r], o);
+            if (lane >= o) at[r] += u;
+        }
+        if (lane == 31) s_part[r * 32 + warp] = at[r];
+        at[r] -= own;
+    }
+    __syncthreads();
+    if (warp == 0) {   // the warps' sums, piece after piece
+        int4 q = reinterpret_cast<const int4*>(s_part)[lane];
+        const int own = q.x + q.y + q.z + q.w;
+        int u = own;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(0xffffffffu, u, o);
+            if (lane >= o) u += w;
+        }
+        u += __reduce_add_sync(0xffffffffu, s_before[lane]);
+        if (lane == 31) s_carry = u;
+        u -= own;
+        q = make_int4(u, u + q.x, u + q.x + q.y, u + q.x + q.y + q.z);
+        reinterpret_cast<int4*>(s_part)[lane] = q;
+    }
+    __syncthreads();
+    #pragma unroll
+    for (int r = 0; r < SCAN_PIECES; ++r) {
+        const int i = base + 4 * (r * 1024 + t);
+        const int a = at[r] + s_part[r * 32 + warp];
+        const int4 q = make_int4(a, a + v[r].x, a + v[r].x + v[r].y, a + v[r].x + v[r].y + v[r].z);
+        if (i + 4 <= n) {
+            reinterpret_cast<int4*>(J.start)[i >> 2] = q;
+        } else {
+            if (i < n) J.start[i] = q.x;
+            if (i + 1 < n) J.start[i + 1] = q.y;
+            if (i + 2 < n) J.start[i + 2] = q.z;
+        }
+    }
+    if (t == 0 && n - base <= SCAN_CHUNK) J.start[n] = s_carry;
 }
-__global__ void __launch_bounds__(1024) k_sort_scan(const __grid_constant__ SortJob J) { sort_scan(J); }
+__global__ void __launch_bounds__(1024) k_sort_scan(const __grid_constant__ SortJob J) { sort_scan(J, blockIdx.x); }
 __global__ void __launch_bounds__(1024) k_sort_scan_many(const SortJob* __restrict__ jobs) {
-    sort_scan(jobs[blockIdx.x]);
+    sort_scan(jobs[blockIdx.x], blockIdx.y);
 }
 
 __global__ void k_put_descs(const DescPut* __restrict__ puts, int n) {
@@ -272,19 +323,12 @@ cudaError_t launch_gather_pairs(const float2* src, float2* dst, const int* perm,
     return cudaGetLastError();
 }
 
-// Counts that one CTA scans (four rounds of a load, a scan and a store), for
-// less than the two launches that the scan of many CTAs adds.  A thrown block
-// re-sorts before every step: with this, the status taken and cleared by one
-// launch and the descriptor's device copy left to its readers, its 200 replayed
-// steps went from 105 to 90 us each (6528 particles in 21k cells).
-constexpr int SCAN_ONE_CTA = 32 * 1024;
-
 cudaError_t launch_sort_order(const SortJob& J, int* block_sums, bool buckets, cudaStream_t s) {
     const int nb = J.nx * J.ny + 1, n = (nb + 1024) / 1024;   // room for start[nb]
     k_sort_clear<<<one_grid(nb), XFER_THREADS, 0, s>>>(J);
     if (J.np > 0) k_sort_keys<<<one_grid(J.np), XFER_THREADS, 0, s>>>(J);
-    if (nb <= SCAN_ONE_CTA) {
-        k_sort_scan<<<1, 1024, 0, s>>>(J);
+    if (nb - 1 <= SORT_MANY_CELLS) {
+        k_sort_scan<<<(nb + SCAN_CHUNK - 1) / SCAN_CHUNK, 1024, 0, s>>>(J);
     } else {
         k_scan_blocks<<<n, 1024, 0, s>>>(J.count, J.start, nb, block_sums);
         k_scan_sums<<<1, 1024, 0, s>>>(block_sums, n);
@@ -305,7 +349,7 @@ cudaError_t launch_sort_many(const SortJob* jobs, int n, int most_np, int most_c
     const dim3 gp = many_grid(n, most_np), gc = many_grid(n, most_cells + 1);
     k_sort_clear_many<<<gc, XFER_THREADS, 0, s>>>(jobs);
     k_sort_keys_many<<<gp, XFER_THREADS, 0, s>>>(jobs);
-    k_sort_scan_many<<<n, 1024, 0, s>>>(jobs);
+    k_sort_scan_many<<<dim3(n, (most_cells + SCAN_CHUNK) / SCAN_CHUNK), 1024, 0, s>>>(jobs);
     k_sort_place_many<<<gp, XFER_THREADS, 0, s>>>(jobs);
     k_sort_buckets_many<<<gc, XFER_THREADS, 0, s>>>(jobs);
     k_sort_move_many<<<gp, XFER_THREADS, 0, s>>>(jobs);
