@@ -93,6 +93,21 @@ __device__ __forceinline__ bool in_cell(const CellGeo& g, float x, float y) {
     return g.x0 <= x && x < g.x1 && g.y0 <= y && y < g.y1;
 }
 
+// Two sums in one instruction, each rounded as fa rounds it.
+__device__ __forceinline__ float2 fa2(float2 a, float2 b) {
+    float2 c;
+    asm("{\n\t"
+        ".reg .b64 x, y, z;\n\t"
+        "mov.b64 x, {%2, %3};\n\t"
+        "mov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 z, x, y;\n\t"
+        "mov.b64 {%0, %1}, z;\n\t"
+        "}"
+        : "=f"(c.x), "=f"(c.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return c;
+}
+
 // Natural coordinate (x - (x0+x1)/2) * (2/(x1-x0)) (diffmpm/particle.py:203-205).
 __device__ __forceinline__ float natural(float x, float c, float r) { return fm(fs(x, c), r); }
 
