@@ -1113,38 +1113,40 @@ __device__ __forceinline__ float2 g2p_particle(const SimDev& S, int q, const flo
     return make_float2(xn, yn);
 }
 
-template <bool USL, bool REINIT, bool REC = false>
+// The tile's rows from row0 on, CY of them (a warp each).
+template <bool USL, bool REINIT, bool REC = false, int CY = TILE_CY>
 __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const int4 T,
                                                          Control* __restrict__ ctl, int k,
-                                                         const TileDesc* rec = nullptr) {
+                                                         const TileDesc* rec = nullptr, int row0 = 0) {
+    constexpr int NODE_H = CY + 2, THREADS = CY * TILE_CX;   // node rows of the CTA's cells
     constexpr int NF = G2PStage<USL>::NF, DEPTH = G2PStage<USL>::DEPTH;
-    __shared__ float4 s_nd[G_W * G_H];    // nodal (vx, vy, ax, ay) of the tile's nodes
-    __shared__ __align__(16) float s_stage[TILE_CY][DEPTH][NF][32];
-    __shared__ int s_cs[TILE_CY][33];
-    __shared__ unsigned char s_map[TILE_CY][G2P_MAP];   // sort-cell of the row's first particles
-    __shared__ int s_flag[TILE_CY][32];   // drift flag after this step
+    __shared__ float4 s_nd[G_W * NODE_H];    // nodal (vx, vy, ax, ay) of the tile's nodes
+    __shared__ __align__(16) float s_stage[CY][DEPTH][NF][32];
+    __shared__ int s_cs[CY][33];
+    __shared__ unsigned char s_map[CY][G2P_MAP];   // sort-cell of the row's first particles
+    __shared__ int s_flag[CY][32];   // drift flag after this step
     __shared__ int s_status;
     __shared__ TileGeo G;
     const int tid = threadIdx.x, lane = tid & 31, w = tid / 32;
-    const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
+    const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1 + row0;
     // row w + 1 of the tile: owned sort-cells c0x+1 .. c0x+31 -> starts cs[0..31]
     const int sj = c0y + 1 + w;
-    const bool row_ok = w < TILE_NY && sj < S.ny;
+    const bool row_ok = w + row0 < TILE_NY && sj < S.ny;
     const int col = min(c0x + 1 + lane, S.nx);
-    // (a batched tile's row starts come with its record: row w + 1,
+    // (a batched tile's row starts come with its record: row w + 1 + row0,
     // column lane + 1 of the record's table)
-    const int cs_l = row_ok ? (REC ? rec->cs[w + 1][lane + 1] : S.cstart[sj * S.nx + col]) : 0;
+    const int cs_l = row_ok ? (REC ? rec->cs[w + 1 + row0][lane + 1] : S.cstart[sj * S.nx + col]) : 0;
     const uint8_t fl = row_ok && col < S.nx ? S.cflag[sj * S.nx + col] : 0;
     // the node tile, both entries of a thread in flight together and with the
     // row starts and the rows' first chunks
-    static_assert(G_W * G_H <= 2 * TILE_THREADS, "two node-tile entries per thread");
+    static_assert(G_W * NODE_H <= 2 * THREADS, "two node-tile entries per thread");
     float4 nd[2];
     #pragma unroll
     for (int e = 0; e < 2; ++e) {
-        const int idx = tid + e * TILE_THREADS;
+        const int idx = tid + e * THREADS;
         const int I = c0x + idx % G_W, J = c0y + idx / G_W;
         nd[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (idx < G_W * G_H && I >= 0 && I <= S.nx && J >= 0 && J <= S.ny) {
+        if (idx < G_W * NODE_H && I >= 0 && I <= S.nx && J >= 0 && J <= S.ny) {
             const int n = J * (S.nx + 1) + I;
             nd[e] = make_float4(S.nvbx[n], S.nvby[n], S.nax[n], S.nay[n]);
         }
@@ -1178,7 +1180,7 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
     if constexpr (USL) stage_materials<false>(S);
     #pragma unroll
     for (int e = 0; e < 2; ++e)
-        if (tid + e * TILE_THREADS < G_W * G_H) s_nd[tid + e * TILE_THREADS] = nd[e];
+        if (tid + e * THREADS < G_W * NODE_H) s_nd[tid + e * THREADS] = nd[e];
     if (row_ok && lane < TILE_NX) {
         // storage index rb + j of the row holds a particle of sort-cell s_map[j]
         const int lo = s_cs[w][lane] - rb, hi = min(s_cs[w][lane + 1] - rb, G2P_MAP);
@@ -1236,7 +1238,7 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
         const CellGeo g = in_tile ? geo_of(G, kc, kr) : cell_geo(ci, cj, S.hx, S.hy);
         float4 nd[4];
         const int li = ci - c0x, lj = cj - c0y;
-        if (li >= 0 && li + 1 < G_W && lj >= 0 && lj + 1 < G_H) {
+        if (li >= 0 && li + 1 < G_W && lj >= 0 && lj + 1 < NODE_H) {
             const int a = lj * G_W + li;
             nd[0] = s_nd[a];
             nd[1] = s_nd[a + 1];
@@ -1284,13 +1286,16 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
     if (tid == 0 && s_status) atomicOr(&ctl->status, s_status);
 }
 
-template <bool USL, bool REINIT, int MINB = (USL ? TILE_MIN_CTAS : TILE_CTAS_LIGHT)>
-__global__ void __launch_bounds__(TILE_THREADS, MINB)
+// CY rows of a tile to a CTA: whole tiles, or halves for fewer tiles than the
+// chip holds CTAs (see particle_kinematics).
+template <bool USL, bool REINIT, int MINB = (USL ? TILE_MIN_CTAS : TILE_CTAS_LIGHT), int CY = TILE_CY>
+__global__ void __launch_bounds__(CY * TILE_CX, MINB * (TILE_CY / CY))
 k_particle_kinematics(const __grid_constant__ SimDev S, const int4* __restrict__ tiles,
                       Control* __restrict__ ctl, int k) {
-    const int4 T = tiles[blockIdx.x];
+    constexpr int PARTS = TILE_CY / CY;
+    const int4 T = tiles[blockIdx.x / PARTS];
     if (T.x < 0) return;
-    particle_kinematics_tile<USL, REINIT>(S, T, ctl, k);
+    particle_kinematics_tile<USL, REINIT, false, CY>(S, T, ctl, k, nullptr, blockIdx.x % PARTS * CY);
 }
 
 template <bool USL, bool REINIT, int MINB = (USL ? TILE_MIN_CTAS : TILE_CTAS_LIGHT)>
@@ -1456,13 +1461,28 @@ cudaError_t launch_forces(const StepConfig& c, const SimDev& S, const int4* tile
     return cudaGetLastError();
 }
 
+// From MOVE_WHOLE listed tiles on (two for each of 152 SMs) a CTA moves a whole
+// tile's particles, below that half of one: the halves fill the chip and wait
+// less for their slowest warp (USL, 35 tiles: 7.9 -> 5.9 us; USF, 77: 4.2 ->
+// 3.9), while more CTAs than the chip holds only repeat the set-up (USL, 704
+// tiles: 24.0 us whole, 24.6 in halves; USF, 1173: 21.2 and 23.1).
+constexpr int MOVE_WHOLE = 304;
+
 template <bool USL, bool REINIT>
 static void particle_kinematics(const SimDev& S, const int4* tiles, int ntiles, Control* ctl,
                                 int k, int ctas, cudaStream_t s) {
-    if (!USL && ctas == 2) {
-        prefer_shared(k_particle_kinematics<USL, REINIT, 2>);
-        k_particle_kinematics<USL, REINIT, 2><<<ntiles, TILE_THREADS, 0, s>>>(S, tiles, ctl, k);
+    if (ntiles < MOVE_WHOLE) {
+        constexpr int CY = TILE_CY / 2, MINB = USL ? TILE_MIN_CTAS : 2;
+        prefer_shared(k_particle_kinematics<USL, REINIT, MINB, CY>);
+        k_particle_kinematics<USL, REINIT, MINB, CY><<<2 * ntiles, CY * TILE_CX, 0, s>>>(S, tiles, ctl, k);
         return;
+    }
+    if constexpr (!USL) {
+        if (ctas == 2) {
+            prefer_shared(k_particle_kinematics<USL, REINIT, 2>);
+            k_particle_kinematics<USL, REINIT, 2><<<ntiles, TILE_THREADS, 0, s>>>(S, tiles, ctl, k);
+            return;
+        }
     }
     prefer_shared(k_particle_kinematics<USL, REINIT>);
     k_particle_kinematics<USL, REINIT><<<ntiles, TILE_THREADS, 0, s>>>(S, tiles, ctl, k);
@@ -1531,10 +1551,12 @@ cudaError_t launch_forces_batch(const StepConfig& c, const TileDesc* td, int nti
 
 template <bool USL, bool REINIT>
 static void particle_kinematics_batch(const TileDesc* td, int ntiles, int k, int ctas, cudaStream_t s) {
-    if (!USL && ctas == 2) {
-        prefer_shared(k_particle_kinematics_batch<USL, REINIT, 2>);
-        k_particle_kinematics_batch<USL, REINIT, 2><<<ntiles, TILE_THREADS, 0, s>>>(td, k);
-        return;
+    if constexpr (!USL) {
+        if (ctas == 2) {
+            prefer_shared(k_particle_kinematics_batch<USL, REINIT, 2>);
+            k_particle_kinematics_batch<USL, REINIT, 2><<<ntiles, TILE_THREADS, 0, s>>>(td, k);
+            return;
+        }
     }
     prefer_shared(k_particle_kinematics_batch<USL, REINIT>);
     k_particle_kinematics_batch<USL, REINIT><<<ntiles, TILE_THREADS, 0, s>>>(td, k);
