@@ -200,13 +200,15 @@ __device__ __forceinline__ void apply_constraint(const SimDev& S, uint16_t code,
 // (storage order within the cell), so on an undrifted tile they give bitwise
 // the same partials.
 // ---------------------------------------------------------------------------
-// tile_loads for a batched tile: the row starts come from its record (rec, in
-// shared memory); only the drift flags are loaded.
-__device__ __forceinline__ TileLoads record_loads(const SimDev& S, const TileDesc& rec, int c0x, int c0y,
+// The row starts of a tile in shared memory: a batched tile's record holds them,
+// resident steps keep them.  tile_loads for such a tile: only the drift flags
+// are loaded.
+using RowStarts = int[TILE_CY][33];
+__device__ __forceinline__ TileLoads record_loads(const SimDev& S, const RowStarts& cs, int c0x, int c0y,
                                                   int r, int lane) {
     TileLoads L;
-    L.cs = rec.cs[r][lane];
-    L.cs32 = lane == 0 ? rec.cs[r][32] : 0;
+    L.cs = cs[r][lane];
+    L.cs32 = lane == 0 ? cs[r][32] : 0;
     drift_loads(S, c0x, c0y, L);
     return L;
 }
@@ -243,7 +245,10 @@ __device__ __forceinline__ void gather_setup(const SimDev& S, int c0x, int c0y, 
 // (lx, ly), geometry g: the sort-cells around it row by row; a neighbour is
 // scanned only when its drift flag is set, and particles of a flagged
 // sort-cell are tested.  (Sort-cells off the mesh are never flagged.)
-template <class F>
+// WIDE: four positions in flight at a time.  (Resident steps of drifted tiles:
+// 2050 -> 1820 us for 100 steps of 54 tiles, 962 -> 893 of one; the kernels of
+// one phase, where few tiles drift, keep the shorter code: 2 to 5% slower with it.)
+template <bool WIDE, class F>
 __device__ __forceinline__ void visit_cell(const SimDev& S, const GatherTile& W, int lx, int ly,
                                            const CellGeo& g, F&& f) {
     #pragma unroll 1
@@ -253,6 +258,19 @@ __device__ __forceinline__ void visit_cell(const SimDev& S, const GatherTile& W,
             const bool flagged = W.flag[r][c] != 0;
             if (!(r == ly + 1 && c == lx + 1) && !flagged) continue;
             const int b = W.start[r][c], e = W.start[r][c + 1];
+            if (WIDE && flagged) {
+                #pragma unroll 1
+                for (int q0 = b; q0 < e; q0 += 4) {
+                    unsigned in = 0;
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int q = min(q0 + i, e - 1);
+                        if (in_cell(g, S.x[q], S.y[q]) && q0 + i < e) in |= 1u << i;
+                    }
+                    for (; in; in &= in - 1) f(q0 + __ffs(in) - 1);
+                }
+                continue;
+            }
             #pragma unroll 1
             for (int q = b; q < e; ++q) {
                 if (flagged && !in_cell(g, S.x[q], S.y[q])) continue;
@@ -263,9 +281,10 @@ __device__ __forceinline__ void visit_cell(const SimDev& S, const GatherTile& W,
 }
 
 // The number of those particles, with the first GATHER_SLOTS slots kept ...
+template <bool WIDE>
 __device__ __forceinline__ int gather_cell(const SimDev& S, GatherTile& W, int lx, int ly, const CellGeo& g) {
     int n = 0;
-    visit_cell(S, W, lx, ly, g, [&](int q) {
+    visit_cell<WIDE>(S, W, lx, ly, g, [&](int q) {
         if (n < GATHER_SLOTS) W.slot[n][threadIdx.x] = q;
         ++n;
     });
@@ -276,7 +295,7 @@ template <class F>
 __device__ __forceinline__ void for_gathered(const SimDev& S, const GatherTile& W, int lx, int ly,
                                              const CellGeo& g, int n, F&& f) {
     if (n > GATHER_SLOTS) {
-        visit_cell(S, W, lx, ly, g, f);
+        visit_cell<false>(S, W, lx, ly, g, f);
     } else {
         #pragma unroll 1
         for (int i = 0; i < n; ++i) f(W.slot[i][threadIdx.x]);
@@ -486,27 +505,28 @@ constexpr int K1_NF = 5;   // x, y, vx, vy, rho (solve_jit) or mass (solve)
 // starting anywhere in a 16-byte piece, fits one pass (three CTAs per SM)
 constexpr int K1_ROW_P = 132;
 
-template <bool REINIT, bool REC = false>
+// starts: the tile's row starts when REC; G: its geometry, filled here unless
+// RES (resident steps keep both, and k is the step itself).
+template <bool REINIT, bool REC = false, bool RES = false>
 __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int4 T,
-                                                      Control* __restrict__ ctl, int k,
-                                                      const TileDesc* rec = nullptr) {
+                                                      Control* __restrict__ ctl, int k, TileGeo& G,
+                                                      const RowStarts* starts = nullptr) {
     constexpr int NQ = 12;
     __shared__ float s_c[NQ][SC_STRIDE];               // [m, px, py] x corner, per cell
     __shared__ union {
         __align__(16) float row[TILE_CY][K1_NF][K1_ROW_P];   // staged particles of each cell row
         GatherTile gather;
     } sh;
-    __shared__ TileGeo G;
     const int tid = threadIdx.x, lx = tid & (TILE_CX - 1), ly = tid / TILE_CX;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
     const int ci = c0x + lx, cj = c0y + ly;
-    const TileLoads L = REC ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
-    const int parity = (load_step(ctl) + k) & 1;
+    const TileLoads L = REC ? record_loads(S, *starts, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
+    const int parity = (RES ? k : load_step(ctl) + k) & 1;
     const float* rho = S.rho[parity];
     const bool node_ok = lx < TILE_NX && ly < TILE_NY && c0x + 1 + lx <= S.nx && c0y + 1 + ly <= S.ny;
     const int node = (c0y + 1 + ly) * (S.nx + 1) + c0x + 1 + lx;
     const uint16_t ncons = node_ok ? S.ncons[node] : 0;   // node-phase input, fetched early
-    build_geo(S, c0x, c0y, G);
+    if constexpr (!RES) build_geo(S, c0x, c0y, G);
     // the row's particles are on their way before the drift flags are known
     const RowRange R(L, lx);
     const float* const src[K1_NF] = {S.x, S.y, S.vx, S.vy, REINIT ? rho : S.mass};
@@ -537,7 +557,7 @@ __device__ __forceinline__ void nodal_kinematics_tile(const SimDev& S, const int
         for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
         if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
             const CellGeo g = geo_of(G, lx + 1, ly + 1);
-            const int cnt = gather_cell(S, sh.gather, lx, ly, g);
+            const int cnt = gather_cell<RES>(S, sh.gather, lx, ly, g);
             const float V0 = REINIT && cnt ? fdv(S.vol_el, (float)cnt) : 0.0f;
             for_gathered(S, sh.gather, lx, ly, g, cnt, [&](int q) {
                 const float m = REINIT ? fm(V0, rho[q]) : S.mass[q];
@@ -576,7 +596,8 @@ k_nodal_kinematics(const __grid_constant__ SimDev S, const int4* __restrict__ ti
                    Control* __restrict__ ctl, int k) {
     const int4 T = tiles[blockIdx.x];
     if (T.x < 0) return;   // past the active tiles
-    nodal_kinematics_tile<REINIT>(S, T, ctl, k);
+    __shared__ TileGeo G;
+    nodal_kinematics_tile<REINIT>(S, T, ctl, k, G);
 }
 
 template <bool REINIT, int MINB = TILE_CTAS_LIGHT>
@@ -585,7 +606,8 @@ k_nodal_kinematics_batch(const TileDesc* __restrict__ td, int k) {
     __shared__ TileDesc sT;
     load_tile(td + blockIdx.x, sT, k);
     if (sT.T.x < 0) return;   // past the listed tiles
-    nodal_kinematics_tile<REINIT, true>(sT.S, sT.T, sT.ctl, k, &sT);
+    __shared__ TileGeo G;
+    nodal_kinematics_tile<REINIT, true>(sT.S, sT.T, sT.ctl, k, G, &sT.cs);
 }
 
 // Nodal update shared by both schemes: concentrated forces (element.py:270-284),
@@ -746,20 +768,20 @@ __device__ __forceinline__ void staged_arrays(const SimDev& S, int parity, int t
     src[tid] = a;
 }
 
-template <bool USL, bool REINIT, bool TRAC, bool VD, int MODE = FM_ROW>
+// starts, G, RES: as in nodal_kinematics_tile.
+template <bool USL, bool REINIT, bool TRAC, bool VD, int MODE = FM_ROW, bool RES = false>
 __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
-                                            Control* __restrict__ ctl, int k,
-                                            const TileDesc* rec = nullptr) {
+                                            Control* __restrict__ ctl, int k, TileGeo& G,
+                                            const RowStarts* starts = nullptr) {
     constexpr int NQ = 8;
     __shared__ __align__(16) ForceShared<MODE, NQ, USL, REINIT> sh;
     auto& s_c = sh.c;                                   // [f x, f y] x corner, per cell
     __shared__ float2 s_v[NV_W * NV_H];   // nodal velocity after phase 1 of the tile's nodes
-    __shared__ TileGeo G;
     const int tid = threadIdx.x, lx = tid & (TILE_CX - 1), ly = tid / TILE_CX;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1;
     const int ci = c0x + lx, cj = c0y + ly;
-    const TileLoads L = VD ? record_loads(S, *rec, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
-    const int step = load_step(ctl) + k;
+    const TileLoads L = VD || RES ? record_loads(S, *starts, c0x, c0y, ly, lx) : tile_loads(S, c0x, c0y, cj, lx);
+    const int step = RES ? k : load_step(ctl) + k;
     const int parity = step & 1;
     const float t = step_time(step, S.dt);
     const bool node_ok = lx < TILE_NX && ly < TILE_NY && c0x + 1 + lx <= S.nx && c0y + 1 + ly <= S.ny;
@@ -781,9 +803,9 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
             nv[e] = make_float2(S.nvax[n], S.nvay[n]);
         }
     }
-    build_geo(S, c0x, c0y, G);
+    if constexpr (!RES) build_geo(S, c0x, c0y, G);
     if constexpr (MODE == FM_STAGED) staged_arrays<USL, REINIT, VD>(S, parity, tid, sh.src);
-    if constexpr (!USL) stage_materials<VD>(S);
+    if constexpr (!USL && !RES) stage_materials<VD>(S);
     if constexpr (MODE != FM_STAGED) {
         #pragma unroll
         for (int q = 0; q < NQ; ++q) s_c[q][tid] = 0.0f;
@@ -966,7 +988,7 @@ __device__ __forceinline__ void forces_tile(const SimDev& S, const int4 T,
         }
         if (ci >= 0 && ci < S.nx && cj >= 0 && cj < S.ny) {
             const CellGeo g = geo_of(G, lx + 1, ly + 1);
-            const int cnt = gather_cell(S, sh.gather, lx, ly, g);
+            const int cnt = gather_cell<RES>(S, sh.gather, lx, ly, g);
             float nvx[4], nvy[4], V0, size0, dvol;
             if (!USL) cell_velocities(lx, ly, nvx, nvy);
             force_cell_values<USL, REINIT, VD, TRAC>(S, cnt, g, nvx, nvy, V0, size0, dvol);
@@ -995,7 +1017,8 @@ k_forces(const __grid_constant__ SimDev S, const int4* __restrict__ tiles,
          Control* __restrict__ ctl, int k) {
     const int4 T = tiles[blockIdx.x];
     if (T.x < 0) return;
-    forces_tile<USL, REINIT, TRAC, false, MODE>(S, T, ctl, k);
+    __shared__ TileGeo G;
+    forces_tile<USL, REINIT, TRAC, false, MODE>(S, T, ctl, k, G);
 }
 
 template <bool USL, bool REINIT, bool TRAC, int MODE = FM_ROW>
@@ -1004,7 +1027,8 @@ k_forces_batch(const TileDesc* __restrict__ td, int k) {
     __shared__ TileDesc sT;
     load_tile(td + blockIdx.x, sT, k);
     if (sT.T.x < 0) return;   // past the listed tiles
-    forces_tile<USL, REINIT, TRAC, true, MODE>(sT.S, sT.T, sT.ctl, k, &sT);
+    __shared__ TileGeo G;
+    forces_tile<USL, REINIT, TRAC, true, MODE>(sT.S, sT.T, sT.ctl, k, G, &sT.cs);
 }
 
 // ---------------------------------------------------------------------------
@@ -1113,11 +1137,12 @@ __device__ __forceinline__ float2 g2p_particle(const SimDev& S, int q, const flo
     return make_float2(xn, yn);
 }
 
-// The tile's rows from row0 on, CY of them (a warp each).
-template <bool USL, bool REINIT, bool REC = false, int CY = TILE_CY>
+// The tile's rows from row0 on, CY of them (a warp each); starts, G, RES: as in
+// nodal_kinematics_tile.
+template <bool USL, bool REINIT, bool REC = false, int CY = TILE_CY, bool RES = false>
 __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const int4 T,
-                                                         Control* __restrict__ ctl, int k,
-                                                         const TileDesc* rec = nullptr, int row0 = 0) {
+                                                         Control* __restrict__ ctl, int k, TileGeo& G,
+                                                         const RowStarts* starts = nullptr, int row0 = 0) {
     constexpr int NODE_H = CY + 2, THREADS = CY * TILE_CX;   // node rows of the CTA's cells
     constexpr int NF = G2PStage<USL>::NF, DEPTH = G2PStage<USL>::DEPTH;
     __shared__ float4 s_nd[G_W * NODE_H];    // nodal (vx, vy, ax, ay) of the tile's nodes
@@ -1126,16 +1151,14 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
     __shared__ unsigned char s_map[CY][G2P_MAP];   // sort-cell of the row's first particles
     __shared__ int s_flag[CY][32];   // drift flag after this step
     __shared__ int s_status;
-    __shared__ TileGeo G;
     const int tid = threadIdx.x, lane = tid & 31, w = tid / 32;
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1 + row0;
     // row w + 1 of the tile: owned sort-cells c0x+1 .. c0x+31 -> starts cs[0..31]
     const int sj = c0y + 1 + w;
     const bool row_ok = w + row0 < TILE_NY && sj < S.ny;
     const int col = min(c0x + 1 + lane, S.nx);
-    // (a batched tile's row starts come with its record: row w + 1 + row0,
-    // column lane + 1 of the record's table)
-    const int cs_l = row_ok ? (REC ? rec->cs[w + 1 + row0][lane + 1] : S.cstart[sj * S.nx + col]) : 0;
+    // (at hand: row w + 1 + row0, column lane + 1 of the table)
+    const int cs_l = row_ok ? (REC ? (*starts)[w + 1 + row0][lane + 1] : S.cstart[sj * S.nx + col]) : 0;
     const uint8_t fl = row_ok && col < S.nx ? S.cflag[sj * S.nx + col] : 0;
     // the node tile, both entries of a thread in flight together and with the
     // row starts and the rows' first chunks
@@ -1151,8 +1174,7 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
             nd[e] = make_float4(S.nvbx[n], S.nvby[n], S.nax[n], S.nay[n]);
         }
     }
-    const int step = load_step(ctl) + k;
-    const int parity = step & 1, next = parity ^ 1;
+    const int parity = (RES ? k : load_step(ctl) + k) & 1, next = parity ^ 1;
     if (tid == 0) s_status = 0;
     s_flag[w][lane] = 0;
     s_cs[w][lane] = cs_l;
@@ -1176,8 +1198,10 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
     RowStage16<NF, DEPTH> st(&s_stage[w][0][0][0], src, rb, re, lane);
     const int rb4 = st.rb4;
     st.prime();
-    build_geo(S, c0x, c0y, G);
-    if constexpr (USL) stage_materials<false>(S);
+    if constexpr (!RES) {
+        build_geo(S, c0x, c0y, G);
+        if constexpr (USL) stage_materials<false>(S);
+    }
     #pragma unroll
     for (int e = 0; e < 2; ++e)
         if (tid + e * THREADS < G_W * NODE_H) s_nd[tid + e * THREADS] = nd[e];
@@ -1295,7 +1319,8 @@ k_particle_kinematics(const __grid_constant__ SimDev S, const int4* __restrict__
     constexpr int PARTS = TILE_CY / CY;
     const int4 T = tiles[blockIdx.x / PARTS];
     if (T.x < 0) return;
-    particle_kinematics_tile<USL, REINIT, false, CY>(S, T, ctl, k, nullptr, blockIdx.x % PARTS * CY);
+    __shared__ TileGeo G;
+    particle_kinematics_tile<USL, REINIT, false, CY>(S, T, ctl, k, G, nullptr, blockIdx.x % PARTS * CY);
 }
 
 template <bool USL, bool REINIT, int MINB = (USL ? TILE_MIN_CTAS : TILE_CTAS_LIGHT)>
@@ -1308,7 +1333,8 @@ k_particle_kinematics_batch(const TileDesc* __restrict__ td, int k) {
     // moves, and the sort-cells' drift flags are already clear (a flag is set
     // only for a sort-cell that stores a particle, and a re-sort clears all)
     if (!sT.occ) return;
-    particle_kinematics_tile<USL, REINIT, true>(sT.S, sT.T, sT.ctl, k, &sT);
+    __shared__ TileGeo G;
+    particle_kinematics_tile<USL, REINIT, true>(sT.S, sT.T, sT.ctl, k, G, &sT.cs);
 }
 
 // ---------------------------------------------------------------------------
@@ -1316,29 +1342,31 @@ k_particle_kinematics_batch(const TileDesc* __restrict__ td, int k) {
 // for runs whose tiles are all resident at once (at most one per SM).  The
 // phases are the tile functions above with a grid barrier between them; each
 // kernel of a step costs such a run 2 to 3 us of launch, block scheduling and
-// drain around a CTA's own 3 to 5 us (144 particles, one tile: 14.1 -> 10.1 us
-// a step; 17k particles, 20 tiles: 22 -> 19).  Every wait is bounded: a CTA that gives
-// up sets ST_STALLED and returns, and so do the others in turn.
+// drain around a CTA's own 3 to 5 us, and the set-up of a tile is done once
+// (144 particles, one tile: 14.1 -> 8.2 us a step; 17k particles with tractions,
+// 20 tiles: 22 -> 17.7, of which the three barriers take 5, skew included).
+// Every wait is bounded: a CTA that gives up sets ST_STALLED and returns, and
+// so do the others in turn.
 // ---------------------------------------------------------------------------
 constexpr unsigned BARRIER_POLLS = 1u << 22;
 
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, Control* ctl) {
+// False for every CTA when the wait ran out or `stop` is set for their threads 0.
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, Control* ctl, bool stop = false) {
     __shared__ int s_ok;
     __syncthreads();
-    if (gridDim.x == 1) return true;
     target += gridDim.x;
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(arrived, 1u);
-        bool ok = false;
-        for (unsigned i = 0; i < BARRIER_POLLS && !ok; ++i) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
-            ok = (int)(v - target) >= 0;
+        bool ok = gridDim.x == 1;
+        if (!ok) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+            for (unsigned i = 0; i < BARRIER_POLLS && !ok; ++i) {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+                ok = (int)(v - target) >= 0;
+            }
+            if (!ok) atomicOr(&ctl->status, ST_STALLED);
         }
-        __threadfence();
-        s_ok = ok;
-        if (!ok) atomicOr(&ctl->status, ST_STALLED);
+        s_ok = ok && !stop;
     }
     __syncthreads();
     return s_ok != 0;
@@ -1348,21 +1376,32 @@ template <bool USL, bool REINIT, bool TRAC>
 __global__ void __launch_bounds__(TILE_THREADS, 1)
 k_steps_resident(const __grid_constant__ SimDev S, const int4* __restrict__ tiles, Control* ctl,
                  unsigned* arrived, int n) {
+    // kept over the steps: the row starts (nothing re-sorts within a sequence),
+    // the geometry and the materials
+    __shared__ RowStarts starts;
+    __shared__ TileGeo G;
     const int4 T = tiles[blockIdx.x];
+    const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1, w = threadIdx.x / 32, lane = threadIdx.x & 31;
+    const int step0 = load_step(ctl);
+    const TileLoads L = tile_loads(S, c0x, c0y, c0y + w, lane);
+    starts[w][lane] = L.cs;
+    if (lane == 0) starts[w][32] = L.cs32;
+    build_geo(S, c0x, c0y, G);
+    stage_materials<false>(S);
     unsigned target = 0;
+    __syncthreads();
     #pragma unroll 1
     for (int k = 0; k < n; ++k) {
-        nodal_kinematics_tile<REINIT>(S, T, ctl, k);
+        // A two-cell drift of the step before: the sequence will be rolled back.
+        // (Its G2P, before the last barrier, was the last to set the bit, and
+        // this step's comes after the next two: every CTA reads the same.)
+        const int status = threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(&ctl->status) : 0;
+        nodal_kinematics_tile<REINIT, true, true>(S, T, ctl, step0 + k, G, &starts);
+        if (!grid_barrier(arrived, target, ctl, status & ST_DRIFT_VIOLATION)) return;
+        forces_tile<USL, REINIT, TRAC, false, USL ? FM_LPC : FM_ROW, true>(S, T, ctl, step0 + k, G, &starts);
         if (!grid_barrier(arrived, target, ctl)) return;
-        forces_tile<USL, REINIT, TRAC, false, USL ? FM_LPC : FM_ROW>(S, T, ctl, k);
+        particle_kinematics_tile<USL, REINIT, true, TILE_CY, true>(S, T, ctl, step0 + k, G, &starts);
         if (!grid_barrier(arrived, target, ctl)) return;
-        particle_kinematics_tile<USL, REINIT>(S, T, ctl, k);
-        if (!grid_barrier(arrived, target, ctl)) return;
-        // a two-cell drift: the sequence will be rolled back (every CTA reads
-        // the same bit, which this step's G2P was the last to set)
-        if (__syncthreads_or(threadIdx.x == 0 &&
-                             (*reinterpret_cast<volatile int*>(&ctl->status) & ST_DRIFT_VIOLATION)))
-            return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->step += n;
 }
