@@ -131,8 +131,8 @@ int read_ctl(MpmHandle* h, cudaStream_t s) {
     return sync(h, s);
 }
 
-int take_ctl(MpmHandle* h, cudaStream_t s) {
-    CK(h, launch_take_control(h->ctl, h->h_ctl, s));
+int take_ctl(MpmHandle* h, cudaStream_t s, int advance) {
+    CK(h, launch_take_control(h->ctl, h->h_ctl, advance, s));
     return sync(h, s);
 }
 
@@ -300,8 +300,6 @@ static int launch_steps(MpmHandle* h, int n, cudaStream_t s) {
     CK(h, launch_advance_step(h->ctl, n, s));
     return MPM_OK;
 }
-
-
 
 // Whether the run's steps go in one cooperative launch (see k_steps_resident):
 // a CTA per listed tile fits the SMs, the forces path is the default one and
@@ -505,9 +503,10 @@ int replay_block(MpmHandle* h, int64_t step0, int B, int& st, cudaStream_t s) {
     st = 0;
     for (int i = 0; i < B; ++i) {
         if (st & ST_DRIFTED) TRY(resort(h, s));
-        TRY(run_steps(h, 1, s));
+        TRY(classify_tiles(h, s));
+        for (int p = 0; p < 3; ++p) TRY(launch_phase(h, h->hs, p, 0, s));
         h->step++;
-        TRY(take_ctl(h, s));
+        TRY(take_ctl(h, s, 1));
         TRY(check_status(h, st));
         if (st & ST_DRIFT_VIOLATION)
             return fail(h, MPM_ERR_CFL, "a particle crossed more than one cell in one step (step %lld)",
@@ -739,6 +738,7 @@ int mpm_create(const MpmDesc* d, MpmHandle** out) {
     for (float* p : {h->nvax, h->nvay, h->nvbx, h->nvby, h->nax, h->nay})
         if (cudaMemset(p, 0, sizeof(float) * h->nn) != cudaSuccess) r = MPM_ERR_CUDA;
     if (cudaMemset(h->cflag, 0, h->ncell) != cudaSuccess) r = MPM_ERR_CUDA;
+    if (cudaMemset(h->sw.count, 0, sizeof(int) * (h->ncell + 1)) != cudaSuccess) r = MPM_ERR_CUDA;
     Control c{};
     up(h->ctl, &c, sizeof c);
     if (r != MPM_OK) return failc(r, "initialisation of the nodal state failed");

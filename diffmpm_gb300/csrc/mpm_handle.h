@@ -222,8 +222,8 @@ std::vector<float**> movable_f32(MpmHandle* h, PSet& p, bool for_snapshot);
 int ensure_stage(MpmHandle* h, size_t bytes);
 int sync(MpmHandle* h, cudaStream_t s);
 int read_ctl(MpmHandle* h, cudaStream_t s);
-// read_ctl, then clear the drift bit: one launch and a wait.
-int take_ctl(MpmHandle* h, cudaStream_t s);
+// Advance the step counter, read_ctl, clear the drift bit: one launch and a wait.
+int take_ctl(MpmHandle* h, cudaStream_t s, int advance = 0);
 // Bring h->ds, the device copy of the descriptor, up to date.
 int flush_desc(MpmHandle* h, cudaStream_t s);
 int clear_status(MpmHandle* h, cudaStream_t s);

@@ -2094,15 +2094,16 @@ cudaError_t launch_zero_controls(Control* const* ctls, int n, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-__global__ void k_take_control(Control* ctl, Control* host) {
+__global__ void k_take_control(Control* ctl, Control* host, int advance) {
     if (threadIdx.x == 0) {
+        ctl->step += advance;
         *host = *ctl;
         ctl->status &= ~ST_DRIFTED;
     }
 }
 
-cudaError_t launch_take_control(Control* ctl, Control* host, cudaStream_t s) {
-    k_take_control<<<1, 32, 0, s>>>(ctl, host);
+cudaError_t launch_take_control(Control* ctl, Control* host, int advance, cudaStream_t s) {
+    k_take_control<<<1, 32, 0, s>>>(ctl, host, advance);
     return cudaGetLastError();
 }
 

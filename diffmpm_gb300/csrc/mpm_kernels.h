@@ -148,8 +148,9 @@ struct SortJob {
     const float2* trtau_src;
     float2* trtau_dst;
 };
-// Clears the counts and drift flags, then count, start and perm (each bucket
-// in storage order with `buckets`); the arrays' move is apart.
+// count, start and perm (each bucket in storage order with `buckets`), and the
+// drift flags cleared; the arrays' move is apart.  With `buckets` the counts
+// are zero before and after.
 cudaError_t launch_sort_order(const SortJob& J, int* block_sums, bool buckets, cudaStream_t s);
 cudaError_t launch_sort_move(const SortJob& J, cudaStream_t s);
 // Meshes of at most SORT_MANY_CELLS cells take one launch for the scan, and
@@ -233,9 +234,9 @@ cudaError_t launch_compare_segments(const CopyChunk* chunks, unsigned nchunks, i
 
 // *ctls[i] = 0 for i < n.
 cudaError_t launch_zero_controls(Control* const* ctls, int n, cudaStream_t s);
-// *host = *ctl (pinned host memory), then the drift bit of ctl->status is
-// cleared (the bits of errors stay).
-cudaError_t launch_take_control(Control* ctl, Control* host, cudaStream_t s);
+// The step counter advances, *host = *ctl (pinned host memory), and the drift
+// bit of ctl->status is cleared (the bits of errors stay).
+cudaError_t launch_take_control(Control* ctl, Control* host, int advance, cudaStream_t s);
 // out[i] = *ctls[i], then ctls[i]->status = 0, for i < n.
 cudaError_t launch_gather_status(Control* const* ctls, int n, Control* out, cudaStream_t s);
 

@@ -72,7 +72,9 @@ __device__ __forceinline__ void sort_key(const SortJob& J, int q) {
 __device__ __forceinline__ void sort_place(const SortJob& J, int q) {
     J.perm[J.start[J.key[q]] + J.rank[q]] = q;
 }
+// (The counts are zero between sorts: a launch less before the keys.)
 __device__ __forceinline__ void sort_bucket(const SortJob& J, int c) {
+    sort_clear(J, c);
     const int b = J.start[c], e = J.start[c + 1];
     int* __restrict__ perm = J.perm;
     #pragma unroll 1
@@ -112,6 +114,9 @@ __device__ __forceinline__ void sort_move(const SortJob& J, int i) {
 struct Particles_ { __device__ int operator()(const SortJob& J) const { return J.np; } };
 struct Buckets_ { __device__ int operator()(const SortJob& J) const { return J.nx * J.ny + 1; } };
 
+__global__ void __launch_bounds__(XFER_THREADS) k_sort_clear(const __grid_constant__ SortJob J) {
+    for_one(J, Buckets_{}, [](const SortJob& j, int i) { sort_clear(j, i); });
+}
 #define MPM_SORT_KERNELS(name, count_of, fn)                                                              \
     __global__ void __launch_bounds__(XFER_THREADS) name(const __grid_constant__ SortJob J) {             \
         for_one(J, count_of{}, [](const SortJob& j, int i) { fn(j, i); });                                \
@@ -119,7 +124,6 @@ struct Buckets_ { __device__ int operator()(const SortJob& J) const { return J.n
     __global__ void __launch_bounds__(XFER_THREADS) name##_many(const SortJob* __restrict__ jobs) {       \
         for_many(jobs, count_of{}, [](const SortJob& j, int i) { fn(j, i); });                            \
     }
-MPM_SORT_KERNELS(k_sort_clear, Buckets_, sort_clear)
 MPM_SORT_KERNELS(k_sort_keys, Particles_, sort_key)
 MPM_SORT_KERNELS(k_sort_place, Particles_, sort_place)
 MPM_SORT_KERNELS(k_sort_buckets, Buckets_, sort_bucket)
@@ -325,7 +329,7 @@ cudaError_t launch_gather_pairs(const float2* src, float2* dst, const int* perm,
 
 cudaError_t launch_sort_order(const SortJob& J, int* block_sums, bool buckets, cudaStream_t s) {
     const int nb = J.nx * J.ny + 1, n = (nb + 1024) / 1024;   // room for start[nb]
-    k_sort_clear<<<one_grid(nb), XFER_THREADS, 0, s>>>(J);
+    if (!buckets) k_sort_clear<<<one_grid(nb), XFER_THREADS, 0, s>>>(J);
     if (J.np > 0) k_sort_keys<<<one_grid(J.np), XFER_THREADS, 0, s>>>(J);
     if (nb - 1 <= SORT_MANY_CELLS) {
         k_sort_scan<<<(nb + SCAN_CHUNK - 1) / SCAN_CHUNK, 1024, 0, s>>>(J);
@@ -347,7 +351,6 @@ cudaError_t launch_sort_move(const SortJob& J, cudaStream_t s) {
 cudaError_t launch_sort_many(const SortJob* jobs, int n, int most_np, int most_cells, cudaStream_t s) {
     if (n < 1) return cudaSuccess;
     const dim3 gp = many_grid(n, most_np), gc = many_grid(n, most_cells + 1);
-    k_sort_clear_many<<<gc, XFER_THREADS, 0, s>>>(jobs);
     k_sort_keys_many<<<gp, XFER_THREADS, 0, s>>>(jobs);
     k_sort_scan_many<<<dim3(n, (most_cells + SCAN_CHUNK) / SCAN_CHUNK), 1024, 0, s>>>(jobs);
     k_sort_place_many<<<gp, XFER_THREADS, 0, s>>>(jobs);
