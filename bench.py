@@ -388,7 +388,7 @@ def plain_scaleup(args, D, workloads, torch):
 def mixed_large(args, D, workloads, torch):
     """The large mixed-material workload: 4096^2 mesh, 16,777,216 particles in
     a LinearElastic and a Newtonian block, USL, dt 2e-7; device-timed steps
-    in graphs of 100 and per-phase kernel times."""
+    in blocks of 100 and per-phase kernel times."""
     K = args.mixed_steps
     solver, g, info = workloads.mixed_large(D, sim_steps=K)
     np_, nn = info["np"], (info["n"] + 1) ** 2
