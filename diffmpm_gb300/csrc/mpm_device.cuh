@@ -16,13 +16,8 @@ __device__ __forceinline__ float fa(float a, float b) { return __fadd_rn(a, b); 
 __device__ __forceinline__ float fs(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdv(float a, float b) { return __fdiv_rn(a, b); }
 
-// Asynchronous 4-byte global -> shared copies (cp.async), committed in groups.
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
-// 16-byte global -> shared copy through L2 only (cp.async.cg); both
-// addresses 16-byte aligned.
+// Asynchronous 16-byte global -> shared copy through L2 only (cp.async.cg),
+// committed in groups; both addresses 16-byte aligned.
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");

@@ -368,8 +368,6 @@ struct ForceIn {
     float x, y, sxx, syy, szz, sxy, rho, vol;
 };
 
-enum ForceField { FF_X, FF_Y, FF_SXX, FF_SYY, FF_SZZ, FF_SXY, FF_RHO, FF_VOL, FF_N };
-
 template <bool VD = false>
 __device__ __forceinline__ ForceIn force_in_global(const SimDev& S, int q, int parity,
                                                    bool reinit) {
