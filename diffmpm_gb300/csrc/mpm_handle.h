@@ -164,7 +164,7 @@ struct MpmHandle {
     float* d_pvc_vel = nullptr;
     bool initialized = false, needs_resort = false;
     int block_steps = 100;
-    int nk_ctas = 3, g2p_ctas = 2;     // kernel builds (StepConfig), set by mpm_set_kernel_variant
+    int nk_ctas = 3, g2p_ctas = 3;     // kernel builds (StepConfig), set by mpm_set_kernel_variant
     int forces_lpc = 0;
     int empty_split_min = mpm::EMPTY_SPLIT_MIN;   // mpm_set_empty_split
     int64_t resorts = 0, rollbacks = 0;

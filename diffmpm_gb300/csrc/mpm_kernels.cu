@@ -1502,7 +1502,7 @@ cudaError_t launch_forces(const StepConfig& c, const SimDev& S, const int4* tile
 // tile's particles, below that half of one: the halves fill the chip and wait
 // less for their slowest warp (USL, 35 tiles: 7.9 -> 5.9 us; USF, 77: 4.2 ->
 // 3.9), while more CTAs than the chip holds only repeat the set-up (USL, 704
-// tiles: 24.0 us whole, 24.6 in halves; USF, 1173: 21.2 and 23.1).
+// tiles: 24.0 us whole, 24.6 in halves; USF, 1173: 20.2 and 23.1).
 constexpr int MOVE_WHOLE = 304;
 
 template <bool USL, bool REINIT>
