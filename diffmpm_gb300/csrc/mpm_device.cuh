@@ -439,8 +439,11 @@ struct RowStage16 {
         for (int c = 0; c < DEPTH - 1; ++c) issue(c);
     }
     // Issue chunk c + DEPTH - 1 and wait until chunk c has landed (visible to
-    // the whole warp).
+    // the whole warp).  The new chunk takes the buffer of chunk c - 1, which
+    // other lanes may still be reading where the work on a particle diverges:
+    // the warp meets before it is overwritten.
     __device__ __forceinline__ const float (*advance(int c))[32] {
+        __syncwarp();
         issue(c + DEPTH - 1);
         cp_async_wait<DEPTH - 1>();
         __syncwarp();
