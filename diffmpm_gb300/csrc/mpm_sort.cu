@@ -174,7 +174,8 @@ __device__ __forceinline__ void sort_scan(const SortJob& J, int c) {
     const int n = J.nx * J.ny + 1, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int base = c * SCAN_CHUNK;
     if (base >= n) return;
-    __shared__ int s_part[SCAN_PIECES * 32], s_before[32], s_carry;
+    __shared__ __align__(16) int s_part[SCAN_PIECES * 32];   // (also read and written four at a time)
+    __shared__ int s_before[32], s_carry;
     const int4* __restrict__ in = reinterpret_cast<const int4*>(J.count);
     int4 v[SCAN_PIECES];
     #pragma unroll
