@@ -25,7 +25,8 @@
 namespace mpm {
 
 // The step counter at the start of the launched sequence.  No kernel that reads
-// it writes it, so it goes through L1: as a volatile load every warp of the
+// it so writes it (resident steps, which advance it, read it once themselves),
+// so it goes through L1: as a volatile load every warp of the
 // grid fetched the same word from L2, which queued there (1024^2: 1850 cycles
 // at the start of every forces CTA, 430 for the load before it).
 __device__ __forceinline__ int load_step(const Control* ctl) { return __ldg(&ctl->step); }
@@ -1380,7 +1381,8 @@ k_steps_resident(const __grid_constant__ SimDev S, const int4* __restrict__ tile
     __shared__ TileGeo G;
     const int4 T = tiles[blockIdx.x];
     const int c0x = T.y * TILE_NX - 1, c0y = T.z * TILE_NY - 1, w = threadIdx.x / 32, lane = threadIdx.x & 31;
-    const int step0 = load_step(ctl);
+    // (read before this CTA's first barrier, advanced by CTA 0 after its last one)
+    const int step0 = *reinterpret_cast<volatile int*>(&ctl->step);
     const TileLoads L = tile_loads(S, c0x, c0y, c0y + w, lane);
     starts[w][lane] = L.cs;
     if (lane == 0) starts[w][32] = L.cs32;
