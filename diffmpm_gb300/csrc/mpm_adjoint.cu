@@ -108,7 +108,8 @@ struct AdjointState {
     int nep = 0;               // epochs captured in the current segment
     int64_t seg_first = 0;     // first step of the taped segment
     // the tiles with particles in any sort of the taped segment (the reverse
-    // node passes' list), valid while every run had its empty tiles apart
+    // node passes' list), valid while every run had its empty tiles apart;
+    // else (all_tiles) they visit every tile
     int* tile_union = nullptr;
     int4 *rtiles = nullptr, *rempty = nullptr;
     int nrtiles = -1;          // grid over rtiles; -1: not formed since the segment was taped
@@ -502,8 +503,10 @@ SimDev slot_desc(MpmHandle* h, AdjointState* a, int slot, int k, int len, int pa
 }
 
 // The taped segment starts: its first epoch and its tile set are the current
-// sort's.
-int tape_begin(MpmHandle* h, AdjointState* a, int len, cudaStream_t s, bool capture = true) {
+// sort's.  Taped by a batch (`batched`), which captures the epochs of all members
+// together and keeps one tile set for them, the member has no tile set of its
+// own: its own adjoint then visits every tile.
+int tape_begin(MpmHandle* h, AdjointState* a, int len, cudaStream_t s, bool batched = false) {
     if (!a->tile_union) {
         TRY(dalloc(h, &a->tile_union, (size_t)h->ntiles));
         TRY(dalloc(h, &a->rtiles, (size_t)h->ntiles));
@@ -511,12 +514,12 @@ int tape_begin(MpmHandle* h, AdjointState* a, int len, cudaStream_t s, bool capt
     }
     CK(h, cudaMemsetAsync(a->tile_union, 0, sizeof(int) * (size_t)h->ntiles, s));
     a->nrtiles = -1;
-    a->all_tiles = false;
+    a->all_tiles = batched;
     a->tape_seg = -1;
     a->seg_first = h->step;
     a->epoch_of.assign(len, 0);
     a->nep = 0;
-    return capture ? capture_epoch(h, a, s) : MPM_OK;
+    return batched ? MPM_OK : capture_epoch(h, a, s);
 }
 
 // Advance len steps within one sort, tape slots slot .. slot + len - 1.
@@ -926,7 +929,7 @@ int batch_tape_begin(MpmBatch* b, BatchAdjoint* x, int len, cudaStream_t s) {
     BCK(b, cudaMemsetAsync(x->tile_union, 0, sizeof(int) * (size_t)b->ntiles, s));
     x->nrtiles = -1;
     for (int i = 0; i < (int)b->sims.size(); ++i) {
-        BTRY(b, i, tape_begin(b->sims[i], b->sims[i]->adj, len, s, false));
+        BTRY(b, i, tape_begin(b->sims[i], b->sims[i]->adj, len, s, true));
         every.push_back(i);
     }
     return capture_epochs(b, x, every, s);
