@@ -36,6 +36,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <map>
 #include <vector>
 
@@ -95,6 +96,7 @@ struct AdjointState {
     std::vector<int64_t> resort_steps;
     std::vector<Checkpoint> ck;   // ck[s]: start of segment s; ck[nseg]: end state (several segments)
     int tape_seg = -1;         // the segment whose steps the tape holds, or -1
+    uint64_t taped_with = 0;   // what taped it: BatchAdjoint::tape_id, or 0 for the handle alone
     // sized for np_alloc particles and tape_slots steps
     int64_t np_alloc = -1;
     int tape_slots = 0;
@@ -137,10 +139,12 @@ struct BatchAdjoint {
     SegBuf misc;
     int* mismatch = nullptr;
     int* h_mismatch = nullptr;
-    // the tiles with particles in any sort of the taped segment
+    // the tiles with particles in any sort of the segment that the batch taped
+    // (the one of its members whose taped_with is tape_id, unique per taping)
+    uint64_t tape_id = 0;
     int* tile_union = nullptr;
     int4 *rtiles = nullptr, *rempty = nullptr;
-    int nrtiles = -1;
+    int nrtiles = -1;          // grid over rtiles; -1: not formed yet, -2: the set lacks a replay's sorts
     // graphs of the reverse steps (first and last slot, tiles, particle
     // blocks), valid for the buffers in `gsig`
     GraphMap g_rev;
@@ -516,6 +520,7 @@ int tape_begin(MpmHandle* h, AdjointState* a, int len, cudaStream_t s, bool batc
     a->nrtiles = -1;
     a->all_tiles = batched;
     a->tape_seg = -1;
+    a->taped_with = 0;
     a->seg_first = h->step;
     a->epoch_of.assign(len, 0);
     a->nep = 0;
@@ -925,11 +930,14 @@ int capture_epochs(MpmBatch* b, BatchAdjoint* x, const std::vector<int>& members
 
 // tape_begin for every member.
 int batch_tape_begin(MpmBatch* b, BatchAdjoint* x, int len, cudaStream_t s) {
+    static std::atomic<uint64_t> tapings{0};   // (a member may belong to several batches)
     std::vector<int> every;
     BCK(b, cudaMemsetAsync(x->tile_union, 0, sizeof(int) * (size_t)b->ntiles, s));
     x->nrtiles = -1;
+    x->tape_id = ++tapings;
     for (int i = 0; i < (int)b->sims.size(); ++i) {
         BTRY(b, i, tape_begin(b->sims[i], b->sims[i]->adj, len, s, true));
+        b->sims[i]->adj->taped_with = x->tape_id;
         every.push_back(i);
     }
     return capture_epochs(b, x, every, s);
@@ -1008,9 +1016,13 @@ int batch_taped_steps(MpmBatch* b, BatchAdjoint* x, int n, cudaStream_t s) {
     return r;
 }
 
-// The tiles of the batched reverse node passes (reverse_tiles).
+// The tiles of the batched reverse node passes (reverse_tiles): every tile when a
+// member's segment was not taped with the batch's present tile set (members may
+// be recorded one by one).
 int batch_reverse_tiles(MpmBatch* b, BatchAdjoint* x, const int4*& tiles, int& ntiles, cudaStream_t s) {
-    if (x->nrtiles == -2) {
+    bool apart = x->nrtiles == -2;
+    for (const MpmHandle* h : b->sims) apart = apart || !x->tape_id || h->adj->taped_with != x->tape_id;
+    if (apart) {
         tiles = b->d_tiles;
         ntiles = b->ntiles;
         return MPM_OK;

@@ -1,6 +1,8 @@
-"""A member of a batch stays an ordinary simulation: its own adjoint after
-Batch.record gives the bits of a recording of its own -- kept whole or as
-checkpoints, and with a rolled-back member."""
+"""Recordings of a batch's members made together and apart: a member of a batch
+stays an ordinary simulation, so its own adjoint after Batch.record, and the
+batch's adjoint after each member recorded alone, give the bits of the call that
+matches the recording -- kept whole or as checkpoints, in a fresh batch, after an
+earlier recording of other particles' tiles, and with a rolled-back member."""
 import numpy as np
 import pytest
 
@@ -58,4 +60,31 @@ def test_member_after_batch_record(built, limit, K, thrown):
     equal([gradients(m[0], m[2]) for m in out], refs, "each member again")
     if thrown:
         assert out[-1][0].counters()["rollbacks"] > 0
+    batch.close()
+
+
+@pytest.mark.parametrize("limit,K", [(-1, 40), (-1, 20), (0, 20)])
+@pytest.mark.parametrize("before", [False, True])
+def test_batch_after_members_record(built, limit, K, before):
+    out, batch = members(CASES, limit)
+    refs = references(CASES, K)
+    if before:                               # a recording of other tiles
+        for sim, start, _ in out:
+            loc = sim.read("loc")
+            sim.write("loc", loc + np.float32(100.0 / 128))
+            sim.initialize()
+        batch.record(STEPS, K)
+        batched(batch, out)
+        for _, start, _ in out:
+            start()
+    for sim, _, _ in out:
+        sim.record(STEPS, K)
+    equal(batched(batch, out), refs, "recorded apart")
+    batch.record(STEPS, K)
+    for _, start, _ in out:
+        start()
+    batch.record(STEPS, K)
+    out[0][1]()
+    out[0][0].record(STEPS, K)               # one member again, alone
+    equal(batched(batch, out), refs, "one member recorded apart")
     batch.close()
