@@ -34,7 +34,7 @@ def _dev_f32(t, device):
 
 class ExplicitRun(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, E, loc, velocity, mpm, gravity, nsteps, checkpoint_steps):
+    def forward(ctx, E, loc, velocity, mpm, gravity, nsteps, checkpoint_steps, tape_limit=-1):
         lease = mpm.lease_simulation(gravity, reinit=True)
         sim = lease.sim
         mpm._upload(sim)
@@ -48,6 +48,7 @@ class ExplicitRun(torch.autograd.Function):
         if velocity is not None:
             sim.write("velocity", put(velocity.reshape(-1, d)))
         sim.initialize()
+        sim.set_tape_limit(tape_limit)
         sim.record(nsteps, checkpoint_steps)
         n = sim.n
         if dev is not None:
@@ -89,12 +90,15 @@ class ExplicitRun(torch.autograd.Function):
                 continue
             g = out[key] if dev is not None else torch.from_numpy(out[key])
             grads.append(g.reshape(shape).to(dtype))
-        return grads[0], grads[1], grads[2], None, None, None, None
+        return grads[0], grads[1], grads[2], None, None, None, None, None
 
 
-def explicit_run(mpm, gravity, E, loc=None, velocity=None, nsteps=None, checkpoint_steps=100):
+def explicit_run(mpm, gravity, E, loc=None, velocity=None, nsteps=None, checkpoint_steps=100, tape_limit=-1):
     """Final (positions, velocities) of ``nsteps`` (default ``mpm.sim_steps``)
-    steps, differentiable w.r.t. ``E`` and the optional ``loc``/``velocity``."""
+    steps, differentiable w.r.t. ``E`` and the optional ``loc``/``velocity``;
+    ``checkpoint_steps`` and ``tape_limit`` set the memory that the recorded run
+    may take (``Simulation.record``, ``Simulation.set_tape_limit``)."""
     g = torch.as_tensor(np.asarray(gravity, dtype=np.float64))
     return ExplicitRun.apply(E, loc, velocity, mpm, tuple(g.tolist()),
-                             int(mpm.sim_steps if nsteps is None else nsteps), int(checkpoint_steps))
+                             int(mpm.sim_steps if nsteps is None else nsteps), int(checkpoint_steps),
+                             int(tape_limit))

@@ -10,7 +10,8 @@
 // where re-sorts, snapshots and reads find the state.
 //
 // mpm_record tapes the whole run when that fits a bounded share of the device
-// memory; mpm_adjoint then only runs the reverse passes of mpm_adjoint.h from
+// memory and a bounded multiple of what the checkpoints asked for would take;
+// mpm_adjoint then only runs the reverse passes of mpm_adjoint.h from
 // the last step to the first.  A longer run is cut into segments of K steps,
 // with a full copy of the state at the start of every segment (and at the
 // end) and the steps before which the particles were re-sorted: record tapes
@@ -185,15 +186,8 @@ void free_tape(MpmHandle* h, AdjointState* a) {
     a->tape_seg = -1;
 }
 
-void free_buffers(MpmHandle* h, AdjointState* a) {
-    free_tape(h, a);
-    for (auto& c : a->ck) checkpoint_free(h, c);
-    a->ck.clear();
-    dfree(h, a->tile_union);
-    dfree(h, a->rtiles);
-    dfree(h, a->rempty);
-    a->tile_union = nullptr;
-    a->rtiles = a->rempty = nullptr;
+void free_epochs(MpmHandle* h, AdjointState* a) {
+    drop_adj_graphs(a);
     for (Epoch& e : a->epochs) {
         dfree(h, e.pid);
         dfree(h, e.mat);
@@ -206,6 +200,18 @@ void free_buffers(MpmHandle* h, AdjointState* a) {
         dfree(h, e.psize);
     }
     a->epochs.clear();
+}
+
+void free_buffers(MpmHandle* h, AdjointState* a) {
+    free_tape(h, a);
+    for (auto& c : a->ck) checkpoint_free(h, c);
+    a->ck.clear();
+    dfree(h, a->tile_union);
+    dfree(h, a->rtiles);
+    dfree(h, a->rempty);
+    a->tile_union = nullptr;
+    a->rtiles = a->rempty = nullptr;
+    free_epochs(h, a);
     for (float*& p : a->lam) { dfree(h, p); p = nullptr; }
     for (float*& p : a->pscr) { dfree(h, p); p = nullptr; }
     for (float*& p : a->nscr) { dfree(h, p); p = nullptr; }
@@ -300,20 +306,56 @@ size_t tape_step_bytes(const MpmHandle* h) {
            (size_t)h->nn * 4 * NTN + (size_t)h->ncell * 5;
 }
 
-// Whether a run of nsteps steps of these bytes each is taped whole, however
-// short the segments asked for: it takes at most a tenth of the device's
-// memory and a quarter of what is free (`have`: tape bytes already held).
-// `limit`: the caller's bound in bytes, negative for none.
-bool tape_whole(size_t step_bytes, int nsteps, size_t have, int64_t limit) {
-    const size_t need = step_bytes * (size_t)nsteps;
-    if (limit >= 0 && need > (size_t)limit) return false;
-    if (need <= have) return true;
+// Bytes of a checkpoint (Checkpoint).
+size_t checkpoint_bytes(MpmHandle* h) {
+    const size_t nf = movable_f32(h, h->ps[h->pcur], false).size();
+    return (size_t)h->np * (4 * nf + 1 + (h->has_trac ? 10 : 0) + (h->has_pvc ? 2 : 0)) + (size_t)h->ncell * 5 +
+           (size_t)h->nn * 8;
+}
+
+// What a recording of one handle, or of all members of a batch, holds or would.
+struct TapeNeed {
+    size_t step = 0, checkpoint = 0, have = 0;   // bytes of a taped step, of a checkpoint; of the tape held
+    int64_t limit = -1;                          // mpm_set_tape_limit, of a batch the least; negative: none
+    void add(MpmHandle* h) {
+        step += tape_step_bytes(h);
+        checkpoint += checkpoint_bytes(h);
+        have += tape_step_bytes(h) * (size_t)h->adj->tape_slots;
+        if (h->tape_limit >= 0 && (limit < 0 || h->tape_limit < limit)) limit = h->tape_limit;
+    }
+};
+
+// Whether a run of nsteps steps is taped whole rather than in segments of the
+// K steps that the caller asked for: within the caller's bound, or without one
+// within TAPE_OVER times what checkpoints every K steps and a segment's tape
+// take (K is how a caller trades memory for re-runs), and at most a tenth of
+// the device's memory and a quarter of what is free.
+bool tape_whole(const TapeNeed& m, int nsteps, int K) {
+    const size_t need = m.step * (size_t)nsteps, nseg = ((size_t)nsteps + K - 1) / (size_t)K;
+    const size_t asked = m.checkpoint * (nseg + 1) + m.step * (size_t)std::min(K, nsteps);
+    if (need > (m.limit >= 0 ? (size_t)m.limit : TAPE_OVER * asked)) return false;
+    if (need <= m.have) return true;
     size_t free_b = 0, total = 0;
     if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return need <= total / 10 && need - have <= free_b / 4;
+    return need <= total / 10 && need - m.have <= free_b / 4;
+}
+
+// Before a recording of `slots` taped steps: give back a longer tape (and the
+// sort epochs) that is over the caller's bound or TAPE_OVER times as long, and
+// the checkpoints when it keeps none.
+void shrink(MpmHandle* h, AdjointState* a, const TapeNeed& m, int slots, bool checkpoints) {
+    const bool over = m.limit >= 0 && m.have > (size_t)m.limit;
+    if (a->tape_slots > slots && (over || (size_t)a->tape_slots > TAPE_OVER * (size_t)slots)) {
+        free_tape(h, a);
+        free_epochs(h, a);
+    }
+    if (!checkpoints) {
+        for (auto& c : a->ck) checkpoint_free(h, c);
+        a->ck.clear();
+    }
 }
 
 void add_seg(std::vector<CopySeg>& v, const void* src, void* dst, size_t bytes, size_t step) {
@@ -1184,8 +1226,10 @@ int mpm_record(MpmHandle* h, int nsteps, int checkpoint_steps, void* stream) {
     TRY(record_begin(h, nsteps, checkpoint_steps));
     cudaStream_t s = S(stream);
     AdjointState* a = h->adj;
-    if (tape_whole(tape_step_bytes(h), nsteps, tape_step_bytes(h) * (size_t)a->tape_slots, h->tape_limit))
-        record_segments(a, nsteps);
+    TapeNeed need;
+    need.add(h);
+    if (tape_whole(need, nsteps, checkpoint_steps)) record_segments(a, nsteps);
+    shrink(h, a, need, std::min(a->K, nsteps), a->nseg > 1);
     bool taped = ensure_tape(h, a, std::min(a->K, nsteps)) == MPM_OK;
     if (!taped && a->K > checkpoint_steps) {
         record_segments(a, checkpoint_steps);
@@ -1258,14 +1302,8 @@ int mpm_batch_record(MpmBatch* b, int nsteps, int checkpoint_steps, void* stream
     const int n = (int)b->sims.size();
     for (int i = 0; i < n; ++i) BTRY(b, i, record_begin(b->sims[i], nsteps, checkpoint_steps));
     cudaStream_t s = S(stream);
-    size_t step_bytes = 0, have = 0;
-    for (MpmHandle* h : b->sims) {
-        step_bytes += tape_step_bytes(h);
-        have += tape_step_bytes(h) * (size_t)h->adj->tape_slots;
-    }
-    int64_t limit = -1;   // of the whole batch: the least of its members' bounds
-    for (MpmHandle* h : b->sims)
-        if (h->tape_limit >= 0 && (limit < 0 || h->tape_limit < limit)) limit = h->tape_limit;
+    TapeNeed need;   // of the whole batch
+    for (MpmHandle* h : b->sims) need.add(h);
     auto ensure_tapes = [&](int K) {
         for (MpmHandle* h : b->sims) {
             record_segments(h->adj, K);
@@ -1273,7 +1311,9 @@ int mpm_batch_record(MpmBatch* b, int nsteps, int checkpoint_steps, void* stream
         }
         return true;
     };
-    const bool whole = tape_whole(step_bytes, nsteps, have, limit);
+    const bool whole = tape_whole(need, nsteps, checkpoint_steps);
+    const int slots = whole ? nsteps : std::min(checkpoint_steps, nsteps);
+    for (MpmHandle* h : b->sims) shrink(h, h->adj, need, slots, slots < nsteps);
     bool taped = ensure_batch_tape(b) == MPM_OK && ensure_tapes(whole ? nsteps : checkpoint_steps);
     if (!taped && whole) {
         for (MpmHandle* h : b->sims) free_tape(h, h->adj);

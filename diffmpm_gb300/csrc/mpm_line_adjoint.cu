@@ -447,9 +447,10 @@ int line_record(MpmHandle* h, int nsteps, cudaStream_t s) {
     const size_t np = (size_t)h->np, nn = (size_t)h->nn, T = (size_t)nsteps;
     const size_t bytes = T * (np * (LP_N + 1) + (size_t)(h->nx + 2) + nn * LN_N) * 4;
     // the arrays of the last recording serve the next one of the same bar that
-    // is no longer (a training loop records the same run again and again)
+    // is no longer, nor much shorter (a training loop records the same run
+    // again and again)
     LineAdjoint* a = h->line_adj;
-    if (a && (a->np != h->np || a->nn != h->nn || a->cap < nsteps)) {
+    if (a && (a->np != h->np || a->nn != h->nn || a->cap < nsteps || (size_t)a->cap > TAPE_OVER * T)) {
         line_adjoint_free(h);
         a = nullptr;
     }

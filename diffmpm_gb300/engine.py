@@ -408,14 +408,17 @@ class Simulation:
 
     # ------------------------------------------------------------------
     def set_tape_limit(self, nbytes):
-        """Bound the memory of a run that :meth:`record` keeps whole (0: always
-        checkpoints, negative: the default bound); the same gradients."""
+        """Bound, in bytes, the memory of a run that :meth:`record` keeps whole
+        (0: always checkpoints; negative: the default, a multiple of what its
+        ``checkpoint_steps`` asks for); the same gradients.  The next record
+        gives back what an earlier one holds beyond it."""
         self._ok(self._lib.mpm_set_tape_limit(self._h, int(nbytes)))
 
     def record(self, nsteps, checkpoint_steps=100, stream=None):
-        """Advance ``nsteps`` steps keeping what :meth:`adjoint` needs: every
-        step's start state when that fits a bounded share of the device
-        memory, else a checkpoint every ``checkpoint_steps`` steps."""
+        """Advance ``nsteps`` steps keeping what :meth:`adjoint` needs: a
+        checkpoint every ``checkpoint_steps`` steps, or every step's start
+        state where that takes at most six times the memory and fits a bounded
+        share of the device's (:meth:`set_tape_limit` sets another bound)."""
         self._ok(self._lib.mpm_record(self._h, int(nsteps), int(checkpoint_steps), stream))
 
     def adjoint(self, dl_dloc, dl_dvel=None, *, want=("youngs_modulus", "loc", "velocity")):
@@ -591,6 +594,12 @@ class Batch:
         if path is not None:
             _write_tuning_cache(path, key, out)
         return dict(out, from_cache=False, key=key)
+
+    def set_tape_limit(self, nbytes):
+        """``Simulation.set_tape_limit`` of every member: in a batch it bounds
+        the members' tapes together."""
+        for sim in self.sims:
+            sim.set_tape_limit(nbytes)
 
     def record(self, nsteps, checkpoint_steps=100, stream=None):
         """``Simulation.record`` for every member at once."""

@@ -257,17 +257,20 @@ int mpm_get_counters(const MpmHandle* h, int64_t* resorts, int64_t* rollbacks);
  * or USL, with or without the per-step volume set-up, particle tractions and
  * particle velocity constraints.
  *
- * mpm_record advances `nsteps` steps like mpm_step and keeps every step's start
- * state and nodal results (the tape) when they take at most a tenth of the
- * device's memory and a quarter of what is free (mpm_set_tape_limit lowers
- * that).  Otherwise it keeps a checkpoint of the full state every
- * `checkpoint_steps` steps (and at the end) and the tape of the last
- * checkpoint_steps steps.  A Linear1D mesh always keeps the tape.  The
- * gradients are the same bits either way. */
+ * mpm_record advances `nsteps` steps like mpm_step and keeps a checkpoint of
+ * the full state every `checkpoint_steps` steps (and at the end) and the tape
+ * (every step's start state and nodal results) of the last checkpoint_steps
+ * steps.  Where the tape of the whole run takes at most 6 times that, a tenth
+ * of the device's memory and a quarter of what is free, it keeps that tape
+ * and no checkpoints (mpm_set_tape_limit sets another bound).  A Linear1D mesh
+ * always keeps the tape.  The gradients are the same bits either way.  A tape
+ * is kept for the handle's next recording, which gives it back when it is over
+ * the bound set by then or more than 6 times as long as needed. */
 int mpm_record(MpmHandle* h, int nsteps, int checkpoint_steps, void* stream);
 
-/* Bound, in bytes, on the tape of a run that mpm_record keeps whole (0: always
- * checkpoints; negative, the default: the bound above).  In a batch the least
+/* Bound, in bytes, on the tape of a run that mpm_record keeps whole, in place of
+ * the 6 times (0: checkpoints, with the tape of checkpoint_steps steps;
+ * negative, the default: no such bound).  In a batch the least
  * of the members' bounds holds for the whole batch.  Applies from the next
  * record.  No counterpart in the reference. */
 int mpm_set_tape_limit(MpmHandle* h, int64_t bytes);
