@@ -97,6 +97,7 @@ SIGNATURES = [
     ("mpm_set_block_steps", C.c_int, [_VP, C.c_int]),
     ("mpm_set_kernel_variant", C.c_int, [_VP, C.c_int, C.c_int, C.c_int]),
     ("mpm_set_empty_split", C.c_int, [_VP, C.c_int]),
+    ("mpm_set_wait_polls", C.c_int, [_VP, C.c_int64]),
     ("mpm_set_tape_limit", C.c_int, [_VP, C.c_int64]),
     ("mpm_device_name", C.c_int, [C.c_int, C.c_char_p, C.c_int]),
     ("mpm_get_counters", C.c_int, [_VP, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),

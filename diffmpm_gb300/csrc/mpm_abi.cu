@@ -316,7 +316,8 @@ int run_steps(MpmHandle* h, int n, cudaStream_t s) {
     TRY(classify_tiles(h, s));
     if (n >= RESIDENT_STEPS && resident(h)) {
         CK(h, launch_empty_nodes(h->hs, h->d_empty, h->nemp, h->ctl, 0, s));
-        CK(h, launch_steps_resident(step_config(h), h->hs, h->step_tiles, h->nlist, h->ctl, h->d_arrived, n, s));
+        CK(h, launch_steps_resident(step_config(h), h->hs, h->step_tiles, h->nlist, h->ctl, h->d_arrived, n,
+                                    h->wait_polls, s));
         return MPM_OK;
     }
     if (n >= GRAPH_STEPS) {
@@ -1272,7 +1273,10 @@ int mpm_step(MpmHandle* h, int nsteps, void* stream) {
         // a two-cell drift corrupts the rest of the block (a particle may even be
         // thrown out of the mesh by it): roll back before judging anything else
         int st = h->h_ctl->status;
-        if (st & ST_STALLED) TRY(check_status(h, st));
+        if (st & ST_STALLED) {   // the block did not run to its end: back to its start
+            TRY(restore_snapshot(h, step0, s));
+            TRY(check_status(h, st));
+        }
         if (st & ST_DRIFT_VIOLATION) TRY(replay_block(h, step0, B, st, s));
         else TRY(check_status(h, st));
         h->needs_resort = (st & ST_DRIFTED) != 0;
@@ -1369,6 +1373,13 @@ int mpm_set_empty_split(MpmHandle* h, int min_empty) {
     if (!h) return MPM_ERR_INVALID;
     if (min_empty < 0) return fail(h, MPM_ERR_INVALID, "min_empty is negative");
     h->empty_split_min = min_empty;   // applies from the next classification
+    return MPM_OK;
+}
+
+int mpm_set_wait_polls(MpmHandle* h, int64_t polls) {
+    if (!h) return MPM_ERR_INVALID;
+    if (polls > (int64_t)0xffffffffu) return fail(h, MPM_ERR_INVALID, "polls must be below 2^32");
+    h->wait_polls = polls < 0 ? BARRIER_POLLS : (unsigned)polls;
     return MPM_OK;
 }
 

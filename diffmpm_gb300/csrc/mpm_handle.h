@@ -144,6 +144,7 @@ struct MpmHandle {
     int nlist = 0;                   // tiles on the step kernels' list (nact without its rounding)
     int sm_count = 0;
     unsigned* d_arrived = nullptr;   // barrier word of resident steps
+    unsigned wait_polls = mpm::BARRIER_POLLS;   // mpm_set_wait_polls
     const int4* step_tiles = nullptr; // the step kernels' list: d_active after a split, else dtiles
     int64_t step = 0;
     // staging and pointer tables

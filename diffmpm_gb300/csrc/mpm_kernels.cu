@@ -1347,10 +1347,9 @@ k_particle_kinematics_batch(const TileDesc* __restrict__ td, int k) {
 // Every wait is bounded: a CTA that gives up sets ST_STALLED and returns, and
 // so do the others in turn.
 // ---------------------------------------------------------------------------
-constexpr unsigned BARRIER_POLLS = 1u << 22;
-
 // False for every CTA when the wait ran out or `stop` is set for their threads 0.
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, Control* ctl, bool stop = false) {
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, Control* ctl, unsigned polls,
+                                             bool stop = false) {
     __shared__ int s_ok;
     __syncthreads();
     target += gridDim.x;
@@ -1358,7 +1357,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target
         bool ok = gridDim.x == 1;
         if (!ok) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
-            for (unsigned i = 0; i < BARRIER_POLLS && !ok; ++i) {
+            for (unsigned i = 0; i < polls && !ok; ++i) {
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
                 ok = (int)(v - target) >= 0;
@@ -1374,7 +1373,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target
 template <bool USL, bool REINIT, bool TRAC>
 __global__ void __launch_bounds__(TILE_THREADS, 1)
 k_steps_resident(const __grid_constant__ SimDev S, const int4* __restrict__ tiles, Control* ctl,
-                 unsigned* arrived, int n) {
+                 unsigned* arrived, int n, unsigned polls) {
     // kept over the steps: the row starts (nothing re-sorts within a sequence),
     // the geometry and the materials
     __shared__ RowStarts starts;
@@ -1397,11 +1396,11 @@ k_steps_resident(const __grid_constant__ SimDev S, const int4* __restrict__ tile
         // this step's comes after the next two: every CTA reads the same.)
         const int status = threadIdx.x == 0 ? *reinterpret_cast<volatile int*>(&ctl->status) : 0;
         nodal_kinematics_tile<REINIT, true, true>(S, T, ctl, step0 + k, G, &starts);
-        if (!grid_barrier(arrived, target, ctl, status & ST_DRIFT_VIOLATION)) return;
+        if (!grid_barrier(arrived, target, ctl, polls, status & ST_DRIFT_VIOLATION)) return;
         forces_tile<USL, REINIT, TRAC, false, USL ? FM_LPC : FM_ROW, true>(S, T, ctl, step0 + k, G, &starts);
-        if (!grid_barrier(arrived, target, ctl)) return;
+        if (!grid_barrier(arrived, target, ctl, polls)) return;
         particle_kinematics_tile<USL, REINIT, true, TILE_CY, true>(S, T, ctl, step0 + k, G, &starts);
-        if (!grid_barrier(arrived, target, ctl)) return;
+        if (!grid_barrier(arrived, target, ctl, polls)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->step += n;
 }
@@ -1423,9 +1422,9 @@ static void prefer_shared(K kernel) {
 
 template <bool USL, bool REINIT, bool TRAC>
 static cudaError_t steps_resident(const SimDev& S, const int4* tiles, int ntiles, Control* ctl, unsigned* arrived,
-                                  int n, cudaStream_t s) {
+                                  int n, unsigned polls, cudaStream_t s) {
     prefer_shared(k_steps_resident<USL, REINIT, TRAC>);
-    void* args[] = {const_cast<SimDev*>(&S), &tiles, &ctl, &arrived, &n};
+    void* args[] = {const_cast<SimDev*>(&S), &tiles, &ctl, &arrived, &n, &polls};
     cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_steps_resident<USL, REINIT, TRAC>), dim3(ntiles),
@@ -1433,14 +1432,14 @@ static cudaError_t steps_resident(const SimDev& S, const int4* tiles, int ntiles
 }
 
 cudaError_t launch_steps_resident(const StepConfig& c, const SimDev& S, const int4* tiles, int ntiles, Control* ctl,
-                                  unsigned* arrived, int n, cudaStream_t s) {
-    using Fn = cudaError_t (*)(const SimDev&, const int4*, int, Control*, unsigned*, int, cudaStream_t);
+                                  unsigned* arrived, int n, unsigned polls, cudaStream_t s) {
+    using Fn = cudaError_t (*)(const SimDev&, const int4*, int, Control*, unsigned*, int, unsigned, cudaStream_t);
     static constexpr Fn fns[8] = {
         steps_resident<false, false, false>, steps_resident<false, false, true>,
         steps_resident<false, true, false>,  steps_resident<false, true, true>,
         steps_resident<true, false, false>,  steps_resident<true, false, true>,
         steps_resident<true, true, false>,   steps_resident<true, true, true>};
-    return fns[c.usl * 4 + c.reinit * 2 + c.traction](S, tiles, ntiles, ctl, arrived, n, s);
+    return fns[c.usl * 4 + c.reinit * 2 + c.traction](S, tiles, ntiles, ctl, arrived, n, polls, s);
 }
 
 // The nodal kinematics and USF G2P kernels come in two builds: 40 registers

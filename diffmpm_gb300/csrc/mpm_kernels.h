@@ -48,13 +48,15 @@ cudaError_t launch_particle_kinematics(const StepConfig& c, const SimDev& S, con
                                        int ntiles, Control* ctl, int k, cudaStream_t s);
 // n whole steps over at most one tile per SM in one cooperative launch, with
 // the default forces path; advances the step counter.  `arrived`: one word of
-// scratch.  ST_STALLED in the status means that a wait ran out.  A cooperative
+// scratch.  ST_STALLED in the status means that a wait of `polls` reads ran out
+// (BARRIER_POLLS reads take seconds, a step of such a run microseconds).  A cooperative
 // launch costs about two steps of plain launches, so fewer than RESIDENT_STEPS
 // steps take those (a thrown block whose 200 steps are replayed one at a time:
 // 26.0 ms with one-step resident launches, 21 without).
 constexpr int RESIDENT_STEPS = 8;
+constexpr unsigned BARRIER_POLLS = 1u << 22;
 cudaError_t launch_steps_resident(const StepConfig& c, const SimDev& S, const int4* tiles, int ntiles, Control* ctl,
-                                  unsigned* arrived, int n, cudaStream_t s);
+                                  unsigned* arrived, int n, unsigned polls, cudaStream_t s);
 // Split the tile list into active tiles (cells or their ring store a
 // particle; the step kernels' grid) and empty ones (node updates only,
 // k_empty_nodes), in tile order, both padded to ntiles entries with

@@ -239,6 +239,11 @@ class Simulation:
         of them (mpm_set_empty_split): the same results either way."""
         self._ok(self._lib.mpm_set_empty_split(self._h, int(min_empty)))
 
+    def set_wait_polls(self, polls):
+        """Reads after which a wait between the CTAs of one launch gives up
+        (mpm_set_wait_polls; negative: the default)."""
+        self._ok(self._lib.mpm_set_wait_polls(self._h, int(polls)))
+
     def set_kernel_variant(self, nk_ctas=3, g2p_ctas=2, forces_lpc=0):
         """Kernel builds of the step (mpm_set_kernel_variant): the same results,
         built for 2 or 3 resident CTAs per SM, and any of the three forces

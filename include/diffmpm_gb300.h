@@ -237,6 +237,12 @@ int mpm_set_kernel_variant(MpmHandle* h, int nk_ctas, int g2p_ctas, int forces_l
  * INT_MAX never does.  No counterpart in the reference. */
 int mpm_set_empty_split(MpmHandle* h, int min_empty);
 
+/* Steps of a small run go in one launch whose CTAs wait for one another.  A wait
+ * gives up after `polls` reads (negative, the default: 2^22, some seconds); the
+ * call then returns MPM_ERR_CUDA and the handle is back at the start of the step
+ * block, as good as before the call.  No counterpart in the reference. */
+int mpm_set_wait_polls(MpmHandle* h, int64_t polls);
+
 /* Name of CUDA device `device` with its compute capability and SM count
  * (NUL-terminated, truncated to len bytes), the GPU part of the key under
  * which tuning results are cached.  No counterpart in the reference. */
