@@ -1262,6 +1262,7 @@ int mpm_step(MpmHandle* h, int nsteps, void* stream) {
         TRY(clear_status(h, s));
         return sync(h, s);
     }
+    if (nsteps == 0) return sync(h, s);   // (the call waits for its stream)
     while (nsteps > 0) {
         const int B = nsteps < h->block_steps ? nsteps : h->block_steps;
         if (h->needs_resort) TRY(resort(h, s));
