@@ -558,7 +558,7 @@ int tape_begin(MpmHandle* h, AdjointState* a, int len, cudaStream_t s, bool batc
         TRY(dalloc(h, &a->rtiles, (size_t)h->ntiles));
         TRY(dalloc(h, &a->rempty, (size_t)h->ntiles));
     }
-    CK(h, cudaMemsetAsync(a->tile_union, 0, sizeof(int) * (size_t)h->ntiles, s));
+    if (!batched) CK(h, cudaMemsetAsync(a->tile_union, 0, sizeof(int) * (size_t)h->ntiles, s));
     // (a step writes the flags of its listed tiles' cells; those of an empty tile,
     // which a listed one beside it reads, are clear in every slot)
     CK(h, cudaMemsetAsync(a->tflag, 0, (size_t)h->ncell * (size_t)len, s));
