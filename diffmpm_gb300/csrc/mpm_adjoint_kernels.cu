@@ -1025,7 +1025,7 @@ constexpr RevParticlesFn kRevStress[4] = {
 // idle and a thread per particle fills it; above it the gathers through L2
 // bind.  A reverse USF step of one simulation by tile / by particle: 117 tiles
 // 29.1 / 25.8 us, 216 tiles 38.9 / 34.8, 294 tiles 40.2 / 40.8, 442 tiles
-// 62.9 / 67.4, 672 tiles 100 / 109; 40 simulations in a batch (1.5M
+// 62.9 / 67.4, 672 tiles 100 / 109; 40 simulations in a batch (1.94M
 // particles), forces pass 72 / 91 us, mass pass 30 / 38.
 constexpr int REV_BY_TILE = 304;
 

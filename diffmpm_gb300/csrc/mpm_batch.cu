@@ -8,9 +8,9 @@
 // tile, its simulation's control pointer, a copy of the simulation's
 // descriptor (the handle's device copy, which a re-sort updates in place) and
 // the tile's row starts; the batched kernels read their tile's record, so a
-// captured graph of a step block stays valid across re-sorts.  Per block:
+// captured graph (of GRAPH_STEPS steps) stays valid across re-sorts.  Per block:
 // re-sort the simulations that drifted, snapshot all of them (one segmented
-// copy), refresh the records, run the block graph, gather every status word
+// copy), refresh the records, run the steps, gather every status word
 // in one copy; a simulation whose particle drifted two cells is rolled back
 // and replayed alone, step by step.
 // No counterpart in the reference, which runs one simulation per solve.

@@ -679,8 +679,8 @@ enum ForcesMode { FM_ROW = 0, FM_LPC = 1, FM_STAGED = 2 };
 // after it: the lanes of a quarter warp write consecutive j and read every
 // fourth (cells of 4 particles) without bank conflicts.  (Issue-bound: two
 // wide accesses and four packed sums in place of eight of each, and half of
-// the stress products: 47.9 -> 46.3 us for 2.1M particles, 40 simulations'
-// batch 69.5 -> 66.6.  Rows of 128 a pass: 53, the larger buffers leave too
+// the stress products: 47.9 -> 46.3 us for 2.1M particles, a batch of 64
+// simulations (2.27M) 69.5 -> 66.6.  Rows of 128 a pass: 53, the larger buffers leave too
 // little L1 for the loads in flight; loads of the next chunk prefetched: 50.8.)
 constexpr __host__ __device__ int slot_unit(int j) { return 2 * j + (j >> 2); }
 struct ForceRows {

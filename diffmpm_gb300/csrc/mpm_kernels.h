@@ -24,7 +24,7 @@ struct StepConfig {
     bool traction;     // particle tractions present
     // resident CTAs per SM the nodal kinematics and USF G2P kernels are
     // built for: 3 (40 registers a thread) or 2 (up to 64).  (G2P, 2.1M particles:
-    // 20.2 us with 3, 21.2 with 2; a batch of 40: 29.0 and 31.4.)
+    // 20.2 us with 3, 21.2 with 2; a batch of 64, 2.27M: 29.0 and 31.4.)
     int nk_ctas = 3;
     int g2p_ctas = 3;
     // forces kernel fast path: particle per lane with row slots (0), lane

@@ -221,7 +221,8 @@ int mpm_run_phase(MpmHandle* h, int phase, void* stream);
  * measurement; the state advances as with mpm_step. */
 int mpm_time_phases(MpmHandle* h, int nsteps, float* ms_out, void* stream);
 
-/* Steps per captured CUDA graph (default 100). */
+/* Steps per block (default 100): re-sort if a particle drifted, snapshot, steps,
+ * one look at the status. */
 int mpm_set_block_steps(MpmHandle* h, int steps);
 /* Kernel builds of the step: the nodal-kinematics and USF G2P kernels for
  * nk_ctas / g2p_ctas resident CTAs per SM (2 or 3), and the forces kernel's
@@ -231,7 +232,8 @@ int mpm_set_kernel_variant(MpmHandle* h, int nk_ctas, int g2p_ctas, int forces_l
 
 /* Tiles whose cells and ring of cells store no particle need only a node
  * update per step.  When a simulation has at least `min_empty` such tiles
- * (default 128), its step kernels are launched over the other tiles and one
+ * (default 128; by default also when only the other tiles fit one to an SM),
+ * its step kernels are launched over the other tiles and one
  * kernel updates the empty tiles' nodes; otherwise every tile goes through
  * the step kernels.  Results are the same bits either way; 0 always splits,
  * INT_MAX never does.  No counterpart in the reference. */
@@ -297,7 +299,7 @@ int mpm_adjoint(MpmHandle* h, const float* dl_dloc, const float* dl_dvel, float*
 /* Batches of independent simulations.  No counterpart in the reference, which
  * runs one simulation per solve; a batch advances many (of any mesh and
  * particle counts) with one kernel launch per phase per step for all of
- * them, captured in CUDA graphs of step blocks.  The handles must be
+ * them, in captured CUDA graphs.  The handles must be
  * initialised, on one device, and share the scheme, volume set-up and
  * traction set-up; each keeps its own state, so mpm_read_field etc. work on
  * them as usual.  Destroy the batch before its handles (mpm_batch_destroy
@@ -327,11 +329,11 @@ int mpm_batch_restart(MpmBatch* b, void* stream);
 
 /* Advance every simulation by `nsteps` steps (as mpm_step does for one). */
 int mpm_batch_step(MpmBatch* b, int nsteps, void* stream);
-/* Steps per captured graph (default 100). */
+/* Steps per block (default 100), as for one simulation. */
 int mpm_batch_set_block_steps(MpmBatch* b, int steps);
 /* Tuning of a batch's step loop (no counterpart in the reference, which
  * runs one simulation per solve_jit):
- *   block_steps   steps per captured CUDA graph (a step block);
+ *   block_steps   steps per block;
  *   resort_every  a simulation whose particles left their sort-cells is
  *                 re-sorted at the start of every resort_every-th block (in
  *                 between its drifted cells take the gathering path; a
