@@ -611,7 +611,9 @@ __device__ __forceinline__ void rev_forces_at(const AdjStep& A, int q, const In&
     p.szz = in.template get<RF_SZZ>();
     p.sxy = in.template get<RF_SXY>();
     p.rho = rho0;
-    p.vsc = NEWT ? A.vsc[q] : 0.0f;   // taped when a material uses it (Newtonian)
+    // taped when a material uses it (Newtonian); in a batch with such members the
+    // others have none
+    p.vsc = NEWT && A.vsc ? A.vsc[q] : 0.0f;
     float f = 1.0f, V = V0;
     const MatDev& mat = A.mats[A.mat[q]];
     const float Ep = A.E ? A.E[q] : -1.0f;
