@@ -477,12 +477,14 @@ cudaError_t launch_line_steps(const SimDev& S, int par, int step0, int n, Contro
     return S.np <= T ? go(k_line_steps<REINIT, USL, 1>) : go(k_line_steps<REINIT, USL, 2>);
 }
 
-// Element of each storage slot: the bucket it was sorted into.
+// Element of each storage slot: the bucket it was sorted into.  Particles outside
+// the mesh (the last bucket; the call ends with an error) get the last element, so
+// that the kernels until then stay within their arrays.
 __global__ void k_line_eid(const int* __restrict__ cstart, int nx, int* __restrict__ eid) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nx) return;
+    if (e > nx) return;
     #pragma unroll 1
-    for (int q = cstart[e]; q < cstart[e + 1]; ++q) eid[q] = e;
+    for (int q = cstart[e]; q < cstart[e + 1]; ++q) eid[q] = min(e, nx - 1);
 }
 
 // Each element's particles in increasing original index (insertion sort of a
@@ -527,7 +529,7 @@ cudaError_t launch_line_segsort(int nbucket, const int* start, int* perm, const 
 }
 
 cudaError_t launch_line_eid(const int* cstart, int nx, int* eid, cudaStream_t s) {
-    if (nx > 0) k_line_eid<<<blocks(nx), LINE_THREADS, 0, s>>>(cstart, nx, eid);
+    if (nx > 0) k_line_eid<<<blocks(nx + 1), LINE_THREADS, 0, s>>>(cstart, nx, eid);
     return cudaGetLastError();
 }
 
