@@ -458,6 +458,10 @@ k_line_steps(const __grid_constant__ SimDev S, int par, int step0, int nsteps, C
         S.nvbx[i] = W.vb[i];
         S.nax[i] = W.a[i];
     }
+    // the element starts of the last step, as a sort before every step leaves them
+    // (a momentum read counts by them; the particles stay in their storage slots,
+    // which the next use sorts)
+    for (int i = tid; i < nx + 2; i += T) S.cstart[i] = W.start[i];
     if (status) atomicOr(&ctl->status, status);
 }
 
