@@ -1254,6 +1254,10 @@ __device__ __forceinline__ void particle_kinematics_tile(const SimDev& S, const 
         if (ci < 0 || ci >= S.nx || cj < 0 || cj >= S.ny) {
             status |= ST_OUT_OF_MESH;
             s_flag[w][l] = 1;
+            S.xo[q] = x;   // (a taped next step reads it from its own slot)
+            S.yo[q] = y;
+            S.vxo[q] = b[GF_VX][lane];
+            S.vyo[q] = b[GF_VY][lane];
             continue;
         }
         const int kc = ci - c0x + 1, kr = cj - c0y + 1;   // geometry table indices
