@@ -315,7 +315,7 @@ bool resident(const MpmHandle* h) {
 int run_steps(MpmHandle* h, int n, cudaStream_t s) {
     constexpr size_t GRAPH_CACHE = 8;
     TRY(classify_tiles(h, s));
-    if (n >= RESIDENT_STEPS && resident(h)) {
+    if (resident(h)) {
         CK(h, launch_empty_nodes(h->hs, h->d_empty, h->nemp, h->ctl, 0, s));
         CK(h, launch_steps_resident(step_config(h), h->hs, h->step_tiles, h->nlist, h->ctl, h->d_arrived, n,
                                     h->wait_polls, s));

@@ -49,11 +49,11 @@ cudaError_t launch_particle_kinematics(const StepConfig& c, const SimDev& S, con
 // n whole steps over at most one tile per SM in one cooperative launch, with
 // the default forces path; advances the step counter.  `arrived`: one word of
 // scratch.  ST_STALLED in the status means that a wait of `polls` reads ran out
-// (BARRIER_POLLS reads take seconds, a step of such a run microseconds).  A cooperative
-// launch costs about two steps of plain launches, so fewer than RESIDENT_STEPS
-// steps take those (a thrown block whose 200 steps are replayed one at a time:
-// 26.0 ms with one-step resident launches, 21 without).
-constexpr int RESIDENT_STEPS = 8;
+// (BARRIER_POLLS reads take seconds, a step of such a run microseconds).  One
+// such launch is shorter than the launches of its steps for any n (a call of one
+// step, of seven: 160 particles 40 -> 32 us, 138 -> 65; 136k particles 74 -> 69,
+// 212 -> 160), but not than the launches of a replayed step, whose status the
+// host waits for anyway (a thrown block of 200 of them: 26.0 ms with, 21 without).
 constexpr unsigned BARRIER_POLLS = 1u << 22;
 cudaError_t launch_steps_resident(const StepConfig& c, const SimDev& S, const int4* tiles, int ntiles, Control* ctl,
                                   unsigned* arrived, int n, unsigned polls, cudaStream_t s);
